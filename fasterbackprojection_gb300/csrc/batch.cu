@@ -35,6 +35,7 @@ struct BatchGroup {
     uint32_t nitems = 0;
     size_t smem = 0;
     int ctas = 0;
+    float* d_totals = nullptr;  // sums over chains, one slice per CTA (cfg 0)
 };
 
 constexpr int kMaxGroups = 64;
@@ -58,6 +59,8 @@ struct fbp_batch {
     fbp::BatchItem* d_items = nullptr;
     size_t items_cap = 0;
     unsigned int* d_counters = nullptr;
+    float* d_totals = nullptr;
+    size_t totals_cap = 0;  // floats
     std::vector<fbp::ConfocalGatherParams> params;
     std::vector<fbp::BatchGroup> groups;
     cudaGraph_t graph = nullptr;
@@ -90,10 +93,10 @@ void drop_graph(fbp_batch* b) {
 // rows are made), so one set of kernels serves all of them.
 constexpr size_t kRowBytes = sizeof(float);
 
-fbp_status prepare_any(const BatchLaunch& l, int* occ) { return batch_prepare_kernel<float>(l, occ); }
+fbp_status prepare_any(const BatchLaunch& l, int* occ) { return batch_prepare_kernel(l, occ); }
 
 fbp_status launch_any(fbp_context* ctx, const BatchLaunch& l, int ctas, cudaStream_t s) {
-    return batch_launch<float>(ctx, l, ctas, s);
+    return batch_launch(ctx, l, ctas, s);
 }
 
 fbp_status rows_any(fbp_context* ctx, int dtype, const fbp_capture_desc& c, uint32_t pitch, void* dst,
@@ -111,7 +114,7 @@ fbp_status rows_any(fbp_context* ctx, int dtype, const fbp_capture_desc& c, uint
 fbp_status plan_config(fbp_batch* b, int cfg, cudaStream_t s) {
     const TileCfg tc = kTileCfgs[cfg];
     const int align = (int)(16 / kRowBytes);
-    const size_t meta = ConfocalGatherParams::meta_bytes(32) + kahan_smem_bytes(tc.kv, 32 * tc.wy * tc.wz) + 16;
+    const size_t meta = ConfocalGatherParams::meta_bytes(tc.kv) + kahan_smem_bytes(tc.kv, 32 * tc.wy * tc.wz) + 16;
     const uint32_t n = (uint32_t)b->caps.size();
     b->params.assign(n, ConfocalGatherParams{});
     b->groups.clear();
@@ -125,13 +128,13 @@ fbp_status plan_config(fbp_batch* b, int cfg, cudaStream_t s) {
         const double ez = (double)std::min<uint32_t>(8 * tc.wy, in.voxel_res[1]) * std::fabs(in.voxel_size[2]);
         WindowPlan wp;
         FBP_TRY(plan_window(b->ctx, ex, ey, ez, in.time_step, in.num_time_bins, align, kRowBytes, meta, &wp,
-                            "fbp_batch"));
+                            "fbp_batch", 0.0, kGatherCtasPerSm, ConfocalGatherParams::kWindowBufs));
         // Leave room for the persistent kernel's own static shared memory
         // (replanning only the windows that fill the SM, so the others keep
         // the single-capture gather's plan).
         if (wp.smem + kBatchStaticSmem > (size_t)b->ctx->smem_optin)
             FBP_TRY(plan_window(b->ctx, ex, ey, ez, in.time_step, in.num_time_bins, align, kRowBytes,
-                                meta + kBatchStaticSmem, &wp, "fbp_batch"));
+                                meta + kBatchStaticSmem, &wp, "fbp_batch", 0.0, kGatherCtasPerSm, ConfocalGatherParams::kWindowBufs));
         pitches[i] = wp.pitch;
         rows_off[i] = rows_total;
         rows_total += ((size_t)in.num_laser_targets * wp.pitch * kRowBytes + 255) & ~size_t(255);
@@ -152,11 +155,13 @@ fbp_status plan_config(fbp_batch* b, int cfg, cudaStream_t s) {
         p.row_pitch = wp.pitch;
         p.slot_w = wp.slot_w;
         p.ch = wp.ch;
+        // The single call's chains where the tile is the single call's.
+        p.chains = cfg == 0 ? gather_chains(b->ctx, in, wp.smem) : 1;
         p.exact_weights = b->ctx->weight_mode == FBP_WEIGHTS_REFERENCE;
         // Group by arithmetic variant and occupancy.
         const int path = path_of(in);
         const bool bounce = in.discard_first_last_bounces == 0;
-        const bool clamp = path == PATH_EXACT || wp.capped;
+        const bool clamp = wp.capped;
         BatchLaunch probe{};
         probe.smem = wp.smem;
         probe.smem_limit = (size_t)b->ctx->smem_optin;
@@ -234,11 +239,27 @@ fbp_status plan_config(fbp_batch* b, int cfg, cudaStream_t s) {
                                  cudaMemcpyHostToDevice, s));
     // Resident CTAs of each group (outside any capture), capped by its items.
     for (auto& g : b->groups) {
-        BatchLaunch l{b->d_params, g.d_items, g.nitems, nullptr, g.smem, g.path, g.bounce, g.clamp, cfg,
+        BatchLaunch l{b->d_params, g.d_items, g.nitems, nullptr, nullptr, g.smem, g.path, g.bounce, g.clamp, cfg,
                       (size_t)b->ctx->smem_optin};
         int occ = 0;
         FBP_TRY(prepare_any(l, &occ));
         g.ctas = (int)std::min<uint64_t>((uint64_t)std::max(1, occ) * b->ctx->sm_count, g.nitems);
+    }
+    // The chains' totals (cfg 0 only): a slice per resident CTA of every group.
+    const size_t slice = cfg == 0 ? (size_t)2 * tc.kv * 32 * tc.wy * tc.wz : 0;
+    size_t totals = 0;
+    for (const auto& g : b->groups) totals += slice * g.ctas;
+    if (totals > b->totals_cap) {
+        if (b->d_totals) FBP_TRY_CUDA(cudaFree(b->d_totals));
+        b->d_totals = nullptr;
+        b->totals_cap = 0;
+        FBP_TRY_CUDA(cudaMalloc(&b->d_totals, totals * sizeof(float)));
+        b->totals_cap = totals;
+    }
+    totals = 0;
+    for (auto& g : b->groups) {
+        g.d_totals = b->d_totals + totals;
+        totals += slice * g.ctas;
     }
     // Side streams and events for the groups after the first.
     if (!b->fork) FBP_TRY_CUDA(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
@@ -270,7 +291,7 @@ fbp_status enqueue_run(fbp_batch* b, cudaStream_t s) {
     }
     for (size_t gi = 0; gi < ng; ++gi) {
         const auto& g = b->groups[gi];
-        BatchLaunch l{b->d_params, g.d_items, g.nitems, b->d_counters + gi, g.smem, g.path, g.bounce, g.clamp, b->cfg,
+        BatchLaunch l{b->d_params, g.d_items, g.nitems, b->d_counters + gi, g.d_totals, g.smem, g.path, g.bounce, g.clamp, b->cfg,
                       (size_t)b->ctx->smem_optin};
         FBP_TRY(launch_any(b->ctx, l, g.ctas, gi == 0 ? s : b->side[gi - 1]));
     }
@@ -299,6 +320,7 @@ extern "C" fbp_status fbp_batch_destroy(fbp_batch* b) {
         cudaFree(b->d_params);
         cudaFree(b->d_items);
         cudaFree(b->d_counters);
+        cudaFree(b->d_totals);
         for (cudaStream_t st : b->side) cudaStreamDestroy(st);
         for (cudaEvent_t ev : b->join) cudaEventDestroy(ev);
         if (b->fork) cudaEventDestroy(b->fork);

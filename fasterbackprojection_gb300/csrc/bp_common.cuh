@@ -11,6 +11,60 @@ __device__ __forceinline__ void cp_async_16(void* smem_dst, const void* gmem_src
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem_src) : "memory");
 }
+// Bulk copy of `bytes` (a multiple of 16, both addresses 16-byte aligned) from
+// global to shared memory, completing on the mbarrier at shared address `bar`.
+__device__ __forceinline__ void bulk_load(uint32_t smem_dst, const void* gmem_src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_dst),
+                 "l"(gmem_src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_inval(uint32_t bar) {
+    asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// Waits for the phase with this parity, at most kWaitLimit polls (each
+// suspends for a while in hardware; the longest wait in earnest is one
+// stage); false when they ran out.
+constexpr uint32_t kWaitLimit = 1u << 22;
+__device__ __forceinline__ bool mbar_wait_parity(uint32_t bar, uint32_t parity) {
+    for (uint32_t i = 0; i < kWaitLimit; ++i) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}\n"
+            : "=r"(done)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+
+// ---------------------------------------------------------------- cluster --
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// Shared address of this CTA's `addr` in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ float cluster_load(uint32_t addr) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
+}
+
 // One FP32 element of shared memory at a shared-state-space byte address.
 __device__ __forceinline__ float lds_f32(uint32_t addr) {
     float v;
@@ -70,23 +124,26 @@ struct ConfocalGatherParams {
     float t0, dt;
     uint32_t row_pitch;  // elements per padded row
     uint32_t slot_w;     // window width in elements (the sentinel zero sits at slot_w)
-    int ch;              // scan points per pipeline stage (<= 32)
+    int ch;              // scan points per window stage (a power of two <= 32)
+    uint32_t chains;     // contiguous ranges of scan-point groups with compensated sums of their own
     const void* rows;    // [L][row_pitch] FP32
     SampleParams smp;    // used by the sampled (MIS) variant only
     float vs[3];         // voxel size (the voxel-scattering variant's extent)
     int exact_weights;   // 1: every weight by its own rcp.approx (FBP_WEIGHTS_REFERENCE)
     int scat_exact;      // voxel scattering: every walk is exactly the unrolled steps long (no tail loop)
 
-    // Per scan point of a stage, in shared memory: (x, y, z, bounce), (bias,
-    // slot address), the sample weight, three planning ints, and the packed
-    // broadcast copies the pair loop reads as 64-bit register pairs:
-    // (x, x, y, y), (z, z, bias, bias), (bounce, bounce, weight, weight).
-    static constexpr int kPackedGeo = 3;
-    // Bytes of per-chunk metadata in front of the window slots (16-byte aligned).
-    __host__ __device__ static constexpr size_t meta_bytes(int ch) {
-        return ((size_t)2 * ch * (sizeof(float4) * (1 + kPackedGeo) + sizeof(int2) + sizeof(float) + 3 * sizeof(int)) +
-                2 * sizeof(int) + 15) &
-               ~size_t(15);
+    // Shared memory in front of the windows: the pipeline's barriers, then per
+    // scan point of kPlanBufs groups: (x, y, z, bounce), (bias, bias, slot
+    // address), the x differences to the tile's kv columns, the window's source
+    // and length, the sample weight; two words per group.
+    static constexpr int kGroup = 32;
+    static constexpr int kWindowBufs = 2;  // stages of windows
+    static constexpr int kPlanBufs = 4;    // groups of plans
+    __host__ __device__ static constexpr size_t meta_bytes(int kv) {
+        return 64 +
+               (size_t)kPlanBufs * kGroup * (sizeof(float4) + sizeof(int4) + (kv + 1) * sizeof(float) + sizeof(void*) +
+                                             sizeof(int)) +
+               (size_t)kPlanBufs * sizeof(int2);
     }
 };
 
@@ -109,7 +166,12 @@ struct WindowPlan {
 };
 fbp_status plan_window(const fbp_context* ctx, double ex, double ey, double ez, double time_step, uint32_t T, int align,
                        size_t elem_bytes, size_t meta_bytes, WindowPlan* out, const char* who,
-                       double extra_path = 0.0);
+                       double extra_path = 0.0, int ctas_per_sm = 1, int window_bufs = 2);
+// The confocal gather's chains for a volume and a capture (of the whole
+// volume, whatever part of it a launch computes, so that slabs and batches sum
+// like the single call).
+uint32_t gather_chains(const fbp_context* ctx, const fbp_recon_info& in, size_t smem);
+constexpr int kGatherCtasPerSm = 3;  // 256 threads of 80 registers
 
 // The confocal gather over all scan points (smp == nullptr) or over K sampled
 // scan points per tile (the unbiased MIS estimator).

@@ -21,6 +21,7 @@
 #include "fbp_internal.cuh"
 #include "bp_common.cuh"
 #include "bp_gather.cuh"
+#include "confocal_launch.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -145,62 +146,6 @@ fbp_status prepare_rows(fbp_context* ctx, const void* cube, int layout, uint32_t
     return prepare_rows_into<S>(ctx, cube, layout, L, T, pitch, *rows_out, stream);
 }
 
-// Voxels per thread along x: 16 for the full gather (the scan point's
-// geometry and the stage's bookkeeping amortised over more pairs: 2.67e12 ->
-// 2.74e12 pairs/s at 256^3), 8 for the sampled gather (its tiles are the MIS
-// sampling tiles) and the voxel-scattering walk.
-constexpr int kKV = 8, kKVFull = 16, kWY = 2, kWZ = 4;
-
-template <typename S, int PATH, bool BOUNCE, bool SAMPLED, bool CLAMP, int KV = SAMPLED ? kKV : kKVFull>
-fbp_status go_confocal(fbp_context* ctx, const ConfocalGatherParams& p, dim3 grid, size_t smem, cudaStream_t stream) {
-    auto kernel = confocal_gather_kernel<S, KV, kWY, kWZ, PATH, BOUNCE, SAMPLED, CLAMP>;
-    FBP_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<grid, 32 * kWY * kWZ, smem, stream>>>(p);
-    FBP_CHECK_LAUNCH(ctx, "confocal_gather_kernel");
-    return FBP_OK;
-}
-
-template <typename S, bool SAMPLED>
-fbp_status dispatch_confocal(fbp_context* ctx, const ConfocalGatherParams& p, dim3 grid, size_t smem,
-                             cudaStream_t stream, bool bounce, float t0, bool capped) {
-    if (t0 > 0.f) {
-        if (bounce) return go_confocal<S, PATH_EXACT, true, SAMPLED, true>(ctx, p, grid, smem, stream);
-        return go_confocal<S, PATH_EXACT, false, SAMPLED, true>(ctx, p, grid, smem, stream);
-    }
-    if (!bounce && t0 == 0.f) {
-        if (capped) return go_confocal<S, PATH_2D, false, SAMPLED, true>(ctx, p, grid, smem, stream);
-        return go_confocal<S, PATH_2D, false, SAMPLED, false>(ctx, p, grid, smem, stream);
-    }
-    if (bounce) {
-        if (capped) return go_confocal<S, PATH_FAST, true, SAMPLED, true>(ctx, p, grid, smem, stream);
-        return go_confocal<S, PATH_FAST, true, SAMPLED, false>(ctx, p, grid, smem, stream);
-    }
-    if (capped) return go_confocal<S, PATH_FAST, false, SAMPLED, true>(ctx, p, grid, smem, stream);
-    return go_confocal<S, PATH_FAST, false, SAMPLED, false>(ctx, p, grid, smem, stream);
-}
-
-// The voxel-scattering walk with unconditional unrolled steps (prefix sp),
-// clamped window index only where the window is the whole row.
-fbp_status dispatch_scatter_free(fbp_context* ctx, const ConfocalGatherParams& p, dim3 grid, size_t smem,
-                                 cudaStream_t stream, int sp, bool bounce, bool capped) {
-    constexpr int F = PATH_SCATTER + kScatterForms;
-    switch ((sp - 2) + (bounce ? 4 : 0) + (capped ? 8 : 0)) {
-        case 0: return go_confocal<float, F, false, false, false, kKV>(ctx, p, grid, smem, stream);
-        case 1: return go_confocal<float, F + 1, false, false, false, kKV>(ctx, p, grid, smem, stream);
-        case 2: return go_confocal<float, F + 2, false, false, false, kKV>(ctx, p, grid, smem, stream);
-        case 4: return go_confocal<float, F, true, false, false, kKV>(ctx, p, grid, smem, stream);
-        case 5: return go_confocal<float, F + 1, true, false, false, kKV>(ctx, p, grid, smem, stream);
-        case 6: return go_confocal<float, F + 2, true, false, false, kKV>(ctx, p, grid, smem, stream);
-        case 8: return go_confocal<float, F, false, false, true, kKV>(ctx, p, grid, smem, stream);
-        case 9: return go_confocal<float, F + 1, false, false, true, kKV>(ctx, p, grid, smem, stream);
-        case 10: return go_confocal<float, F + 2, false, false, true, kKV>(ctx, p, grid, smem, stream);
-        case 12: return go_confocal<float, F, true, false, true, kKV>(ctx, p, grid, smem, stream);
-        case 13: return go_confocal<float, F + 1, true, false, true, kKV>(ctx, p, grid, smem, stream);
-        case 14: return go_confocal<float, F + 2, true, false, true, kKV>(ctx, p, grid, smem, stream);
-        default: return set_error(FBP_ERR_INTERNAL, "voxel scattering: no kernel for this step prefix");
-    }
-}
-
 // Depth slices [z_begin, z_end) of the volume (the whole volume by default)
 // into `volume` ([z_end - z_begin][Vy][Vx]).  The window plan and the voxel
 // tables are those of the whole volume, so with z_begin a multiple of the
@@ -216,7 +161,7 @@ fbp_status launch_confocal(fbp_context* ctx, const fbp_recon_info& in, const voi
     constexpr int ALIGN = 4;  // FP32 rows
 
     // World extents of the largest tile (clamped to the volume).
-    const uint32_t kv = (smp || scatter) ? kKV : kKVFull;
+    const uint32_t kv = smp ? kKV : kKVFull;
     const double ex = (double)std::min<uint32_t>(kv, Vx) * std::fabs(in.voxel_size[0]);
     const double ey = (double)std::min<uint32_t>(4 * kWZ, Vz) * std::fabs(in.voxel_size[1]);
     const double ez = (double)std::min<uint32_t>(8 * kWY, Vy) * std::fabs(in.voxel_size[2]);
@@ -230,9 +175,11 @@ fbp_status launch_confocal(fbp_context* ctx, const fbp_recon_info& in, const voi
                                    (double)in.voxel_size[2] * in.voxel_size[2]);
     const double extra = scatter ? 1.52 * vdiag + 2.0 * std::fabs((double)in.time_step) : 0.0;
     FBP_TRY(plan_window(ctx, ex, ey, ez, in.time_step, T, ALIGN, sizeof(float),
-                        ConfocalGatherParams::meta_bytes(32) + (smp ? kSampledStaticSmem : 0) +
+                        ConfocalGatherParams::meta_bytes((int)kv) + (smp ? kSampledStaticSmem : 0) +
                             kahan_smem_bytes((int)kv, 32 * kWY * kWZ) + 16,
-                        &wp, "fbp_backproject_confocal", extra));
+                        &wp, "fbp_backproject_confocal", extra,
+                        gather_ctas(32 * kWY * kWZ),
+                        ConfocalGatherParams::kWindowBufs));
     if (smp) wp.smem -= kSampledStaticSmem;
 
     float* rows = nullptr;
@@ -250,6 +197,7 @@ fbp_status launch_confocal(fbp_context* ctx, const fbp_recon_info& in, const voi
     p.row_pitch = wp.pitch;
     p.slot_w = wp.slot_w;
     p.ch = wp.ch;
+    p.chains = smp ? 1 : gather_chains(ctx, in, wp.smem);
     for (int k = 0; k < 3; ++k) p.vs[k] = in.voxel_size[k];
     p.exact_weights = ctx->weight_mode == FBP_WEIGHTS_REFERENCE;
     if (smp) p.smp = *smp;
@@ -268,22 +216,46 @@ fbp_status launch_confocal(fbp_context* ctx, const fbp_recon_info& in, const voi
         const bool free_walk = (sp - 1) * step + 1e-4 < vdiag;
         // ... and where none takes more (sp steps already pass the far end).
         p.scat_exact = free_walk && sp * step > vdiag + 1e-4;
-        switch ((sp - 2) + (free_walk ? kScatterForms : 0) + (bounce ? 8 : 0)) {
-            case 0: return go_confocal<float, PATH_SCATTER, false, false, true, kKV>(ctx, p, grid, wp.smem, stream);
-            case 1: return go_confocal<float, PATH_SCATTER + 1, false, false, true, kKV>(ctx, p, grid, wp.smem, stream);
-            case 2: return go_confocal<float, PATH_SCATTER + 2, false, false, true, kKV>(ctx, p, grid, wp.smem, stream);
-            case 8: return go_confocal<float, PATH_SCATTER, true, false, true, kKV>(ctx, p, grid, wp.smem, stream);
-            case 9: return go_confocal<float, PATH_SCATTER + 1, true, false, true, kKV>(ctx, p, grid, wp.smem, stream);
-            case 10: return go_confocal<float, PATH_SCATTER + 2, true, false, true, kKV>(ctx, p, grid, wp.smem, stream);
-            default: break;
-        }
-        return dispatch_scatter_free(ctx, p, grid, wp.smem, stream, sp, bounce, wp.capped);
+        if (p.chains > 1) return gather_scatter_cluster(ctx, p, grid, wp.smem, stream, sp, free_walk, bounce, wp.capped);
+        return gather_scatter(ctx, p, grid, wp.smem, stream, sp, free_walk, bounce, wp.capped);
     }
-    if (smp) return dispatch_confocal<float, true>(ctx, p, grid, wp.smem, stream, bounce, in.time_offset, wp.capped);
-    return dispatch_confocal<float, false>(ctx, p, grid, wp.smem, stream, bounce, in.time_offset, wp.capped);
+    if (smp) return gather_sampled(ctx, p, grid, wp.smem, stream, bounce, in.time_offset, wp.capped);
+    if (p.chains > 1) return gather_full_cluster(ctx, p, grid, wp.smem, stream, bounce, in.time_offset, wp.capped);
+    return gather_full(ctx, p, grid, wp.smem, stream, bounce, in.time_offset, wp.capped);
 }
 
 }  // namespace
+
+// Chains (CTAs per tile) of a gather: 1 where the tiles alone keep every SM
+// busy, else as many as a model of the launch asks for.  The model, in units of
+// one group of scan points at an SM's full rate: the busiest SM's CTAs, each
+// with its share of the groups and 0.3 groups of set-up, at the rate of the
+// CTAs resident together (one or two reach 0.68 and 0.88 of three), and 0.3
+// CTAs for the uneven end.  Larger clusters only where they gain 2 %: clusters
+// of 7, 8, 14 and 16 CTAs leave part of a GPC's slots empty (128^2 x 1024 ->
+// 128^3: 12.2 ms with 2, 12.1 with 6, 12.9 with 8, 15.3 with 16; 14.3 with one
+// CTA per tile).  One CTA per tile against this rule: 32^2 x 256 -> 32^3 291
+// -> 48 us (12 chains), 64^2 x 512 -> 64^3 1133 -> 482 us (6).
+uint32_t gather_chains(const fbp_context* ctx, const fbp_recon_info& in, size_t smem) {
+    const uint64_t tiles = (uint64_t)cdiv(in.voxel_res[0], kKVFull) * cdiv(in.voxel_res[1], 8 * kWY) *
+                           cdiv(in.voxel_res[2], 4 * kWZ);
+    const uint32_t groups = cdiv(in.num_laser_targets, ConfocalGatherParams::kGroup);
+    const int occ = (int)std::min<size_t>(kGatherCtasPerSm, std::max<size_t>(1, kSmSharedBytes / (smem + kCtaReservedShared)));
+    constexpr double kRate[kGatherCtasPerSm] = {0.68, 0.88, 1.0};
+    uint32_t best = 1;
+    double best_t = 0.0;
+    for (uint32_t c : {1u, 2u, 4u, 6u, 12u}) {
+        if (c > groups) break;
+        const uint64_t per_sm = cdiv(tiles * c, (uint64_t)ctx->sm_count);
+        const double rate = kRate[std::min<uint64_t>(per_sm, (uint64_t)occ) - 1] / kRate[occ - 1];
+        const double t = ((double)per_sm + 0.3) * ((double)groups / c + 0.3) / rate * (c == 12 ? 1.05 : 1.0);
+        if (c == 1 || t < 0.98 * best_t) {
+            best = c;
+            best_t = t;
+        }
+    }
+    return best;
+}
 
 // Tile grid of the confocal gather (also the MIS sampling tiles).
 void confocal_tile_grid(const fbp_recon_info& in, uint32_t out[3]) {
@@ -353,7 +325,8 @@ fbp_status build_tables(fbp_context* ctx, const fbp_recon_info& in, const float*
 }
 
 fbp_status plan_window(const fbp_context* ctx, double ex, double ey, double ez, double time_step, uint32_t T, int align,
-                       size_t elem_bytes, size_t meta_bytes, WindowPlan* out, const char* who, double extra_path) {
+                       size_t elem_bytes, size_t meta_bytes, WindowPlan* out, const char* who, double extra_path,
+                       int ctas_per_sm, int window_bufs) {
     const double diag = std::sqrt(ex * ex + ey * ey + ez * ez);
     // Round trip across the tile (plus any extra path range), a 2-bin margin
     // on each side, alignment slack.
@@ -365,10 +338,21 @@ fbp_status plan_window(const fbp_context* ctx, double ex, double ey, double ez, 
     out->slot_w = slot_w;
     out->capped = slot_w == cap;
     out->pitch = t_round + slot_w;
-    const size_t per_stage = (size_t)2 * (slot_w + align) * elem_bytes;  // double-buffered, per scan point
+    const size_t per_stage = (size_t)window_bufs * (slot_w + align) * elem_bytes;  // per scan point of a stage
     const size_t zero_slot = (size_t)(slot_w + align) * elem_bytes;
-    int ch = 32;
-    while (ch > 1 && meta_bytes + (size_t)ch * per_stage + zero_slot > (size_t)ctx->smem_optin) ch >>= 1;
+    // Points per stage: 32, halved down to 8 where that lets one more CTA share
+    // the SM (at 128^2 x 1024 -> 128^3 a stage of 16 keeps three CTAs instead
+    // of two), below 8 only where not even one CTA fits otherwise.
+    int ch = 0;
+    for (int n = ctas_per_sm; n >= 2 && !ch; --n) {
+        const size_t room = kSmSharedBytes / n - kCtaReservedShared;
+        for (int c = 32; c >= 8 && !ch; c >>= 1)
+            if (meta_bytes + (size_t)c * per_stage + zero_slot <= room) ch = c;
+    }
+    if (!ch) {
+        ch = 32;
+        while (ch > 1 && meta_bytes + (size_t)ch * per_stage + zero_slot > (size_t)ctx->smem_optin) ch >>= 1;
+    }
     if (meta_bytes + (size_t)ch * per_stage + zero_slot > (size_t)ctx->smem_optin)
         return set_error(FBP_ERR_UNSUPPORTED, std::string(who) + ": time-bin window too large for shared memory");
     out->ch = ch;

@@ -11,10 +11,13 @@ namespace fbp {
 //               x = d * (2 rcp(dt)) and the weight is rcp(d^2) = 4 rcp(dist^2);
 //               the stage's partial sum is scaled by 1/4 (exact).
 //   PATH_FAST   time_offset <= 0 (every path >= 0): dist = fma(d, 2, -t0) [+ bounce].
-//   PATH_EXACT  time_offset > 0: negative paths possible, bin by conversion.
-// In PATH_2D / PATH_FAST the bin is floor(x) - a via a round-toward-zero add of
-// 2^23 - a; without CLAMP the window planner guarantees every bin of the tile
-// lies inside its window, so the -2^23 bias folds into the shared-memory base.
+//   PATH_EXACT  time_offset > 0: negative paths possible.  Groups with a path
+//               near or below zero take the guarded loop and bin by
+//               conversion (int() truncates towards zero); the others run
+//               PATH_FAST's arithmetic, whose floor is the same for x > 0
+//               (a conversion is a third MUFU-pipe operation per pair).
+// CLAMP: windows that are the whole row, whose bins are clamped to the slot;
+// otherwise the planner guarantees that every bin lies inside its window.
 //   PATH_SCATTER + j  the reference's ACCUMULATE_VOXEL_SCATTERING variant
 //               (transient_reconstruction.cuh:112-126): every bin of the
 //               path range dist -/+ the voxel's half diagonal, stepped by
@@ -35,42 +38,44 @@ __host__ __device__ constexpr bool is_scatter(int path) { return path >= PATH_SC
 __host__ __device__ constexpr int scatter_prefix(int path) { return (path - PATH_SCATTER) % kScatterForms + 2; }
 __host__ __device__ constexpr bool scatter_free(int path) { return path - PATH_SCATTER >= kScatterForms; }
 
-template <typename S>
-__device__ __forceinline__ float lds_elem(uint32_t addr);
-template <>
-__device__ __forceinline__ float lds_elem<float>(uint32_t addr) {
-    float v;
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
-    return v;
-}
-template <>
-__device__ __forceinline__ float lds_elem<__nv_bfloat16>(uint32_t addr) {
-    unsigned short v;
-    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
-    return __uint_as_float((uint32_t)v << 16);
-}
-template <>
-__device__ __forceinline__ float lds_elem<__half>(uint32_t addr) {
-    unsigned short v;
-    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
-    return __half2float(__ushort_as_half(v));
-}
+// What the pair loop reads of a planned scan point (broadcast shared loads).
+// dx: the x differences to the tile's KV voxel columns, as packed pairs: the
+// same for every thread, so the planner makes them once (the subtractions were
+// an eighth of the loop's issue slots).
+struct ScanPlan {
+    const float4* geo;      // (x, y, z, bounce)
+    const int4* meta;       // (bias, bias, slot address, 0); see BinIndex
+    const ulonglong2* dx;   // [KV / 4] per point
+    const float* weight;    // WEIGHTED: the sample's weight
+};
 
-template <typename S> struct ElemShift;
-template <> struct ElemShift<float> { static constexpr int value = 2; };
-template <> struct ElemShift<__nv_bfloat16> { static constexpr int value = 1; };
-template <> struct ElemShift<__half> { static constexpr int value = 1; };
+// Word of shared memory a path ratio x reads.
+//   CLAMP   floor(x) - a, clamped to the slot (bias 2^23 - a, the slot's
+//           address beside it).
+//   else    the planner guarantees a <= x < a + slot width, so the slot's word
+//           and the window start fold into one addend: x 2^-149 + word 2^-149
+//           rounded towards zero is a subnormal whose bits are the word
+//           floor(x) - a + slot; no conversion, no shift, no add.
+#define FBP_TINY __int_as_float(1)  // 2^-149
+template <bool CLAMP>
+__device__ __forceinline__ f32x2_t bin_words2(f32x2_t x, f32x2_t bias, f32x2_t tiny) {
+    return CLAMP ? add_rz2(x, bias) : fma_rz2(x, tiny, bias);
+}
+template <bool CLAMP>
+__device__ __forceinline__ float read_bin(const float* smem, float word, int slot, uint32_t slot_w) {
+    if (CLAMP) return lds_f32((uint32_t)slot + (min(__float_as_uint(word) - 0x4B000000u, slot_w) << 2));
+    return smem[__float_as_uint(word)];
+}
 
 // One staged stage of scan points against a thread's KV voxels (consecutive
 // along x, sharing the y/z offsets).
-template <typename S, int KV, int PATH, bool BOUNCE, bool CLAMP, bool SAFE, bool WEIGHTED>
-__device__ __forceinline__ void confocal_stage(const float4* __restrict__ geo, const ulonglong2* __restrict__ geo2,
-                                               const int2* __restrict__ meta, const float* __restrict__ wts, int nl, const float (&px)[KV], float py,
+template <int KV, int PATH, bool BOUNCE, bool CLAMP, bool SAFE, bool WEIGHTED>
+__device__ __forceinline__ void confocal_stage(const ScanPlan pl, const float* __restrict__ smem, int nl, float py,
                                                float pz, float neg_t0, float rcp_dt, uint32_t slot_w,
                                                float (&acc)[KV], float ext = 0.f, float step = 0.f,
                                                bool tail = true) {
-    constexpr int SH = ElemShift<S>::value;
     const float rcp2 = 2.f * rcp_dt;  // exact
+    const f32x2_t tiny = pack2(FBP_TINY, FBP_TINY);
     if constexpr (is_scatter(PATH)) {
         constexpr int SP = scatter_prefix(PATH);
         static_assert(SP >= 1 && SP <= kScatterMaxPrefix, "prefix within the step bound");
@@ -82,35 +87,41 @@ __device__ __forceinline__ void confocal_stage(const float4* __restrict__ geo, c
         // there, so a predicated step past the end only reads (the clamped
         // index keeps it inside the slot).
         for (int i = 0; i < nl; ++i) {
-            const float4 g = geo[i];
-            const int2 m = meta[i];  // (float 2^23 - a for window start bin a, slot shared address)
+            const float4 g = pl.geo[i];
+            const int4 m = pl.meta[i];
             const float bias = __int_as_float(m.x);
-            const float wl = WEIGHTED ? wts[i] : 1.f;
+            const float wl = WEIGHTED ? pl.weight[i] : 1.f;
             const float dy = sub_rn(py, g.y), dz = sub_rn(pz, g.z);
             const float dy2 = mul_rn(dy, dy);
-            auto bin_at = [&](float dd) -> uint32_t {
-                const uint32_t bits = __float_as_uint(add_rz(ref_bin_ratio(dd, rcp_dt), bias));
-                if (CLAMP) return (uint32_t)m.y + (min(bits - 0x4B000000u, slot_w) << SH);
-                return (uint32_t)m.y + (bits << SH);  // every read inside the planned window; bias folded into m.y
+            f32x2_t dxp[KV / 2];
+#pragma unroll
+            for (int j = 0; j < KV / 4; ++j) {
+                const ulonglong2 v = pl.dx[(size_t)i * (KV / 4) + j];
+                dxp[2 * j] = v.x;
+                dxp[2 * j + 1] = v.y;
+            }
+            auto bin_at = [&](float dd) -> float {
+                const float x = ref_bin_ratio(dd, rcp_dt);
+                return read_bin<CLAMP>(smem, CLAMP ? add_rz(x, bias) : fma_rz(x, FBP_TINY, bias), m.z, slot_w);
             };
             // Steps SP.. of one walk (rare: a diagonal longer than the planned steps).
             auto walk_rest = [&](float a, float dd, float dmax, float w) -> float {
                 for (int it = SP; dd < dmax && it < max_it; ++it) {
-                    float I = lds_elem<S>(bin_at(dd));
+                    float I = bin_at(dd);
                     if (WEIGHTED) I *= wl;
                     a = add_rn(a, mul_rn(I, w));
                     dd = add_rn(dd, step);
                 }
                 return a;
             };
-            if constexpr (!SAFE && KV % 2 == 0) {
+            if constexpr (!SAFE) {
                 // Voxel pairs (k, k + 1) in packed FP32 pairs, step by step.
-                const f32x2_t gxp = pack2(g.x, g.x), dy2p = pack2(dy2, dy2), dzp = pack2(dz, dz);
+                const f32x2_t dy2p = pack2(dy2, dy2), dzp = pack2(dz, dz);
                 const f32x2_t gwp = pack2(g.w, g.w), extp = pack2(ext, ext), stepp = pack2(step, step);
                 const f32x2_t rdp = pack2(rcp_dt, rcp_dt), biasp = pack2(bias, bias), wlp = pack2(wl, wl);
 #pragma unroll
                 for (int j = 0; j < KV / 2; ++j) {
-                    const f32x2_t dx = sub_rn2(pack2(px[2 * j], px[2 * j + 1]), gxp);
+                    const f32x2_t dx = dxp[j];
                     float q0, q1, s0, s1, e0, e1, h0, h1;
                     unpack2(fma_rn2(dzp, dzp, fma_rn2(dx, dx, dy2p)), q0, q1);
                     f32x2_t dist = fma_rn2(pack2(sqrt_approx(q0), sqrt_approx(q1)), pack2(2.f, 2.f),
@@ -126,11 +137,8 @@ __device__ __forceinline__ void confocal_stage(const float4* __restrict__ geo, c
                     for (int it = 0; it < SP; ++it) {
                         float d0, d1, b0, b1, p0, p1;
                         unpack2(dd, d0, d1);
-                        unpack2(add_rz2(mul_rn2(dd, rdp), biasp), b0, b1);
-                        const uint32_t i0 = CLAMP ? min(__float_as_uint(b0) - 0x4B000000u, slot_w) : __float_as_uint(b0);
-                        const uint32_t i1 = CLAMP ? min(__float_as_uint(b1) - 0x4B000000u, slot_w) : __float_as_uint(b1);
-                        f32x2_t I = pack2(lds_elem<S>((uint32_t)m.y + (i0 << SH)),
-                                          lds_elem<S>((uint32_t)m.y + (i1 << SH)));
+                        unpack2(bin_words2<CLAMP>(mul_rn2(dd, rdp), biasp, tiny), b0, b1);
+                        f32x2_t I = pack2(read_bin<CLAMP>(smem, b0, m.z, slot_w), read_bin<CLAMP>(smem, b1, m.z, slot_w));
                         if (WEIGHTED) I = mul_rn2(I, wlp);
                         unpack2(mul_rn2(I, w), p0, p1);
                         if constexpr (scatter_free(PATH)) {
@@ -157,17 +165,19 @@ __device__ __forceinline__ void confocal_stage(const float4* __restrict__ geo, c
             } else {
 #pragma unroll
                 for (int k = 0; k < KV; ++k) {
-                    const float dx = sub_rn(px[k], g.x);
+                    float dx2[2];
+                    unpack2(dxp[k / 2], dx2[0], dx2[1]);
+                    const float dx = dx2[k & 1];
                     const float d = sqrt_approx(fma_rn(dz, dz, fma_rn(dx, dx, dy2)));
                     float dist = fma_rn(d, 2.f, neg_t0);
                     if (BOUNCE) dist = add_rn(dist, g.w);
-                    const float w = SAFE ? ref_safe_rcp(mul_rn(dist, dist)) : rcp_approx(mul_rn(dist, dist));
+                    const float w = ref_safe_rcp(mul_rn(dist, dist));
                     float dd = fmaxf(0.f, sub_rn(dist, ext));
                     const float dmax = add_rn(dist, ext);
                     float a = acc[k];
 #pragma unroll
                     for (int it = 0; it < SP; ++it) {
-                        float I = lds_elem<S>(bin_at(dd));
+                        float I = bin_at(dd);
                         if (WEIGHTED) I *= wl;
                         a = add_rn_if_lt(a, mul_rn(I, w), dd, dmax);
                         dd = add_rn(dd, step);
@@ -177,95 +187,78 @@ __device__ __forceinline__ void confocal_stage(const float4* __restrict__ geo, c
             }
         }
         return;
-    }
-    if constexpr (!is_scatter(PATH) && !SAFE && KV % 4 == 0) {
+    } else if constexpr (!SAFE) {
         // Voxel pairs (k, k + 1) in packed FP32 pairs: the bins are the scalar
-        // loop's operations, bit for bit, at half the FP32 instructions.
+        // loop's operations, bit for bit, in half the instructions.  A packed
+        // instruction holds the issue port for two cycles, and the port is what
+        // bounds this loop (issue 66 % + second cycles 34 % of all cycles
+        // before the differences and the bin words left it; MUFU pipe 76 %).
         //
         // Weights by simultaneous inversion (P. L. Montgomery, "Speeding the
         // Pollard and elliptic curve methods of factorization", Math. Comp. 48
-        // (1987), section 10.3.1): the squared paths s_0, s_1 of two packed
-        // pairs share ONE reciprocal per lane, r = 1 / (s_0 s_1), and
-        // 1 / s_0 = r s_1, 1 / s_1 = r s_0 (G = 4 pairs would use a product
-        // tree: 1 / s_0 = (r s_2 s_3) s_1).  That is one rcp.approx per two
-        // voxels instead of one per voxel: the bin's sqrt.approx and the
-        // weight's rcp.approx were the only MUFU operations per pair, and the
-        // MUFU pipe bounded the loop.  Each weight carries at most ~2 ulp (the
-        // rounded product, the approximate reciprocal, one rounded multiply)
-        // instead of rcp.approx's own ~1 ulp.  G = 2 measured faster than
-        // G = 4 (whose extra multiplies load the FMA pipe, which the packed
-        // pairs already keep busy).  Stages where a product could leave the
-        // normal FP32 range (paths under 3.5 mm or over 10 km) take the scalar
-        // loop with the reference's safeRCP.
-        constexpr int G = 2;
-        f32x2_t pxp[KV / 2], accp[KV / 2];
+        // (1987), section 10.3.1): the squared paths of G packed pairs share
+        // ONE reciprocal per lane (G = 2: r = 1 / (s_0 s_1), 1 / s_0 = r s_1;
+        // G = 4: r = 1 / (s_0 s_1 s_2 s_3), 1 / s_0 = (r s_2 s_3) s_1).
+        // Without bounces and time offset (PATH_2D) the squared distance is
+        // there already as the root's argument, which saves the product and
+        // the root's error and pays for G = 4's two more roundings: 8.9e-8 rms
+        // against 64 bits, 1.06e-7 with G = 2 and d * d; 1.25 MUFU operations
+        // per voxel.  The other paths have to square the path and keep G = 2
+        // (1.05e-7 rms; G = 4 would have 1.11e-7).  Groups with a path under
+        // 3.5 mm or over 10 km, whose products could leave the normal FP32
+        // range, take the scalar loop with the reference's safeRCP.
+        constexpr int G = PATH == PATH_2D && KV % 8 == 0 ? 4 : 2;
+        f32x2_t accp[KV / 2];
 #pragma unroll
-        for (int j = 0; j < KV / 2; ++j) {
-            pxp[j] = pack2(px[2 * j], px[2 * j + 1]);
-            accp[j] = pack2(acc[2 * j], acc[2 * j + 1]);
-        }
-        const f32x2_t pyp = pack2(py, py), pzp = pack2(pz, pz);
+        for (int j = 0; j < KV / 2; ++j) accp[j] = pack2(acc[2 * j], acc[2 * j + 1]);
         const f32x2_t rcp2p = pack2(rcp2, rcp2), rdp = pack2(rcp_dt, rcp_dt), two = pack2(2.f, 2.f);
         const f32x2_t nt0p = pack2(neg_t0, neg_t0);
-#pragma unroll 2
+#pragma unroll 4
         for (int i = 0; i < nl; ++i) {
-            // (x, x, y, y), (z, z, bias, bias), (bounce, bounce, w, w) as register pairs.
-            const ulonglong2 ga = geo2[3 * i], gb = geo2[3 * i + 1];
-            const uint32_t m_addr = (uint32_t)meta[i].y;
-            const int m_bias = meta[i].x;
-            const f32x2_t gxp = ga.x, biasp = gb.y;
-            const f32x2_t dyp = sub_rn2(pyp, ga.y), dzp = sub_rn2(pzp, gb.x);
-            const f32x2_t dy2p = mul_rn2(dyp, dyp);
-            f32x2_t gwp = 0ull, wlp = 0ull;
-            if (BOUNCE || WEIGHTED) {
-                const ulonglong2 gc = geo2[3 * i + 2];
-                gwp = gc.x;
-                wlp = gc.y;
+            const float4 g = pl.geo[i];
+            const int4 m = pl.meta[i];
+            const f32x2_t biasp = pack2(__int_as_float(m.x), __int_as_float(m.y));
+            const float dy = sub_rn(py, g.y), dz = sub_rn(pz, g.z);
+            const float dy2 = mul_rn(dy, dy);
+            const f32x2_t dy2p = pack2(dy2, dy2), dzp = pack2(dz, dz);
+            const f32x2_t gwp = pack2(g.w, g.w);
+            f32x2_t wlp = 0ull;
+            if (WEIGHTED) {
+                const float wl = pl.weight[i];
+                wlp = pack2(wl, wl);
             }
 #pragma unroll
             for (int j0 = 0; j0 < KV / 2; j0 += G) {
-                f32x2_t sq[G], Iq[G];
+                f32x2_t sq[G], Iq[G], dx[G];
+#pragma unroll
+                for (int jj = 0; jj < G; jj += 2) {
+                    const ulonglong2 v = pl.dx[(size_t)i * (KV / 4) + (j0 + jj) / 2];
+                    dx[jj] = v.x;
+                    dx[jj + 1] = v.y;
+                }
 #pragma unroll
                 for (int jj = 0; jj < G; ++jj) {
-                    const int j = j0 + jj;
-                    const f32x2_t dx = sub_rn2(pxp[j], gxp);
-                    float q0, q1;
-                    unpack2(fma_rn2(dzp, dzp, fma_rn2(dx, dx, dy2p)), q0, q1);
+                    const f32x2_t q = fma_rn2(dzp, dzp, fma_rn2(dx[jj], dx[jj], dy2p));
+                    float q0, q1, b0, b1;
+                    unpack2(q, q0, q1);
                     const f32x2_t d = pack2(sqrt_approx(q0), sqrt_approx(q1));
                     f32x2_t x;
                     if (PATH == PATH_2D) {
                         x = mul_rn2(d, rcp2p);
-                        sq[jj] = mul_rn2(d, d);
+                        sq[jj] = q;
                     } else {
                         f32x2_t dist = fma_rn2(d, two, nt0p);
                         if (BOUNCE) dist = add_rn2(dist, gwp);
                         x = mul_rn2(dist, rdp);
                         sq[jj] = mul_rn2(dist, dist);
                     }
-                    uint32_t a0, a1;
-                    if (PATH == PATH_EXACT) {
-                        float x0, x1;
-                        unpack2(x, x0, x1);
-                        const int b0 = __float2int_rz(x0), b1 = __float2int_rz(x1);  // static_cast<int>
-                        a0 = m_addr + (min((uint32_t)(b0 - m_bias), slot_w) << SH);
-                        a1 = m_addr + (min((uint32_t)(b1 - m_bias), slot_w) << SH);
-                    } else {
-                        float b0, b1;
-                        unpack2(add_rz2(x, biasp), b0, b1);
-                        if (CLAMP) {
-                            a0 = m_addr + (min(__float_as_uint(b0) - 0x4B000000u, slot_w) << SH);
-                            a1 = m_addr + (min(__float_as_uint(b1) - 0x4B000000u, slot_w) << SH);
-                        } else {
-                            a0 = m_addr + (__float_as_uint(b0) << SH);  // bias folded into the address
-                            a1 = m_addr + (__float_as_uint(b1) << SH);
-                        }
-                    }
-                    Iq[jj] = pack2(lds_elem<S>(a0), lds_elem<S>(a1));
+                    unpack2(bin_words2<CLAMP>(x, biasp, tiny), b0, b1);
+                    Iq[jj] = pack2(read_bin<CLAMP>(smem, b0, m.z, slot_w), read_bin<CLAMP>(smem, b1, m.z, slot_w));
                     if (WEIGHTED) Iq[jj] = mulf2(Iq[jj], wlp);
                 }
+                float m0, m1;
                 if constexpr (G == 4) {
                     const f32x2_t p01 = mul_rn2(sq[0], sq[1]), p23 = mul_rn2(sq[2], sq[3]);
-                    float m0, m1;
                     unpack2(mul_rn2(p01, p23), m0, m1);
                     const f32x2_t r = pack2(rcp_approx(m0), rcp_approx(m1));
                     const f32x2_t r01 = mul_rn2(r, p23), r23 = mul_rn2(r, p01);  // 1/(s0 s1), 1/(s2 s3)
@@ -274,7 +267,6 @@ __device__ __forceinline__ void confocal_stage(const float4* __restrict__ geo, c
                     accp[j0 + 2] = fmaf2(Iq[2], mul_rn2(r23, sq[3]), accp[j0 + 2]);
                     accp[j0 + 3] = fmaf2(Iq[3], mul_rn2(r23, sq[2]), accp[j0 + 3]);
                 } else {
-                    float m0, m1;
                     unpack2(mul_rn2(sq[0], sq[1]), m0, m1);
                     const f32x2_t r = pack2(rcp_approx(m0), rcp_approx(m1));
                     accp[j0 + 0] = fmaf2(Iq[0], mul_rn2(r, sq[1]), accp[j0 + 0]);
@@ -284,79 +276,81 @@ __device__ __forceinline__ void confocal_stage(const float4* __restrict__ geo, c
         }
 #pragma unroll
         for (int j = 0; j < KV / 2; ++j) unpack2(accp[j], acc[2 * j], acc[2 * j + 1]);
-        return;
-    }
+    } else {
+        // Guarded: every weight by the reference's own safeRCP, and with
+        // PATH_EXACT the bin by conversion, like the reference's static_cast.
 #pragma unroll 2
-    for (int i = 0; i < nl; ++i) {
-        const float4 g = geo[i];
-        const int2 m = meta[i];  // (bin bias: float 2^23 - a, or a; slot shared address)
-        const float wl = WEIGHTED ? wts[i] : 1.f;
-        const float dy = sub_rn(py, g.y), dz = sub_rn(pz, g.z);
-        const float dy2 = mul_rn(dy, dy);
+        for (int i = 0; i < nl; ++i) {
+            const float4 g = pl.geo[i];
+            const int4 m = pl.meta[i];
+            const float wl = WEIGHTED ? pl.weight[i] : 1.f;
+            const float dy = sub_rn(py, g.y), dz = sub_rn(pz, g.z);
+            const float dy2 = mul_rn(dy, dy);
 #pragma unroll
-        for (int k = 0; k < KV; ++k) {
-            const float dx = sub_rn(px[k], g.x);
-            const float d = sqrt_approx(fma_rn(dz, dz, fma_rn(dx, dx, dy2)));
-            float x, dist = 0.f;
-            if (PATH == PATH_2D && !SAFE) {
-                x = mul_rn(d, rcp2);
-            } else {
-                dist = fma_rn(d, 2.f, neg_t0);
+            for (int k = 0; k < KV; ++k) {
+                const float dx = reinterpret_cast<const float*>(pl.dx)[i * KV + k];
+                const float d = sqrt_approx(fma_rn(dz, dz, fma_rn(dx, dx, dy2)));
+                float dist = fma_rn(d, 2.f, neg_t0);
                 if (BOUNCE) dist = add_rn(dist, g.w);
-                x = ref_bin_ratio(dist, rcp_dt);
+                const float x = ref_bin_ratio(dist, rcp_dt);
+                float I;
+                if (PATH == PATH_EXACT) {
+                    I = lds_f32((uint32_t)m.z + (min((uint32_t)(__float2int_rz(x) - m.x), slot_w) << 2));
+                } else {
+                    const float bias = __int_as_float(m.x);
+                    I = read_bin<CLAMP>(smem, CLAMP ? add_rz(x, bias) : fma_rz(x, FBP_TINY, bias), m.z, slot_w);
+                }
+                if (WEIGHTED) I *= wl;
+                acc[k] = fmaf(I, ref_safe_rcp(mul_rn(dist, dist)), acc[k]);
             }
-            uint32_t addr;
-            if (PATH == PATH_EXACT) {
-                const int b = __float2int_rz(x);  // static_cast<int>, like the reference
-                addr = (uint32_t)m.y + (min((uint32_t)(b - m.x), slot_w) << SH);
-            } else {
-                const uint32_t bits = __float_as_uint(add_rz(x, __int_as_float(m.x)));
-                if (CLAMP) addr = (uint32_t)m.y + (min(bits - 0x4B000000u, slot_w) << SH);
-                else addr = (uint32_t)m.y + (bits << SH);  // bias folded into m.y
-            }
-            float I = lds_elem<S>(addr);
-            if (WEIGHTED) I *= wl;
-            float w;
-            if (PATH == PATH_2D && !SAFE) w = rcp_approx(mul_rn(d, d));
-            else w = SAFE ? ref_safe_rcp(mul_rn(dist, dist)) : rcp_approx(mul_rn(dist, dist));
-            acc[k] = fmaf(I, w, acc[k]);
         }
     }
 }
 
-// The main kernel.  One CTA of 32*WY*WZ threads owns a tile of KV (x) x 8*WY
-// (rows) x 4*WZ (depth slices) voxels; a warp covers 8 rows x 4 slices, a
-// thread KV consecutive voxels along x.  Scan points (or, SAMPLED, K scan
-// points drawn per tile) are walked in stages of up to 32: one warp plans the
-// bin windows of the stage, all threads copy them from the padded rows into
-// shared memory with cp.async (double buffered), then every thread runs the
-// pair loop against the staged windows.  FP32 partials per stage, Kahan
-// across stages.
-template <typename S, int KV, int WY, int WZ, int PATH, bool BOUNCE, bool SAMPLED, bool CLAMP>
+// The main kernel.  One CTA of 32*WY*WZ threads (or a cluster of CS of them)
+// owns a tile of KV (x) x 8*WY (rows) x 4*WZ (depth slices) voxels; a warp
+// covers 8 rows x 4 slices, a thread KV consecutive voxels along x.  Scan
+// points (or, SAMPLED, K scan points drawn per tile) are taken in groups of 32:
+// FP32 sums inside a group, a Kahan fold per group.
+//
+// Pipeline: one warp plans a group's bin windows two groups ahead (barrier
+// `plan`); the windows arrive in stages of p.ch scan points, double buffered,
+// each window one bulk copy that completes on the stage's `full` barrier; a
+// warp that is through with a stage arrives on its `empty` barrier.  The warps
+// take turns at planning and at copying, so no warp waits for another's
+// planning and no barrier spans the CTA.
+//
+// Chains: the groups are cut into p.chains contiguous ranges, each with its
+// own compensated sums; the chains' sums are folded, compensated, in order.
+// CLUSTER: one CTA of a cluster of p.chains per chain, the fold at the end
+// through distributed shared memory (every CTA folds and stores its share of
+// the tile's voxels).  Otherwise one CTA walks the chains one after the other
+// with the totals in `totals` (global, [2 KV][threads] per CTA): the same
+// operations in the same order, so the volume is the same bit for bit.
+template <int KV, int WY, int WZ, int PATH, bool BOUNCE, bool SAMPLED, bool CLAMP, bool CLUSTER>
 __device__ __forceinline__ void confocal_tile(const ConfocalGatherParams& p, uint32_t bx, uint32_t by, uint32_t bz,
-                                              unsigned long long tile_id) {
-    constexpr int NT = 32 * WY * WZ;
-    constexpr int CHMAX = 32;
-    constexpr int ALIGN = 16 / sizeof(S);  // elements per 16-byte copy
-    constexpr int SH = ElemShift<S>::value;
+                                              unsigned long long tile_id, float* totals = nullptr) {
+    constexpr int NT = 32 * WY * WZ, NW = WY * WZ;
+    constexpr int GRP = ConfocalGatherParams::kGroup;
+    constexpr int ALIGN = 4;  // floats per 16-byte copy
     constexpr int TY = 8 * WY, TZ = 4 * WZ;
-    const int CH = p.ch;
+    const uint32_t CH = p.ch;
 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const uint32_t slot_stride = p.slot_w + ALIGN;  // sentinel element(s) at slot_w
-    float4* s_geo = reinterpret_cast<float4*>(smem_raw);         // [2][CHMAX]
-    ulonglong2* s_geo2 = reinterpret_cast<ulonglong2*>(s_geo + 2 * CHMAX);  // [2][CHMAX][kPackedGeo]
-    constexpr int PG = ConfocalGatherParams::kPackedGeo;
-    int2* s_meta = reinterpret_cast<int2*>(s_geo2 + 2 * CHMAX * PG);  // [2][CHMAX]
-    int* s_cnt = reinterpret_cast<int*>(s_meta + 2 * CHMAX);     // [2][CHMAX]
-    int* s_src = s_cnt + 2 * CHMAX;                              // [2][CHMAX]
-    int* s_row = s_src + 2 * CHMAX;                              // [2][CHMAX]
-    float* s_w = reinterpret_cast<float*>(s_row + 2 * CHMAX);    // [2][CHMAX]
-    int* s_flag = reinterpret_cast<int*>(s_w + 2 * CHMAX);       // [2]
-    const size_t slots_off = ConfocalGatherParams::meta_bytes(CHMAX);
-    S* s_slots = reinterpret_cast<S*>(smem_raw + slots_off);     // [2][CH][slot_stride], then the zero slot
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem_raw);
-    const uint32_t zero_slot = 2u * CH * slot_stride;            // element index of the all-zero slot
+    constexpr uint32_t NB = ConfocalGatherParams::kWindowBufs, MB = ConfocalGatherParams::kPlanBufs;
+    const uint32_t bar_full = sbase, bar_empty = sbase + 8 * NB, bar_plan = sbase + 16 * NB;  // NB, NB and MB of 8 bytes
+    float4* s_geo = reinterpret_cast<float4*>(smem_raw + 64);            // [MB][GRP]
+    int4* s_meta = reinterpret_cast<int4*>(s_geo + MB * GRP);            // [MB][GRP]
+    ulonglong2* s_dx = reinterpret_cast<ulonglong2*>(s_meta + MB * GRP);  // [MB][GRP][KV / 4]
+    const float** s_src = reinterpret_cast<const float**>(s_dx + MB * GRP * (KV / 4));  // [MB][GRP]
+    int* s_cnt = reinterpret_cast<int*>(s_src + MB * GRP);               // [MB][GRP]
+    float* s_w = reinterpret_cast<float*>(s_cnt + MB * GRP);             // [MB][GRP]
+    int2* s_group = reinterpret_cast<int2*>(s_w + MB * GRP);             // [MB] (points kept, guarded)
+    constexpr size_t slots_off = ConfocalGatherParams::meta_bytes(KV);
+    const float* s_all = reinterpret_cast<const float*>(smem_raw);
+    float* s_slots = reinterpret_cast<float*>(smem_raw + slots_off);     // [NB][CH][slot_stride]
 
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
@@ -375,9 +369,6 @@ __device__ __forceinline__ void confocal_tile(const ConfocalGatherParams& p, uin
 
     const float py = p.ys[min(vz, p.Vz - 1)];
     const float pz = p.zs[min(vy, p.Vy - 1)];
-    float px[KV];
-#pragma unroll
-    for (int k = 0; k < KV; ++k) px[k] = p.xs[min(tx0 + k, p.Vx - 1)];
 
     const float rcp_dt = rcp_approx(p.dt);
     const float neg_t0 = -p.t0;
@@ -386,12 +377,19 @@ __device__ __forceinline__ void confocal_tile(const ConfocalGatherParams& p, uin
     const float scat_ext = is_scatter(PATH) ? mul_rn(0.5f, sqrt_approx(ref_dot3(p.vs[0], p.vs[1], p.vs[2]))) : 0.f;
     const float scat_step = is_scatter(PATH) ? add_rn(p.dt, FBP_EPS) : 0.f;
 
-    // Sentinels of every slot and the whole zero slot.
-    for (int i = tid; i < 2 * CH * ALIGN; i += NT) {
-        const int slot = i / ALIGN, e = i % ALIGN;
-        s_slots[(size_t)slot * slot_stride + p.slot_w + e] = from_f32<S>(0.f);
+    const uint32_t rank = CLUSTER ? blockIdx.x % p.chains : 0;  // this CTA's place in the cluster (along x)
+    if (tid == 0) {
+        for (uint32_t b = 0; b < NB; ++b) {
+            mbar_init(bar_full + 8 * b, 1);
+            mbar_init(bar_empty + 8 * b, NW);
+        }
+        for (uint32_t b = 0; b < MB; ++b) mbar_init(bar_plan + 8 * b, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    for (uint32_t i = tid; i < slot_stride; i += NT) s_slots[zero_slot + i] = from_f32<S>(0.f);
+
+    // Sentinel of every slot.
+    for (uint32_t i = tid; i < NB * CH * ALIGN; i += NT)
+        s_slots[(size_t)(i / ALIGN) * slot_stride + p.slot_w + i % ALIGN] = 0.f;
 
     // SAMPLE_CLUSTERS: this tile's clusters, drawn by systematic sampling from
     // its CDF (K positions (k + u) / K), duplicates merged; each chosen
@@ -450,12 +448,23 @@ __device__ __forceinline__ void confocal_tile(const ConfocalGatherParams& p, uin
             s_cw = cw;
         }
     }
-    const uint32_t nchunks = (nitems + CH - 1) / CH;
+    const uint32_t ngroups = (nitems + GRP - 1) / GRP;
+    // Chain k: groups [k ngroups / chains, (k + 1) ngroups / chains).
+    auto chain_begin = [&](uint32_t k) { return (uint32_t)((uint64_t)k * ngroups / p.chains); };
+    const uint32_t g0 = CLUSTER ? chain_begin(rank) : 0;
+    const uint32_t mine = CLUSTER ? chain_begin(rank + 1) - g0 : ngroups;  // groups of this CTA, from g0
+    const uint32_t sub = GRP / CH;                                 // stages per group
+    const uint32_t nstages = mine * sub;
+    const bool warp_ok = __any_sync(0xffffffffu, row_ok);          // the warp owns voxels of the volume
 
-    // Plan a stage: bin window of each scan point (threads < CH, all in warp 0).
-    auto plan_chunk = [&](uint32_t c, int buf) {
-        if (tid < CH) {
-            const uint32_t item = c * CH + tid;
+    // Plan this CTA's group gi (one warp): bin window of each scan point.  Its
+    // buffer held group gi - MB, which every warp is past: this runs once the
+    // first stage of group gi - 2 is full, so once all were through with a
+    // stage of group gi - 3 or, with one stage per group, all of gi - 4.
+    auto plan_group = [&](uint32_t gi) {
+        const uint32_t gb = (gi % MB) * GRP;
+        {
+            const uint32_t item = (g0 + gi) * GRP + lane;
             uint32_t l = item;
             float wgt = 1.f;
             if (SAMPLED && item < nitems) {
@@ -483,14 +492,11 @@ __device__ __forceinline__ void confocal_tile(const ConfocalGatherParams& p, uin
                 if (p.smp.mode != SAMPLE_CLUSTERS) wgt = pl > 0.f ? 1.f / ((float)nitems * pl) : 0.f;
             }
             float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
-            int cnt = 0, src = 0, near = 0, a = 0;
+            int cnt = 0, near = 0, a = 0;
             bool skip = true;
-            // A point of a ragged edge cluster that lies outside the scan grid:
-            // planned with scan point 0's geometry (finite paths and weights)
-            // and read from the zero slot.
-            const bool ragged = item < nitems && l >= p.L;
-            if (item < nitems) {
-                g = p.scan[ragged ? 0u : l];
+            // l >= L: a point of a ragged edge cluster, outside the scan grid.
+            if (item < nitems && l < p.L) {
+                g = p.scan[l];
                 // Nearest and farthest voxel-centre distance of the tile.
                 const float cx = fminf(fmaxf(g.x, bx0), bx1), cy = fminf(fmaxf(g.y, by0), by1),
                             cz = fminf(fmaxf(g.z, bz0), bz1);
@@ -528,78 +534,75 @@ __device__ __forceinline__ void confocal_tile(const ConfocalGatherParams& p, uin
                             if (min(bhi + 1, (int)p.T) - a > (int)p.slot_w) atomicExch(p.status, (int)FBP_ERR_DEVICE);
                             cnt = (int)p.slot_w;
                         } else {
-                            // The planner's span bound failed: read zeros, report.
+                            // The planner's span bound failed: skip, report.
                             atomicExch(p.status, (int)FBP_ERR_DEVICE);
                             skip = true;
                             cnt = 0;
                         }
                     }
-                    src = a;
-                }
-                if (ragged) {
-                    skip = true;
-                    cnt = 0;
-                    wgt = 0.f;
                 }
             }
-            // Slot of this scan point (or the zero slot) as a shared address.
-            const uint32_t slot_elem = skip ? zero_slot : (uint32_t)(buf * CH + tid) * slot_stride;
-            uint32_t saddr = sbase + (uint32_t)slots_off + (slot_elem << SH);
-            int bias;
-            if (PATH == PATH_EXACT) {
-                bias = a;
-            } else {
-                bias = __float_as_int((float)(8388608 - a));
-                if (!CLAMP) saddr -= (0x4B000000u << SH);
+            // Points with nothing to read (also those with a NaN path) drop out;
+            // the others keep their order.
+            const unsigned kept = __ballot_sync(0xffffffffu, !skip);
+            const uint32_t pos = __popc(kept & ((1u << lane) - 1u));
+            const bool guarded = __any_sync(0xffffffffu, near && !skip) || p.exact_weights;
+            if (!skip) {
+                const uint32_t st = gi * sub + pos / CH;
+                const uint32_t slot_elem = ((st % NB) * CH + pos % CH) * slot_stride;
+                const int word = (int)(slots_off / 4 + slot_elem) - a;  // shared-memory word of bin 0
+                int bias;
+                if (PATH == PATH_EXACT && guarded) bias = a;
+                else if (CLAMP) bias = __float_as_int((float)(8388608 - a));
+                else bias = word >= 0 ? word : (int)(0x80000000u | (uint32_t)-word);  // word 2^-149
+                s_geo[gb + pos] = g;
+                s_meta[gb + pos] = make_int4(bias, bias, (int)(sbase + (uint32_t)slots_off + (slot_elem << 2)), 0);
+                float* dx = reinterpret_cast<float*>(s_dx + (gb + pos) * (KV / 4));
+#pragma unroll
+                for (int k = 0; k < KV; ++k) dx[k] = sub_rn(p.xs[min(tx0 + k, p.Vx - 1)], g.x);
+                s_cnt[gb + pos] = cnt;
+                s_src[gb + pos] = static_cast<const float*>(p.rows) + (size_t)l * p.row_pitch + a;
+                s_w[gb + pos] = wgt;
             }
-            if (item >= nitems) {
-                // Beyond the last scan point: x + 0 < 2^23 lands on the sentinel
-                // (CLAMP) or, unclamped, reads the zero slot at index 0.
-                bias = PATH == PATH_EXACT ? 0x40000000 : 0;
-                saddr = sbase + (uint32_t)slots_off + (zero_slot << SH);
-                if (!CLAMP && PATH != PATH_EXACT) saddr -= (__float_as_uint(0.f) << SH);
-                g = make_float4(3.0e18f, 3.0e18f, 3.0e18f, 0.f);  // far away: x is huge
-                wgt = 0.f;
-            }
-            s_geo[buf * CHMAX + tid] = g;
-            {
-                ulonglong2* g2 = s_geo2 + (buf * CHMAX + tid) * PG;
-                const float bf = __int_as_float(bias);
-                g2[0] = make_ulonglong2(pack2(g.x, g.x), pack2(g.y, g.y));
-                g2[1] = make_ulonglong2(pack2(g.z, g.z), pack2(bf, bf));
-                g2[2] = make_ulonglong2(pack2(g.w, g.w), pack2(wgt, wgt));
-            }
-            s_meta[buf * CHMAX + tid] = make_int2(bias, (int)saddr);
-            s_cnt[buf * CHMAX + tid] = cnt;
-            s_src[buf * CHMAX + tid] = src;
-            s_row[buf * CHMAX + tid] = ragged ? 0 : (int)l;
-            s_w[buf * CHMAX + tid] = wgt;
-            const unsigned any_near = __ballot_sync(CH >= 32 ? 0xffffffffu : ((1u << CH) - 1u), near);
-            if (tid == 0) s_flag[buf] = any_near != 0;
+            if (lane == 0) s_group[gi % MB] = make_int2(__popc(kept), guarded);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_plan + 8 * (gi % MB));
         }
     };
 
-    // Copy a stage's windows (all threads).
-    auto copy_chunk = [&](int buf) {
-        const uint32_t vecs_per_slot = p.slot_w / ALIGN;
-        for (uint32_t i = tid; i < CH * vecs_per_slot; i += NT) {
-            const uint32_t s = i / vecs_per_slot, j = i - s * vecs_per_slot;
-            if ((int)(j * ALIGN) < s_cnt[buf * CHMAX + s]) {
-                const uint32_t l = (uint32_t)s_row[buf * CHMAX + s];
-                const S* src = static_cast<const S*>(p.rows) + (size_t)l * p.row_pitch + s_src[buf * CHMAX + s] + j * ALIGN;
-                S* dst = s_slots + (size_t)(buf * CH + s) * slot_stride + j * ALIGN;
-                cp_async_16(dst, src);
-            }
+    // A wait that ran out of polls (status FBP_ERR_TIMEOUT): the warp keeps
+    // walking the barriers of the cluster but touches nothing else.
+    bool dead = false;
+    auto wait = [&](uint32_t bar, uint32_t parity) {
+        if (!dead && !mbar_wait_parity(bar, parity)) {
+            dead = true;
+            if (lane == 0) atomicExch(p.status, (int)FBP_ERR_TIMEOUT);
         }
-        cp_async_commit();
+    };
+
+    // Fill stage st (one warp): one bulk copy per window.
+    auto produce = [&](uint32_t st) {
+        const uint32_t buf = st % NB, gi = st / sub, first = (st % sub) * CH;
+        wait(bar_plan + 8 * (gi % MB), (gi / MB) & 1);
+        if (st >= NB) wait(bar_empty + 8 * buf, (st / NB - 1) & 1);
+        if (dead) return;
+        const uint32_t gb = (gi % MB) * GRP, n = (uint32_t)s_group[gi % MB].x;
+        const uint32_t bytes = lane - first < CH && (uint32_t)lane < n ? (uint32_t)s_cnt[gb + lane] * 4u : 0u;
+        const uint32_t total = __reduce_add_sync(0xffffffffu, bytes);
+        if (lane == 0) mbar_arrive_expect_tx(bar_full + 8 * buf, total);
+        __syncwarp();
+        if (bytes)
+            bulk_load(sbase + (uint32_t)slots_off + (((buf * CH + lane - first) * slot_stride) << 2), s_src[gb + lane],
+                      bytes, bar_full + 8 * buf);
     };
 
     // Compensated sums: in registers, or (16 voxels per thread) in shared
     // memory behind the zero slot, [2 KV][NT] so a warp's accesses are
     // consecutive words.
     constexpr bool KSMEM = kahan_smem_bytes(KV, NT) > 0;
+    static_assert(!CLUSTER || KSMEM, "the cluster folds compensated sums in shared memory");
     float* s_kahan = reinterpret_cast<float*>(
-        smem_raw + ((slots_off + (size_t)(zero_slot + slot_stride) * sizeof(S) + 15) & ~size_t(15)));
+        smem_raw + ((slots_off + (size_t)NB * CH * slot_stride * sizeof(float) + 15) & ~size_t(15)));
     float acc[KV], ksum[KSMEM ? 1 : KV], kcomp[KSMEM ? 1 : KV];
 #pragma unroll
     for (int k = 0; k < KV; ++k) acc[k] = 0.f;
@@ -610,76 +613,113 @@ __device__ __forceinline__ void confocal_tile(const ConfocalGatherParams& p, uin
 #pragma unroll
         for (int k = 0; k < KV; ++k) ksum[k] = kcomp[k] = 0.f;
     }
+    // Compensated (Kahan) addition of a group's sum.
+    auto fold = [](float part, float& sum, float& comp) {
+        const float y = sub_rn(part, comp);
+        const float t = add_rn(sum, y);
+        comp = sub_rn(sub_rn(t, sum), y);
+        sum = t;
+    };
+    // A previous tile's writes to this memory before the bulk copies' writes.
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();  // barriers initialised, sentinels written
+    if (warp < 2 && (uint32_t)warp < mine) plan_group(warp);
+    if (warp == 0 && nstages > 0) produce(0);
+    uint32_t chain = 0;
 
-    if (nchunks > 0) {
-        plan_chunk(0, 0);
-        __syncthreads();
-        copy_chunk(0);
-    }
-
-    for (uint32_t c = 0; c < nchunks; ++c) {
-        const int buf = c & 1;
-        __syncthreads();  // every thread is done with stage c-1, whose buffers plan(c+1) reuses
-        if (c + 1 < nchunks) plan_chunk(c + 1, buf ^ 1);
-        __syncthreads();  // plan(c+1) visible to the copy loop
-        if (c + 1 < nchunks) {
-            copy_chunk(buf ^ 1);
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
-        __syncthreads();  // stage c's windows visible
-
-        const float4* geo = s_geo + buf * CHMAX;
-        const ulonglong2* geo2 = s_geo2 + buf * CHMAX * PG;
-        const int2* meta = s_meta + buf * CHMAX;
-        const float* wts = s_w + buf * CHMAX;
-        const bool safe = s_flag[buf] != 0 || p.exact_weights;
-        const int nl = (int)min((uint32_t)CH, nitems - c * CH);
+    for (uint32_t gi = 0; gi < mine; ++gi) {
+        const uint32_t gb = (gi % MB) * GRP;
         float scale = 1.f;
-        if (!safe) {
-            confocal_stage<S, KV, PATH, BOUNCE, CLAMP, false, SAMPLED>(geo, geo2, meta, wts, nl, px, py, pz, neg_t0, rcp_dt,
-                                                                        p.slot_w, acc, scat_ext, scat_step,
-                                                                        !p.scat_exact);
-            if (PATH == PATH_2D) scale = 0.25f;  // w was rcp(d^2) = 4 rcp(dist^2)
-        } else {
-            confocal_stage<S, KV, PATH, BOUNCE, CLAMP, true, SAMPLED>(geo, geo2, meta, wts, nl, px, py, pz, neg_t0, rcp_dt,
-                                                                       p.slot_w, acc, scat_ext, scat_step);
+        for (uint32_t h = 0; h < sub; ++h) {
+            const uint32_t st = gi * sub + h, buf = st % NB;
+            wait(bar_full + 8 * buf, (st / NB) & 1);
+            if (st + 1 < nstages && warp == (int)((st + 1) % NW)) produce(st + 1);
+            if (h == 0 && gi + 2 < mine && !dead && warp == (int)((st + NW / 2) % NW)) plan_group(gi + 2);
+            const int2 grp = s_group[gi % MB];
+            const int nl = min((int)CH, grp.x - (int)(h * CH));
+            if (warp_ok && !dead) {
+                const uint32_t o = gb + h * CH;
+                const ScanPlan plan{s_geo + o, s_meta + o, s_dx + o * (KV / 4), s_w + o};
+                if (!grp.y) {
+                    confocal_stage<KV, PATH, BOUNCE, CLAMP, false, SAMPLED>(plan, s_all, nl, py, pz, neg_t0, rcp_dt, p.slot_w,
+                                                                            acc, scat_ext, scat_step, !p.scat_exact);
+                    if (PATH == PATH_2D) scale = 0.25f;  // w was rcp(d^2) = 4 rcp(dist^2)
+                } else {
+                    confocal_stage<KV, PATH, BOUNCE, CLAMP, true, SAMPLED>(plan, s_all, nl, py, pz, neg_t0, rcp_dt, p.slot_w,
+                                                                           acc, scat_ext, scat_step);
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_empty + 8 * buf);
         }
-
-        // Compensated (Kahan) fold of this stage's partial sums.
 #pragma unroll
         for (int k = 0; k < KV; ++k) {
-            const float sk = KSMEM ? s_kahan[(2 * k) * NT + tid] : ksum[k];
-            const float ck = KSMEM ? s_kahan[(2 * k + 1) * NT + tid] : kcomp[k];
-            const float y = sub_rn(mul_rn(acc[k], scale), ck);
-            const float t = add_rn(sk, y);
-            const float c = sub_rn(sub_rn(t, sk), y);
             if constexpr (KSMEM) {
-                s_kahan[(2 * k) * NT + tid] = t;
-                s_kahan[(2 * k + 1) * NT + tid] = c;
+                float sk = s_kahan[(2 * k) * NT + tid], ck = s_kahan[(2 * k + 1) * NT + tid];
+                fold(mul_rn(acc[k], scale), sk, ck);
+                s_kahan[(2 * k) * NT + tid] = sk;
+                s_kahan[(2 * k + 1) * NT + tid] = ck;
             } else {
-                kcomp[k] = c;
-                ksum[k] = t;
+                fold(mul_rn(acc[k], scale), ksum[k], kcomp[k]);
             }
             acc[k] = 0.f;
         }
+        if constexpr (KSMEM && !CLUSTER) {
+            // The end of a chain, of several: its sums to the totals.
+            while (p.chains > 1 && chain < p.chains && gi + 1 == chain_begin(chain + 1)) {
+                for (int k = 0; k < KV; ++k) {
+                    float* t = totals + ((size_t)blockIdx.x * KV + k) * (2 * NT) + tid;
+                    float sum = chain ? t[0] : 0.f, comp = chain ? t[NT] : 0.f;
+                    fold(s_kahan[(2 * k) * NT + tid], sum, comp);
+                    fold(-s_kahan[(2 * k + 1) * NT + tid], sum, comp);
+                    t[0] = sum;
+                    t[NT] = comp;
+                    s_kahan[(2 * k) * NT + tid] = s_kahan[(2 * k + 1) * NT + tid] = 0.f;
+                }
+                ++chain;
+            }
+        }
     }
 
-    if (row_ok) {
+    if constexpr (CLUSTER) {
+        cluster_arrive();
+        cluster_wait();  // every chain's sums are in their CTA's shared memory
+        const uint32_t kb = (uint32_t)__cvta_generic_to_shared(s_kahan + tid);
+        float* out = p.volume + ((size_t)vz * p.Vy + vy) * p.Vx + tx0;
+        for (uint32_t k = rank; k < (uint32_t)KV; k += p.chains) {
+            float sum = 0.f, comp = 0.f;
+            for (uint32_t c = 0; c < p.chains; ++c) {
+                const uint32_t src = cluster_map(kb, c) + k * (2 * NT * 4u);
+                fold(cluster_load(src), sum, comp);
+                fold(-cluster_load(src + NT * 4u), sum, comp);
+            }
+            if (row_ok && tx0 + k < p.Vx) out[k] = sum;
+        }
+        cluster_arrive();
+        cluster_wait();  // the others are through with this CTA's sums
+    } else if (row_ok) {
         float* out = p.volume + ((size_t)vz * p.Vy + vy) * p.Vx + tx0;
 #pragma unroll
         for (int k = 0; k < KV; ++k)
-            if (tx0 + k < p.Vx) out[k] = KSMEM ? s_kahan[(2 * k) * NT + tid] : ksum[k];
+            if (tx0 + k < p.Vx)
+                out[k] = !KSMEM ? ksum[KSMEM ? 0 : k]
+                                : (p.chains > 1 ? totals[((size_t)blockIdx.x * KV + k) * (2 * NT) + tid] : s_kahan[(2 * k) * NT + tid]);
+    }
+    __syncthreads();  // every warp is through with the barriers
+    if (tid == 0) {   // (a persistent kernel sets them up again for its next tile)
+        for (uint32_t b = 0; b < 2 * NB + MB; ++b) mbar_inval(bar_full + 8 * b);
     }
 }
 
-template <typename S, int KV, int WY, int WZ, int PATH, bool BOUNCE, bool SAMPLED, bool CLAMP>
-__global__ void __launch_bounds__(32 * WY * WZ)
+// Registers for three CTAs of 256 threads (80 each).
+constexpr int gather_ctas(int threads) { return threads > 256 ? 1 : kGatherCtasPerSm; }
+
+template <int KV, int WY, int WZ, int PATH, bool BOUNCE, bool SAMPLED, bool CLAMP, bool CLUSTER = false>
+__global__ void __launch_bounds__(32 * WY * WZ, gather_ctas(32 * WY * WZ))
 confocal_gather_kernel(ConfocalGatherParams p) {
-    const unsigned long long tile_id =
-        ((unsigned long long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-    confocal_tile<S, KV, WY, WZ, PATH, BOUNCE, SAMPLED, CLAMP>(p, blockIdx.x, blockIdx.y, blockIdx.z, tile_id);
+    const uint32_t cs = CLUSTER ? p.chains : 1, bx = blockIdx.x / cs;
+    const unsigned long long tile_id = ((unsigned long long)blockIdx.z * gridDim.y + blockIdx.y) * (gridDim.x / cs) + bx;
+    confocal_tile<KV, WY, WZ, PATH, BOUNCE, SAMPLED, CLAMP, CLUSTER>(p, bx, blockIdx.y, blockIdx.z, tile_id);
 }
 
 // Persistent form for a batch of captures: CTAs pull (capture, tile) work items
@@ -689,10 +729,10 @@ struct BatchItem {
     uint32_t capture, bx, by, bz;
 };
 
-template <typename S, int KV, int WY, int WZ, int PATH, bool BOUNCE, bool CLAMP>
-__global__ void __launch_bounds__(32 * WY * WZ)
+template <int KV, int WY, int WZ, int PATH, bool BOUNCE, bool CLAMP>
+__global__ void __launch_bounds__(32 * WY * WZ, gather_ctas(32 * WY * WZ))
 confocal_batch_kernel(const ConfocalGatherParams* __restrict__ caps, const BatchItem* __restrict__ items,
-                      uint32_t nitems, unsigned int* __restrict__ counter) {
+                      uint32_t nitems, unsigned int* __restrict__ counter, float* __restrict__ totals) {
     __shared__ uint32_t s_item;
     for (;;) {
         __syncthreads();  // the previous tile is done with shared memory and s_item
@@ -701,7 +741,7 @@ confocal_batch_kernel(const ConfocalGatherParams* __restrict__ caps, const Batch
         const uint32_t it = s_item;
         if (it >= nitems) break;
         const BatchItem w = items[it];
-        confocal_tile<S, KV, WY, WZ, PATH, BOUNCE, false, CLAMP>(caps[w.capture], w.bx, w.by, w.bz, it);
+        confocal_tile<KV, WY, WZ, PATH, BOUNCE, false, CLAMP, false>(caps[w.capture], w.bx, w.by, w.bz, it, totals);
     }
 }
 

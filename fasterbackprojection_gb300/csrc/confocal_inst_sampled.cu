@@ -1,0 +1,9 @@
+// The sampled (MIS) gather.
+#include "confocal_launch.cuh"
+
+namespace fbp {
+fbp_status gather_sampled(fbp_context* ctx, const ConfocalGatherParams& p, dim3 grid, size_t smem, cudaStream_t stream,
+                          bool bounce, float t0, bool capped) {
+    return dispatch_confocal<true, false>(ctx, p, grid, smem, stream, bounce, t0, capped);
+}
+}  // namespace fbp

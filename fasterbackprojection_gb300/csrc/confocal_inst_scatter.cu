@@ -1,0 +1,9 @@
+// The voxel-scattering gather, one CTA per voxel tile.
+#include "confocal_launch.cuh"
+
+namespace fbp {
+fbp_status gather_scatter(fbp_context* ctx, const ConfocalGatherParams& p, dim3 grid, size_t smem, cudaStream_t stream,
+                          int sp, bool free_walk, bool bounce, bool capped) {
+    return dispatch_scatter<false>(ctx, p, grid, smem, stream, sp, free_walk, bounce, capped);
+}
+}  // namespace fbp

@@ -1,0 +1,58 @@
+"""The confocal gather's chains: small volumes split the scan points of a voxel
+tile over the CTAs of a cluster (1, 2, 4, 6 or 12 chains), each with its own
+compensated sums.
+
+  * against the FP64 oracle with the GPU's bins: 1e-6 relative L2, the bound of
+    the unsplit gather (FP32 sums of at most 32 terms and compensated folds:
+    32 * 2^-24 / 2 = 9.5e-7 for the worst case, far less in practice);
+  * a batch walks the same chains one after the other in one CTA: bit for bit.
+"""
+import numpy as np
+import pytest
+
+from oracle import cpu
+from tests.conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+# scan side, bins, volume, bounces kept, time offset.  Groups of 32 scan points:
+# 1, 2, 3, 5, 8 and 13 of them, the last one ragged; volumes of one voxel, one
+# tile, one tile plus a row on each axis, and with idle warps; windows that
+# are the whole row (few bins per voxel) and that are not.
+CASES = [
+    (3, 64, (1, 1, 1), False, 0.0),
+    (5, 128, (16, 16, 16), False, 0.0),
+    (8, 512, (17, 17, 17), False, 0.0),
+    (9, 96, (33, 9, 5), True, 0.0),
+    (12, 512, (40, 33, 17), True, 0.4),
+    (16, 640, (48, 20, 36), False, 0.4),
+    (20, 300, (16, 64, 24), True, -0.1),
+    (20, 2048, (21, 24, 40), False, 0.0),
+]
+
+
+@pytest.mark.parametrize("n,T,vres,bounce,t0", CASES)
+def test_chains_against_fp64_and_against_the_batch(ctx, cuda, n, T, vres, bounce, t0):
+    import torch
+
+    from fasterbackprojection_gb300 import Batch, make_info, scenes
+
+    cap = scenes.confocal_points(n, T, 4.92 / T / scenes.LIGHT_SPEED, n_points=40, depth_range=(0.3, 1.3), seed=n + T)
+    hmin, vs = scenes.volume_geometry(vres, depth_range=(0.0, 1.6))
+    info = make_info(num_laser_targets=n * n, num_time_bins=T, time_step=cap.time_step, voxel_res=vres,
+                     hidden_min=hmin, voxel_size=vs, discard_first_last_bounces=0 if bounce else 1, time_offset=t0,
+                     laser_position=(0.05, -0.25, 0.1), sensor_position=(-0.1, -0.2, 0.05))
+    cube = torch.from_numpy(cap.cube).to(cuda)
+    lx = torch.from_numpy(cap.laser_xyz).to(cuda)
+    vol = ctx.backproject_confocal(info, cube, lx)
+    bins = ctx.debug_confocal_bins(info, lx, torch.arange(vol.numel(), device=cuda)).cpu().numpy()
+    again = torch.full_like(vol, float("nan"))
+    batch = Batch(ctx, [(info, cube, lx, again, 1)])
+    batch.run()
+    torch.cuda.synchronize()
+    ctx.check_device_status()
+    batch.close()
+    want = cpu.confocal_voxel(info, cap.cube, cap.laser_xyz, bins=bins)
+    assert (bins >= 0).any()
+    assert rel_l2(vol.cpu().numpy(), want) < 1e-6
+    assert torch.equal(vol, again)
