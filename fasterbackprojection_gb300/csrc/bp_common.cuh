@@ -5,12 +5,8 @@
 
 namespace fbp {
 
-// ------------------------------------------------------------- cp.async --
+// ---------------------------------------------- bulk copies and mbarriers --
 
-__device__ __forceinline__ void cp_async_16(void* smem_dst, const void* gmem_src) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem_src) : "memory");
-}
 // Bulk copy of `bytes` (a multiple of 16, both addresses 16-byte aligned) from
 // global to shared memory, completing on the mbarrier at shared address `bar`.
 __device__ __forceinline__ void bulk_load(uint32_t smem_dst, const void* gmem_src, uint32_t bytes, uint32_t bar) {
@@ -72,10 +68,18 @@ __device__ __forceinline__ float lds_f32(uint32_t addr) {
     return v;
 }
 
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+// The sample of the bin floor(x) of a window that starts at bin a, from
+// biased = x + (2^23 - a) rounded towards zero: its low bits are floor(x) - a,
+// with no conversion.
+//   CLAMP   clamped to the slot at shared address `slot` (its sentinel, a zero,
+//           sits at slot_w).
+//   else    the planner guarantees a <= x < a + slot_w; `slot` is the address
+//           less the exponent's bits (kBiasBits).
+constexpr uint32_t kBiasBits = 0x4B000000u << 2;  // 2^23 as float bits, in bytes
+template <bool CLAMP>
+__device__ __forceinline__ float read_bin(float biased, int slot, uint32_t slot_w) {
+    if (CLAMP) return lds_f32((uint32_t)slot + (min(__float_as_uint(biased) - 0x4B000000u, slot_w) << 2));
+    return lds_f32((uint32_t)slot + (__float_as_uint(biased) << 2));
 }
 
 // ------------------------------------------------------ confocal gather --
@@ -171,6 +175,14 @@ fbp_status plan_window(const fbp_context* ctx, double ex, double ey, double ez, 
 // volume, whatever part of it a launch computes, so that slabs and batches sum
 // like the single call).
 uint32_t gather_chains(const fbp_context* ctx, const fbp_recon_info& in, size_t smem);
+// Chains for a launch of `tiles` voxel tiles that each walk `groups` groups,
+// occ CTAs to an SM.
+uint32_t split_chains(const fbp_context* ctx, uint64_t tiles, uint64_t groups, int occ);
+// CTAs of `smem` bytes of dynamic shared memory an SM holds, at most `most`.
+inline int resident_ctas(size_t smem, int most) {
+    const size_t n = kSmSharedBytes / (smem + kCtaReservedShared);
+    return n < 1 ? 1 : (n < (size_t)most ? (int)n : most);
+}
 constexpr int kGatherCtasPerSm = 3;  // 256 threads of 80 registers
 
 // The confocal gather over all scan points (smp == nullptr) or over K sampled

@@ -236,11 +236,7 @@ fbp_status launch_confocal(fbp_context* ctx, const fbp_recon_info& in, const voi
 // 128^3: 12.2 ms with 2, 12.1 with 6, 12.9 with 8, 15.3 with 16; 14.3 with one
 // CTA per tile).  One CTA per tile against this rule: 32^2 x 256 -> 32^3 291
 // -> 48 us (12 chains), 64^2 x 512 -> 64^3 1133 -> 482 us (6).
-uint32_t gather_chains(const fbp_context* ctx, const fbp_recon_info& in, size_t smem) {
-    const uint64_t tiles = (uint64_t)cdiv(in.voxel_res[0], kKVFull) * cdiv(in.voxel_res[1], 8 * kWY) *
-                           cdiv(in.voxel_res[2], 4 * kWZ);
-    const uint32_t groups = cdiv(in.num_laser_targets, ConfocalGatherParams::kGroup);
-    const int occ = (int)std::min<size_t>(kGatherCtasPerSm, std::max<size_t>(1, kSmSharedBytes / (smem + kCtaReservedShared)));
+uint32_t split_chains(const fbp_context* ctx, uint64_t tiles, uint64_t groups, int occ) {
     constexpr double kRate[kGatherCtasPerSm] = {0.68, 0.88, 1.0};
     uint32_t best = 1;
     double best_t = 0.0;
@@ -255,6 +251,13 @@ uint32_t gather_chains(const fbp_context* ctx, const fbp_recon_info& in, size_t 
         }
     }
     return best;
+}
+
+uint32_t gather_chains(const fbp_context* ctx, const fbp_recon_info& in, size_t smem) {
+    const uint64_t tiles = (uint64_t)cdiv(in.voxel_res[0], kKVFull) * cdiv(in.voxel_res[1], 8 * kWY) *
+                           cdiv(in.voxel_res[2], 4 * kWZ);
+    return split_chains(ctx, tiles, cdiv(in.num_laser_targets, ConfocalGatherParams::kGroup),
+                        resident_ctas(smem, kGatherCtasPerSm));
 }
 
 // Tile grid of the confocal gather (also the MIS sampling tiles).

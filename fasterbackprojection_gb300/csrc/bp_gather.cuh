@@ -44,38 +44,19 @@ __host__ __device__ constexpr bool scatter_free(int path) { return path - PATH_S
 // an eighth of the loop's issue slots).
 struct ScanPlan {
     const float4* geo;      // (x, y, z, bounce)
-    const int4* meta;       // (bias, bias, slot address, 0); see BinIndex
+    const int4* meta;       // (bias, bias, slot address, 0); see read_bin
     const ulonglong2* dx;   // [KV / 4] per point
     const float* weight;    // WEIGHTED: the sample's weight
 };
 
-// Word of shared memory a path ratio x reads.
-//   CLAMP   floor(x) - a, clamped to the slot (bias 2^23 - a, the slot's
-//           address beside it).
-//   else    the planner guarantees a <= x < a + slot width, so the slot's word
-//           and the window start fold into one addend: x 2^-149 + word 2^-149
-//           rounded towards zero is a subnormal whose bits are the word
-//           floor(x) - a + slot; no conversion, no shift, no add.
-#define FBP_TINY __int_as_float(1)  // 2^-149
-template <bool CLAMP>
-__device__ __forceinline__ f32x2_t bin_words2(f32x2_t x, f32x2_t bias, f32x2_t tiny) {
-    return CLAMP ? add_rz2(x, bias) : fma_rz2(x, tiny, bias);
-}
-template <bool CLAMP>
-__device__ __forceinline__ float read_bin(const float* smem, float word, int slot, uint32_t slot_w) {
-    if (CLAMP) return lds_f32((uint32_t)slot + (min(__float_as_uint(word) - 0x4B000000u, slot_w) << 2));
-    return smem[__float_as_uint(word)];
-}
-
 // One staged stage of scan points against a thread's KV voxels (consecutive
 // along x, sharing the y/z offsets).
 template <int KV, int PATH, bool BOUNCE, bool CLAMP, bool SAFE, bool WEIGHTED>
-__device__ __forceinline__ void confocal_stage(const ScanPlan pl, const float* __restrict__ smem, int nl, float py,
+__device__ __forceinline__ void confocal_stage(const ScanPlan pl, int nl, float py,
                                                float pz, float neg_t0, float rcp_dt, uint32_t slot_w,
                                                float (&acc)[KV], float ext = 0.f, float step = 0.f,
                                                bool tail = true) {
     const float rcp2 = 2.f * rcp_dt;  // exact
-    const f32x2_t tiny = pack2(FBP_TINY, FBP_TINY);
     if constexpr (is_scatter(PATH)) {
         constexpr int SP = scatter_prefix(PATH);
         static_assert(SP >= 1 && SP <= kScatterMaxPrefix, "prefix within the step bound");
@@ -102,7 +83,7 @@ __device__ __forceinline__ void confocal_stage(const ScanPlan pl, const float* _
             }
             auto bin_at = [&](float dd) -> float {
                 const float x = ref_bin_ratio(dd, rcp_dt);
-                return read_bin<CLAMP>(smem, CLAMP ? add_rz(x, bias) : fma_rz(x, FBP_TINY, bias), m.z, slot_w);
+                return read_bin<CLAMP>(add_rz(x, bias), m.z, slot_w);
             };
             // Steps SP.. of one walk (rare: a diagonal longer than the planned steps).
             auto walk_rest = [&](float a, float dd, float dmax, float w) -> float {
@@ -137,8 +118,8 @@ __device__ __forceinline__ void confocal_stage(const ScanPlan pl, const float* _
                     for (int it = 0; it < SP; ++it) {
                         float d0, d1, b0, b1, p0, p1;
                         unpack2(dd, d0, d1);
-                        unpack2(bin_words2<CLAMP>(mul_rn2(dd, rdp), biasp, tiny), b0, b1);
-                        f32x2_t I = pack2(read_bin<CLAMP>(smem, b0, m.z, slot_w), read_bin<CLAMP>(smem, b1, m.z, slot_w));
+                        unpack2(add_rz2(mul_rn2(dd, rdp), biasp), b0, b1);
+                        f32x2_t I = pack2(read_bin<CLAMP>(b0, m.z, slot_w), read_bin<CLAMP>(b1, m.z, slot_w));
                         if (WEIGHTED) I = mul_rn2(I, wlp);
                         unpack2(mul_rn2(I, w), p0, p1);
                         if constexpr (scatter_free(PATH)) {
@@ -191,8 +172,8 @@ __device__ __forceinline__ void confocal_stage(const ScanPlan pl, const float* _
         // Voxel pairs (k, k + 1) in packed FP32 pairs: the bins are the scalar
         // loop's operations, bit for bit, in half the instructions.  A packed
         // instruction holds the issue port for two cycles, and the port is what
-        // bounds this loop (issue 66 % + second cycles 34 % of all cycles
-        // before the differences and the bin words left it; MUFU pipe 76 %).
+        // bounds this loop (issue 66 % + second cycles 34 % of all cycles,
+        // MUFU pipe 76 %, before the differences left it: 362 -> 347 ms).
         //
         // Weights by simultaneous inversion (P. L. Montgomery, "Speeding the
         // Pollard and elliptic curve methods of factorization", Math. Comp. 48
@@ -252,8 +233,8 @@ __device__ __forceinline__ void confocal_stage(const ScanPlan pl, const float* _
                         x = mul_rn2(dist, rdp);
                         sq[jj] = mul_rn2(dist, dist);
                     }
-                    unpack2(bin_words2<CLAMP>(x, biasp, tiny), b0, b1);
-                    Iq[jj] = pack2(read_bin<CLAMP>(smem, b0, m.z, slot_w), read_bin<CLAMP>(smem, b1, m.z, slot_w));
+                    unpack2(add_rz2(x, biasp), b0, b1);
+                    Iq[jj] = pack2(read_bin<CLAMP>(b0, m.z, slot_w), read_bin<CLAMP>(b1, m.z, slot_w));
                     if (WEIGHTED) Iq[jj] = mulf2(Iq[jj], wlp);
                 }
                 float m0, m1;
@@ -298,7 +279,7 @@ __device__ __forceinline__ void confocal_stage(const ScanPlan pl, const float* _
                     I = lds_f32((uint32_t)m.z + (min((uint32_t)(__float2int_rz(x) - m.x), slot_w) << 2));
                 } else {
                     const float bias = __int_as_float(m.x);
-                    I = read_bin<CLAMP>(smem, CLAMP ? add_rz(x, bias) : fma_rz(x, FBP_TINY, bias), m.z, slot_w);
+                    I = read_bin<CLAMP>(add_rz(x, bias), m.z, slot_w);
                 }
                 if (WEIGHTED) I *= wl;
                 acc[k] = fmaf(I, ref_safe_rcp(mul_rn(dist, dist)), acc[k]);
@@ -349,7 +330,6 @@ __device__ __forceinline__ void confocal_tile(const ConfocalGatherParams& p, uin
     float* s_w = reinterpret_cast<float*>(s_cnt + MB * GRP);             // [MB][GRP]
     int2* s_group = reinterpret_cast<int2*>(s_w + MB * GRP);             // [MB] (points kept, guarded)
     constexpr size_t slots_off = ConfocalGatherParams::meta_bytes(KV);
-    const float* s_all = reinterpret_cast<const float*>(smem_raw);
     float* s_slots = reinterpret_cast<float*>(smem_raw + slots_off);     // [NB][CH][slot_stride]
 
     const int tid = threadIdx.x;
@@ -550,13 +530,14 @@ __device__ __forceinline__ void confocal_tile(const ConfocalGatherParams& p, uin
             if (!skip) {
                 const uint32_t st = gi * sub + pos / CH;
                 const uint32_t slot_elem = ((st % NB) * CH + pos % CH) * slot_stride;
-                const int word = (int)(slots_off / 4 + slot_elem) - a;  // shared-memory word of bin 0
-                int bias;
-                if (PATH == PATH_EXACT && guarded) bias = a;
-                else if (CLAMP) bias = __float_as_int((float)(8388608 - a));
-                else bias = word >= 0 ? word : (int)(0x80000000u | (uint32_t)-word);  // word 2^-149
+                uint32_t slot = sbase + (uint32_t)slots_off + (slot_elem << 2);
+                int bias = a;  // PATH_EXACT, guarded
+                if (!(PATH == PATH_EXACT && guarded)) {
+                    bias = __float_as_int((float)(8388608 - a));
+                    if (!CLAMP) slot -= kBiasBits;
+                }
                 s_geo[gb + pos] = g;
-                s_meta[gb + pos] = make_int4(bias, bias, (int)(sbase + (uint32_t)slots_off + (slot_elem << 2)), 0);
+                s_meta[gb + pos] = make_int4(bias, bias, (int)slot, 0);
                 float* dx = reinterpret_cast<float*>(s_dx + (gb + pos) * (KV / 4));
 #pragma unroll
                 for (int k = 0; k < KV; ++k) dx[k] = sub_rn(p.xs[min(tx0 + k, p.Vx - 1)], g.x);
@@ -641,11 +622,11 @@ __device__ __forceinline__ void confocal_tile(const ConfocalGatherParams& p, uin
                 const uint32_t o = gb + h * CH;
                 const ScanPlan plan{s_geo + o, s_meta + o, s_dx + o * (KV / 4), s_w + o};
                 if (!grp.y) {
-                    confocal_stage<KV, PATH, BOUNCE, CLAMP, false, SAMPLED>(plan, s_all, nl, py, pz, neg_t0, rcp_dt, p.slot_w,
+                    confocal_stage<KV, PATH, BOUNCE, CLAMP, false, SAMPLED>(plan, nl, py, pz, neg_t0, rcp_dt, p.slot_w,
                                                                             acc, scat_ext, scat_step, !p.scat_exact);
                     if (PATH == PATH_2D) scale = 0.25f;  // w was rcp(d^2) = 4 rcp(dist^2)
                 } else {
-                    confocal_stage<KV, PATH, BOUNCE, CLAMP, true, SAMPLED>(plan, s_all, nl, py, pz, neg_t0, rcp_dt, p.slot_w,
+                    confocal_stage<KV, PATH, BOUNCE, CLAMP, true, SAMPLED>(plan, nl, py, pz, neg_t0, rcp_dt, p.slot_w,
                                                                            acc, scat_ext, scat_step);
                 }
             }

@@ -210,13 +210,6 @@ __device__ __forceinline__ float add_rz(float a, float b) {
     return r;
 }
 
-// fma with round-toward-zero, no flush to zero (subnormal results are used).
-__device__ __forceinline__ float fma_rz(float a, float b, float c) {
-    float r;
-    asm("fma.rz.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
-}
-
 // Packed FP32 pairs (the f32x2 instructions of sm_100 and later): one
 // instruction applies the scalar operation above to both halves, with the
 // same rounding, so results are bitwise those of two scalar operations.
@@ -252,11 +245,6 @@ __device__ __forceinline__ f32x2_t fma_rn2(f32x2_t a, f32x2_t b, f32x2_t c) {
 __device__ __forceinline__ f32x2_t add_rz2(f32x2_t a, f32x2_t b) {
     f32x2_t r;
     asm("add.rz.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2_t fma_rz2(f32x2_t a, f32x2_t b, f32x2_t c) {
-    f32x2_t r;
-    asm("fma.rz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
 // a * b and fmaf (no flush to zero) on both halves.

@@ -56,3 +56,42 @@ def test_chains_against_fp64_and_against_the_batch(ctx, cuda, n, T, vres, bounce
     assert (bins >= 0).any()
     assert rel_l2(vol.cpu().numpy(), want) < 1e-6
     assert torch.equal(vol, again)
+
+
+# laser side, SPAD side, bins, volume, bounces kept, time offset: laser blocks
+# of 4 that are whole (4, 16, 36 lasers), padded (9, 25) or not taken (1), pair
+# groups of 32 that are one, ragged or many, volumes of one voxel, one tile and
+# one tile plus a row; windows that are the whole row; paths around zero.
+EXHAUSTIVE = [
+    (1, 1, 64, (1, 1, 1), False, 0.0),
+    (2, 3, 96, (8, 16, 16), True, 0.0),
+    (1, 6, 512, (9, 17, 17), False, 0.0),
+    (3, 5, 300, (17, 9, 5), False, 0.5),
+    (3, 7, 1024, (24, 20, 36), True, 0.5),
+    (4, 6, 256, (16, 33, 20), False, -0.3),
+    (5, 4, 2048, (21, 16, 16), False, 0.0),
+    (6, 9, 640, (40, 24, 24), True, -0.2),
+]
+
+
+@pytest.mark.parametrize("nl,ns,T,vres,bounce,t0", EXHAUSTIVE)
+def test_exhaustive_chains_against_fp64(ctx, cuda, nl, ns, T, vres, bounce, t0):
+    import torch
+
+    from fasterbackprojection_gb300 import FBP_EXHAUSTIVE, make_info, scenes
+
+    cap = scenes.exhaustive_points(nl, ns, T, 4.92 / T / scenes.LIGHT_SPEED, n_points=40, depth_range=(0.3, 1.3),
+                                   seed=nl + T)
+    hmin, vs = scenes.volume_geometry(vres, depth_range=(0.0, 1.6))
+    info = make_info(num_laser_targets=nl * nl, num_sensor_targets=ns * ns, num_time_bins=T, time_step=cap.time_step,
+                     voxel_res=vres, hidden_min=hmin, voxel_size=vs, capture_system=FBP_EXHAUSTIVE,
+                     discard_first_last_bounces=0 if bounce else 1, time_offset=t0,
+                     laser_position=(0.05, -0.25, 0.1), sensor_position=(-0.1, -0.2, 0.05))
+    lx = torch.from_numpy(cap.laser_xyz).to(cuda)
+    sx = torch.from_numpy(cap.sensor_xyz).to(cuda)
+    vol = ctx.backproject_exhaustive(info, torch.from_numpy(cap.cube).to(cuda), lx, sx)
+    bins = ctx.debug_exhaustive_bins(info, lx, sx, torch.arange(vol.numel(), device=cuda)).cpu().numpy()
+    ctx.check_device_status()
+    want = cpu.exhaustive_voxel(info, cap.cube, cap.laser_xyz, cap.sensor_xyz, bins=bins)
+    assert (bins >= 0).any()
+    assert rel_l2(vol.cpu().numpy(), want) < 1e-6
