@@ -12,8 +12,408 @@
 #include "bp_common.cuh"
 
 #include <algorithm>
+#include <cmath>
 
 namespace fbp {
+
+struct DepthTileParams {
+    const float4* scan;      // [L] (x, y, z, bounce)
+    const float* xyz;        // [L][3]
+    const double* depths;    // [D]
+    const float* rows;       // [L][pitch]
+    float* act;              // [L][D]
+    int* status;
+    uint32_t L, D, T, pitch;
+    uint32_t side;           // > 0: the scan points are a side x side grid (tiles of 16 x 16), else runs of 256
+    float nx, ny, nz, t0, dt;
+    uint32_t chains;
+
+    static constexpr int kGroup = 32, kPlanBufs = 4, kThreads = 256, kDepths = 16;
+    static constexpr uint32_t kSlot = 256;           // widest window that is not the whole row
+    // Barriers, per scan point of kPlanBufs groups (x, y, z, bounce), (bias,
+    // bias, slot address), the window's source and length, two words per group.
+    static constexpr size_t kMeta = 64 + (size_t)kPlanBufs * kGroup * (16 + 16 + 8 + 4) + kPlanBufs * 8;
+    static constexpr size_t kSums = (size_t)2 * kDepths * kThreads * sizeof(float);
+    static constexpr size_t kSmem = kSmSharedBytes / 3 - kCtaReservedShared - 256;  // three CTAs per SM
+    static constexpr uint32_t kWindowFloats = (uint32_t)((kSmem - kMeta - kSums) / sizeof(float));
+    // Longest row whose whole-row windows fit, one scan point to a stage.
+    static constexpr uint32_t kMaxBins = (kWindowFloats / 2 - 8) / 4 * 4;
+};
+
+// A CTA (or a cluster of p.chains, one per range of scan-point groups) owns 256
+// scan points' test points at 16 consecutive depths: a thread one scan point, a
+// warp 8 x 4 of the grid.  Pipeline, groups and folds as in the confocal
+// gather; the window width is the CTA's own, from the box of its points (the
+// host does not know the positions), and windows wider than kSlot are whole
+// rows, like those of a CTA with a non-finite point (int(NaN) is bin 0).
+// YONLY: the wall normal has only a y component, so x and z do not depend on
+// the depth (adding 0 * depth changes no bit).
+// Bound by the issue port (a packed FP32 instruction holds it two cycles),
+// about 22 cycles per packed pair.  64^2 x 512, 200 planes: 2.87 -> DEPTHMS ms
+// against one thread per point with rows in global memory.
+template <bool YONLY, bool BOUNCE>
+__global__ void __launch_bounds__(DepthTileParams::kThreads, YONLY ? 3 : 2) depth_tile_kernel(DepthTileParams p) {
+    using P = DepthTileParams;
+    constexpr int NT = P::kThreads, NW = NT / 32, KV = P::kDepths;
+    constexpr uint32_t GRP = P::kGroup, NB = 2, MB = P::kPlanBufs;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ float s_box[6][NW];
+    const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem_raw);
+    const uint32_t bar_full = sbase, bar_empty = sbase + 8 * NB, bar_plan = sbase + 16 * NB;  // NB, NB and MB of 8 bytes
+    float4* s_geo = reinterpret_cast<float4*>(smem_raw + 64);              // [MB][GRP]
+    int4* s_meta = reinterpret_cast<int4*>(s_geo + MB * GRP);              // [MB][GRP]
+    const float** s_src = reinterpret_cast<const float**>(s_meta + MB * GRP);  // [MB][GRP]
+    int* s_cnt = reinterpret_cast<int*>(s_src + MB * GRP);                 // [MB][GRP]
+    int2* s_group = reinterpret_cast<int2*>(s_cnt + MB * GRP);             // [MB] (points kept, guarded)
+    float* s_sums = reinterpret_cast<float*>(smem_raw + P::kMeta);         // [2 KV][NT]
+    float* s_slots = s_sums + 2 * KV * NT;                                 // [NB][CH][slot_stride]
+    const uint32_t slots_at = sbase + (uint32_t)(P::kMeta + P::kSums);
+
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t rank = blockIdx.x % p.chains, tile = blockIdx.x / p.chains;
+    // This thread's scan point.
+    uint32_t c = tile * NT + tid;
+    bool ok = c < p.L;
+    if (p.side) {
+        const uint32_t tiles = (p.side + 15) / 16;
+        const uint32_t ix = tile % tiles * 16 + (warp & 1) * 8 + (lane & 7);
+        const uint32_t iz = tile / tiles * 16 + (warp >> 1) * 4 + (lane >> 3);
+        ok = ix < p.side && iz < p.side;
+        c = min(iz, p.side - 1) * p.side + min(ix, p.side - 1);
+    }
+    c = min(c, p.L - 1);
+    const uint32_t d0 = blockIdx.y * KV;
+    const bool warp_ok = __any_sync(0xffffffffu, ok);
+
+    // Test points (transient_reconstruction.cuh:51) and their box.
+    const float lx = p.xyz[3 * (size_t)c], ly = p.xyz[3 * (size_t)c + 1], lz = p.xyz[3 * (size_t)c + 2];
+    float px[YONLY ? 1 : KV], pz[YONLY ? 1 : KV];
+    f32x2_t pyp[KV / 2];
+    float box[6] = {INFINITY, -INFINITY, INFINITY, -INFINITY, INFINITY, -INFINITY};
+    bool finite = true;
+#pragma unroll
+    for (int k = 0; k < KV; k += 2) {
+        float y[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const float df = (float)p.depths[min(d0 + k + h, p.D - 1)];
+            const float x = fma_rn(p.nx, df, lx), z = fma_rn(p.nz, df, lz);
+            y[h] = YONLY && !isfinite(df) ? NAN : fma_rn(p.ny, df, ly);  // (0 * df is NaN in x and z)
+            px[YONLY ? 0 : k + h] = x;
+            pz[YONLY ? 0 : k + h] = z;
+            finite = finite && isfinite(x) && isfinite(y[h]) && isfinite(z);
+            box[0] = fminf(box[0], x); box[1] = fmaxf(box[1], x);
+            box[2] = fminf(box[2], y[h]); box[3] = fmaxf(box[3], y[h]);
+            box[4] = fminf(box[4], z); box[5] = fmaxf(box[5], z);
+        }
+        pyp[k / 2] = pack2(y[0], y[1]);
+    }
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        for (int o = 16; o > 0; o >>= 1) {
+            const float v = __shfl_xor_sync(0xffffffffu, box[i], o);
+            box[i] = i & 1 ? fmaxf(box[i], v) : fminf(box[i], v);
+        }
+        if (lane == 0) s_box[i][warp] = box[i];
+    }
+    if (tid == 0) {
+        for (uint32_t b = 0; b < NB; ++b) {
+            mbar_init(bar_full + 8 * b, 1);
+            mbar_init(bar_empty + 8 * b, NW);
+        }
+        for (uint32_t b = 0; b < MB; ++b) mbar_init(bar_plan + 8 * b, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+#pragma unroll
+    for (int k = 0; k < 2 * KV; ++k) s_sums[k * NT + tid] = 0.f;
+    const bool odd = __syncthreads_or(!finite);
+#pragma unroll
+    for (int i = 0; i < 6; ++i)
+        for (int w = 0; w < NW; ++w) box[i] = i & 1 ? fmaxf(box[i], s_box[i][w]) : fminf(box[i], s_box[i][w]);
+
+    // Window width: the round trip across the box and a 2-bin margin on each
+    // side, or the whole row; scan points per stage: what fits twice.
+    const float rcp_dt = rcp_approx(p.dt);
+    const float ex = box[1] - box[0], ey = box[3] - box[2], ez = box[5] - box[4];
+    const float span = 2.01f * sqrtf(ex * ex + ey * ey + ez * ez) / p.dt + 12.f;
+    const uint32_t t_round = (p.T + 3) & ~3u;
+    const bool whole = odd || !(span < (float)P::kSlot) || t_round + 4 <= (uint32_t)span;
+    const uint32_t slot_w = whole ? t_round + 4 : ((uint32_t)span + 4) & ~3u;
+    const uint32_t slot_stride = slot_w + 4;  // sentinel at slot_w
+    uint32_t CH = GRP;
+    while (CH > 1 && NB * CH * slot_stride > P::kWindowFloats) CH >>= 1;
+    for (uint32_t i = tid; i < NB * CH * 4; i += NT) s_slots[(size_t)(i / 4) * slot_stride + slot_w + i % 4] = 0.f;
+
+    const uint32_t ngroups = (p.L + GRP - 1) / GRP;
+    const uint32_t g0 = (uint32_t)((uint64_t)rank * ngroups / p.chains);
+    const uint32_t mine = (uint32_t)((uint64_t)(rank + 1) * ngroups / p.chains) - g0;
+    const uint32_t sub = GRP / CH, nstages = mine * sub;
+    const float neg_t0 = -p.t0;
+
+    // Plan this CTA's group gi (one warp): see the confocal gather.
+    auto plan_group = [&](uint32_t gi) {
+        const uint32_t gb = (gi % MB) * GRP, l = (g0 + gi) * GRP + lane;
+        float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
+        int a = 0, cnt = 0, near = 0;
+        bool keep = l < p.L;
+        if (keep) {
+            g = p.scan[l];
+            const float cx = fminf(fmaxf(g.x, box[0]), box[1]), cy = fminf(fmaxf(g.y, box[2]), box[3]),
+                        cz = fminf(fmaxf(g.z, box[4]), box[5]);
+            const float dmin = sqrtf((g.x - cx) * (g.x - cx) + (g.y - cy) * (g.y - cy) + (g.z - cz) * (g.z - cz));
+            const float fx = fmaxf(fabsf(g.x - box[0]), fabsf(g.x - box[1])),
+                        fy = fmaxf(fabsf(g.y - box[2]), fabsf(g.y - box[3])),
+                        fz = fmaxf(fabsf(g.z - box[4]), fabsf(g.z - box[5]));
+            const float dmax = sqrtf(fx * fx + fy * fy + fz * fz);
+            const float bnc = BOUNCE ? g.w : 0.f;
+            const float pmin = 2.f * dmin + neg_t0 + bnc, pmax = 2.f * dmax + neg_t0 + bnc;
+            if (odd || !isfinite(pmax) || !isfinite(pmin)) {
+                near = 1;  // int() of every path, over the row from bin 0
+                cnt = (int)slot_w;
+            } else {
+                near = pmin < 0.0035f && (p.t0 > 0.f || BOUNCE);  // int() truncates towards zero
+                const int blo = (int)fmaxf(fminf(floorf(pmin * rcp_dt), 1.0e9f), -1.0e9f) - 2;
+                const int bhi = (int)fmaxf(fminf(floorf(pmax * rcp_dt), 1.0e9f), -1.0e9f) + 2;
+                keep = bhi >= 0 && blo < (int)p.T;  // a bin of the tile is inside [0, T)
+                a = whole ? 0 : max(blo, 0) & ~3;
+                cnt = whole ? (int)slot_w : (max(bhi + 1 - a, 0) + 3) & ~3;
+                if (keep && cnt > (int)slot_w) {  // the span bound failed: skip, report
+                    atomicExch(p.status, (int)FBP_ERR_DEVICE);
+                    keep = false;
+                }
+            }
+            cnt = min(cnt, (int)p.pitch - a);
+        }
+        const unsigned kept = __ballot_sync(0xffffffffu, keep);
+        const bool guarded = __any_sync(0xffffffffu, near && keep);
+        const uint32_t pos = __popc(kept & ((1u << lane) - 1u));
+        if (keep) {
+            const uint32_t st = gi * sub + pos / CH;
+            uint32_t slot = slots_at + (((st % NB) * CH + pos % CH) * slot_stride << 2);
+            int bias = a;
+            if (!guarded) {
+                bias = __float_as_int((float)(8388608 - a));
+                if (!whole) slot -= kBiasBits;
+            }
+            s_geo[gb + pos] = g;
+            s_meta[gb + pos] = make_int4(bias, bias, (int)slot, 0);
+            s_cnt[gb + pos] = cnt;
+            s_src[gb + pos] = p.rows + (size_t)l * p.pitch + a;
+        }
+        if (lane == 0) s_group[gi % MB] = make_int2(__popc(kept), guarded);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_plan + 8 * (gi % MB));
+    };
+    bool dead = false;
+    auto wait = [&](uint32_t bar, uint32_t parity) {
+        if (!dead && !mbar_wait_parity(bar, parity)) {
+            dead = true;
+            if (lane == 0) atomicExch(p.status, (int)FBP_ERR_TIMEOUT);
+        }
+    };
+    auto produce = [&](uint32_t st) {
+        const uint32_t buf = st % NB, gi = st / sub, first = (st % sub) * CH;
+        wait(bar_plan + 8 * (gi % MB), (gi / MB) & 1);
+        if (st >= NB) wait(bar_empty + 8 * buf, (st / NB - 1) & 1);
+        if (dead) return;
+        const uint32_t gb = (gi % MB) * GRP, n = (uint32_t)s_group[gi % MB].x;
+        const uint32_t bytes = lane - first < CH && (uint32_t)lane < n ? (uint32_t)s_cnt[gb + lane] * 4u : 0u;
+        const uint32_t total = __reduce_add_sync(0xffffffffu, bytes);
+        if (lane == 0) mbar_arrive_expect_tx(bar_full + 8 * buf, total);
+        __syncwarp();
+        if (bytes)
+            bulk_load(slots_at + ((buf * CH + lane - first) * slot_stride << 2), s_src[gb + lane], bytes, bar_full + 8 * buf);
+    };
+
+    f32x2_t accp[KV / 2];
+#pragma unroll
+    for (int j = 0; j < KV / 2; ++j) accp[j] = 0ull;
+    const bool plain = !BOUNCE && p.t0 == 0.f;  // x = (2 d) rcp = d (2 rcp), exactly
+    const f32x2_t xs = plain ? pack2(2.f * rcp_dt, 2.f * rcp_dt) : pack2(rcp_dt, rcp_dt);
+    const f32x2_t two = pack2(2.f, 2.f), nt0p = pack2(neg_t0, neg_t0);
+    // Squared distances of depths (2 j, 2 j + 1) to scan point g.
+    auto square = [&](int j, const float4& g, f32x2_t dxc, f32x2_t dzc) -> f32x2_t {
+        const f32x2_t dy = sub_rn2(pyp[j], pack2(g.y, g.y));
+        if (!YONLY) {
+            dxc = sub_rn2(pack2(px[YONLY ? 0 : 2 * j], px[YONLY ? 0 : 2 * j + 1]), pack2(g.x, g.x));
+            dzc = sub_rn2(pack2(pz[YONLY ? 0 : 2 * j], pz[YONLY ? 0 : 2 * j + 1]), pack2(g.z, g.z));
+        }
+        return fma_rn2(dzc, dzc, fma_rn2(dxc, dxc, mul_rn2(dy, dy)));
+    };
+    auto walk = [&](uint32_t o, int n, auto&& sample) {
+#pragma unroll 2
+        for (int i = 0; i < n; ++i) {
+            const float4 g = s_geo[o + i];
+            const int4 m = s_meta[o + i];
+            const float dx = sub_rn(px[0], g.x), dz = sub_rn(pz[0], g.z);
+            const f32x2_t dxc = pack2(dx, dx), dzc = pack2(dz, dz);
+#pragma unroll
+            for (int j = 0; j < KV / 2; ++j) {
+                float q0, q1;
+                unpack2(square(j, g, dxc, dzc), q0, q1);
+                f32x2_t d = pack2(sqrt_approx(q0), sqrt_approx(q1));
+                if (!plain) {
+                    d = fma_rn2(d, two, nt0p);
+                    if (BOUNCE) d = add_rn2(d, pack2(g.w, g.w));
+                }
+                accp[j] = add_rn2(accp[j], sample(mul_rn2(d, xs), m));
+            }
+        }
+    };
+    auto fast = [&](f32x2_t x, const int4& m) -> f32x2_t {
+        float b0, b1;
+        unpack2(add_rz2(x, pack2(__int_as_float(m.x), __int_as_float(m.y))), b0, b1);
+        return pack2(read_bin<false>(b0, m.z, slot_w), read_bin<false>(b1, m.z, slot_w));
+    };
+    auto clamped = [&](f32x2_t x, const int4& m) -> f32x2_t {
+        float b0, b1;
+        unpack2(add_rz2(x, pack2(__int_as_float(m.x), __int_as_float(m.y))), b0, b1);
+        return pack2(read_bin<true>(b0, m.z, slot_w), read_bin<true>(b1, m.z, slot_w));
+    };
+    auto converted = [&](f32x2_t x, const int4& m) -> f32x2_t {  // static_cast<int>, like the reference
+        float x0, x1;
+        unpack2(x, x0, x1);
+        return pack2(lds_f32((uint32_t)m.z + (min((uint32_t)(__float2int_rz(x0) - m.x), slot_w) << 2)),
+                     lds_f32((uint32_t)m.z + (min((uint32_t)(__float2int_rz(x1) - m.x), slot_w) << 2)));
+    };
+    auto fold = [](float part, float& sum, float& comp) {  // compensated (Kahan) addition
+        const float y = sub_rn(part, comp);
+        const float t = add_rn(sum, y);
+        comp = sub_rn(sub_rn(t, sum), y);
+        sum = t;
+    };
+
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();  // sentinels written
+    if (warp < 2 && (uint32_t)warp < mine) plan_group(warp);
+    if (warp == 0 && nstages > 0) produce(0);
+    for (uint32_t gi = 0; gi < mine; ++gi) {
+        const uint32_t gb = (gi % MB) * GRP;
+        for (uint32_t h = 0; h < sub; ++h) {
+            const uint32_t st = gi * sub + h, buf = st % NB;
+            wait(bar_full + 8 * buf, (st / NB) & 1);
+            if (st + 1 < nstages && warp == (int)((st + 1) % NW)) produce(st + 1);
+            if (h == 0 && gi + 2 < mine && !dead && warp == (int)((st + NW / 2) % NW)) plan_group(gi + 2);
+            const int2 grp = s_group[gi % MB];
+            const int n = min((int)CH, grp.x - (int)(h * CH));
+            if (warp_ok && !dead) {
+                const uint32_t o = gb + h * CH;
+                if (grp.y) walk(o, n, converted);
+                else if (whole) walk(o, n, clamped);
+                else walk(o, n, fast);
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_empty + 8 * buf);
+        }
+#pragma unroll
+        for (int j = 0; j < KV / 2; ++j) {
+            float part[2];
+            unpack2(accp[j], part[0], part[1]);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float* s = s_sums + (2 * (2 * j + h)) * NT + tid;
+                float sum = s[0], comp = s[NT];
+                fold(part[h], sum, comp);
+                s[0] = sum;
+                s[NT] = comp;
+            }
+            accp[j] = 0ull;
+        }
+    }
+
+    float* out = p.act + (size_t)c * p.D + d0;
+    if (p.chains == 1) {
+        if (ok) {
+#pragma unroll
+            for (int k = 0; k < KV; ++k)
+                if (d0 + k < p.D) out[k] = s_sums[(2 * k) * NT + tid];
+        }
+        return;
+    }
+    // The chains' sums, folded in order; CTA `rank` stores every chains-th depth.
+    cluster_arrive();
+    cluster_wait();
+    const uint32_t kb = (uint32_t)__cvta_generic_to_shared(s_sums + tid);
+    for (uint32_t k = rank; k < (uint32_t)KV; k += p.chains) {
+        float sum = 0.f, comp = 0.f;
+        for (uint32_t r = 0; r < p.chains; ++r) {
+            const uint32_t from = cluster_map(kb, r) + k * (2 * NT * 4u);
+            fold(cluster_load(from), sum, comp);
+            fold(-cluster_load(from + NT * 4u), sum, comp);
+        }
+        if (ok && d0 + k < p.D) out[k] = sum;
+    }
+    cluster_arrive();
+    cluster_wait();  // the others are through with this CTA's sums
+}
+
+template <bool YONLY, bool BOUNCE>
+fbp_status go_depth_tiles(fbp_context* ctx, const DepthTileParams& p, dim3 grid, cudaStream_t stream) {
+    auto kernel = depth_tile_kernel<YONLY, BOUNCE>;
+    const size_t smem = DepthTileParams::kMeta + DepthTileParams::kSums + DepthTileParams::kWindowFloats * sizeof(float);
+    FBP_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (p.chains == 1) {
+        kernel<<<grid, DepthTileParams::kThreads, smem, stream>>>(p);
+    } else {
+        FBP_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        cudaLaunchAttribute attr{};
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = p.chains;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(grid.x * p.chains, grid.y, 1);
+        cfg.blockDim = dim3(DepthTileParams::kThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        FBP_TRY_CUDA(cudaLaunchKernelEx(&cfg, kernel, p));
+    }
+    FBP_CHECK_LAUNCH(ctx, "depth_tile_kernel");
+    return FBP_OK;
+}
+
+// The confocal planes by tiles of 256 scan points x 16 depths.
+template <typename S>
+fbp_status launch_depth_tiles(fbp_context* ctx, const fbp_recon_info& in, const void* cube, int layout,
+                              const float* laser_xyz, const double* depths, uint32_t D, float* act,
+                              cudaStream_t stream) {
+    const uint32_t L = in.num_laser_targets, T = in.num_time_bins;
+    DepthTileParams p{};
+    p.pitch = (T + 3) / 4 * 4 + DepthTileParams::kSlot;
+    void *rows = nullptr, *sp = nullptr;
+    FBP_TRY(workspace(ctx, WS_CUBE_ROWS, (size_t)L * p.pitch * sizeof(float), stream, &rows));
+    FBP_TRY(prepare_rows_into<S>(ctx, cube, layout, L, T, p.pitch, static_cast<float*>(rows), stream));
+    FBP_TRY(workspace(ctx, WS_SCAN_TABLE, (size_t)L * sizeof(float4), stream, &sp));
+    scan_table_kernel<<<cdiv(L, 256), 256, 0, stream>>>(static_cast<float4*>(sp), laser_xyz, L,
+                                                       (int)in.discard_first_last_bounces, in.laser_position[0],
+                                                       in.laser_position[1], in.laser_position[2],
+                                                       in.sensor_position[0], in.sensor_position[1],
+                                                       in.sensor_position[2], 1);
+    FBP_CHECK_LAUNCH(ctx, "scan_table_kernel");
+    p.scan = static_cast<const float4*>(sp);
+    p.xyz = laser_xyz;
+    p.depths = depths;
+    p.rows = static_cast<const float*>(rows);
+    p.act = act;
+    p.status = ctx->status_dev;
+    p.L = L; p.D = D; p.T = T;
+    const uint32_t side = (uint32_t)std::lround(std::sqrt((double)L));
+    p.side = (uint64_t)side * side == L ? side : 0;
+    p.nx = in.wall_normal[0]; p.ny = in.wall_normal[1]; p.nz = in.wall_normal[2];
+    p.t0 = in.time_offset;
+    p.dt = in.time_step;
+    const uint64_t tiles = p.side ? (uint64_t)cdiv(side, 16) * cdiv(side, 16) : cdiv(L, DepthTileParams::kThreads);
+    const dim3 grid((unsigned)tiles, cdiv(D, DepthTileParams::kDepths));
+    const bool yonly = p.nx == 0.f && p.nz == 0.f, bounce = in.discard_first_last_bounces == 0;
+    p.chains = split_chains(ctx, tiles * grid.y, cdiv(L, DepthTileParams::kGroup), yonly ? 3 : 2);
+    if (yonly) {
+        if (bounce) return go_depth_tiles<true, true>(ctx, p, grid, stream);
+        return go_depth_tiles<true, false>(ctx, p, grid, stream);
+    }
+    if (bounce) return go_depth_tiles<false, true>(ctx, p, grid, stream);
+    return go_depth_tiles<false, false>(ctx, p, grid, stream);
+}
 
 template <typename S>
 __global__ void depth_confocal_kernel(const S* __restrict__ rows, uint32_t pitch, const float4* __restrict__ scan,
@@ -114,6 +514,8 @@ fbp_status launch_depths(fbp_context* ctx, const fbp_recon_info& in, const void*
                          const float* laser_xyz, const float* sensor_xyz, const double* depths, uint32_t D,
                          float* act, cudaStream_t stream) {
     const bool exhaustive = in.capture_system == FBP_EXHAUSTIVE;
+    if (!exhaustive && in.num_time_bins <= DepthTileParams::kMaxBins && cdiv(D, DepthTileParams::kDepths) <= 65535)
+        return launch_depth_tiles<S>(ctx, in, cube, layout, laser_xyz, depths, D, act, stream);
     const uint32_t L = in.num_laser_targets, Sn = exhaustive ? in.num_sensor_targets : 1, T = in.num_time_bins;
     const uint32_t pitch = (T + 7) / 8 * 8;
     const uint64_t R = (uint64_t)L * Sn;
