@@ -176,8 +176,8 @@ fbp_status plan_window(const fbp_context* ctx, double ex, double ey, double ez, 
 // like the single call).
 uint32_t gather_chains(const fbp_context* ctx, const fbp_recon_info& in, size_t smem);
 // Chains for a launch of `tiles` voxel tiles that each walk `groups` groups,
-// occ CTAs to an SM.
-uint32_t split_chains(const fbp_context* ctx, uint64_t tiles, uint64_t groups, int occ);
+// occ CTAs to an SM, a CTA's set-up worth `setup` groups.
+uint32_t split_chains(const fbp_context* ctx, uint64_t tiles, uint64_t groups, int occ, double setup = 0.3);
 // CTAs of `smem` bytes of dynamic shared memory an SM holds, at most `most`.
 inline int resident_ctas(size_t smem, int most) {
     const size_t n = kSmSharedBytes / (smem + kCtaReservedShared);

@@ -236,7 +236,7 @@ fbp_status launch_confocal(fbp_context* ctx, const fbp_recon_info& in, const voi
 // 128^3: 12.2 ms with 2, 12.1 with 6, 12.9 with 8, 15.3 with 16; 14.3 with one
 // CTA per tile).  One CTA per tile against this rule: 32^2 x 256 -> 32^3 291
 // -> 48 us (12 chains), 64^2 x 512 -> 64^3 1133 -> 482 us (6).
-uint32_t split_chains(const fbp_context* ctx, uint64_t tiles, uint64_t groups, int occ) {
+uint32_t split_chains(const fbp_context* ctx, uint64_t tiles, uint64_t groups, int occ, double setup) {
     constexpr double kRate[kGatherCtasPerSm] = {0.68, 0.88, 1.0};
     uint32_t best = 1;
     double best_t = 0.0;
@@ -244,7 +244,7 @@ uint32_t split_chains(const fbp_context* ctx, uint64_t tiles, uint64_t groups, i
         if (c > groups) break;
         const uint64_t per_sm = cdiv(tiles * c, (uint64_t)ctx->sm_count);
         const double rate = kRate[std::min<uint64_t>(per_sm, (uint64_t)occ) - 1] / kRate[occ - 1];
-        const double t = ((double)per_sm + 0.3) * ((double)groups / c + 0.3) / rate * (c == 12 ? 1.05 : 1.0);
+        const double t = ((double)per_sm + 0.3) * ((double)groups / c + setup) / rate * (c == 12 ? 1.05 : 1.0);
         if (c == 1 || t < 0.98 * best_t) {
             best = c;
             best_t = t;

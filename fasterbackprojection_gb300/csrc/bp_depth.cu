@@ -32,37 +32,48 @@ struct DepthTileParams {
     static constexpr uint32_t kSlot = 256;           // widest window that is not the whole row
     // Barriers, per scan point of kPlanBufs groups (x, y, z, bounce), (bias,
     // bias, slot address), the window's source and length, two words per group.
-    static constexpr size_t kMeta = 64 + (size_t)kPlanBufs * kGroup * (16 + 16 + 8 + 4) + kPlanBufs * 8;
+    // (A lattice's x differences, 16 floats, per scan point too.)
+    static constexpr size_t kMeta = 64 + (size_t)kPlanBufs * kGroup * (16 + 16 + 64 + 8 + 4) + kPlanBufs * 8;
     static constexpr size_t kSums = (size_t)2 * kDepths * kThreads * sizeof(float);
-    static constexpr size_t kSmem = kSmSharedBytes / 3 - kCtaReservedShared - 256;  // three CTAs per SM
+    static constexpr size_t kSmem = kSmSharedBytes / 3 - kCtaReservedShared - 512;  // three CTAs per SM
     static constexpr uint32_t kWindowFloats = (uint32_t)((kSmem - kMeta - kSums) / sizeof(float));
     // Longest row whose whole-row windows fit, one scan point to a stage.
     static constexpr uint32_t kMaxBins = (kWindowFloats / 2 - 8) / 4 * 4;
 };
 
 // A CTA (or a cluster of p.chains, one per range of scan-point groups) owns 256
-// scan points' test points at 16 consecutive depths: a thread one scan point, a
-// warp 8 x 4 of the grid.  Pipeline, groups and folds as in the confocal
-// gather; the window width is the CTA's own, from the box of its points (the
-// host does not know the positions), and windows wider than kSlot are whole
-// rows, like those of a CTA with a non-finite point (int(NaN) is bin 0).
+// scan points' test points at 16 consecutive depths.  Pipeline, groups and
+// folds as in the confocal gather; the window width is the CTA's own, from the
+// box of its points (the host does not know the positions), and windows wider
+// than kSlot are whole rows, like those of a CTA with a non-finite point
+// (int(NaN) is bin 0).
 // YONLY: the wall normal has only a y component, so x and z do not depend on
-// the depth (adding 0 * depth changes no bit).
-// Bound by the issue port (a packed FP32 instruction holds it two cycles),
-// about 22 cycles per packed pair.  64^2 x 512, 200 planes: 2.87 -> DEPTHMS ms
-// against one thread per point with rows in global memory.
-template <bool YONLY, bool BOUNCE>
+// the depth (adding 0 * depth changes no bit).  If the CTA's 16 x 16 scan
+// points are then also a lattice (x by column, z by row, one y), a thread takes
+// the 16 columns of one row at one depth, so that the x differences are common
+// to the CTA (made by the planner) and a warp, 2 rows x 16 depths, reads few
+// neighbouring bins; otherwise a thread takes the 16 depths of one scan point,
+// a warp 8 x 4 of the grid.
+// Bound by the issue port (a packed FP32 instruction holds it two cycles):
+// about 20 cycles per packed pair on a lattice, 30 otherwise.  64^2 x 512, 200
+// planes: one thread per point with rows in global memory 2867 us, a thread
+// per scan point 1200 us, the lattice 979 us.
+// PLAIN: no time offset and no bounces.
+template <bool YONLY, bool BOUNCE, bool PLAIN>
 __global__ void __launch_bounds__(DepthTileParams::kThreads, YONLY ? 3 : 2) depth_tile_kernel(DepthTileParams p) {
     using P = DepthTileParams;
     constexpr int NT = P::kThreads, NW = NT / 32, KV = P::kDepths;
     constexpr uint32_t GRP = P::kGroup, NB = 2, MB = P::kPlanBufs;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ float s_box[6][NW];
+    __shared__ float s_lat[33];  // x of the columns, z of the rows, y
+    __shared__ float s_df[KV];   // the depths
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem_raw);
     const uint32_t bar_full = sbase, bar_empty = sbase + 8 * NB, bar_plan = sbase + 16 * NB;  // NB, NB and MB of 8 bytes
     float4* s_geo = reinterpret_cast<float4*>(smem_raw + 64);              // [MB][GRP]
     int4* s_meta = reinterpret_cast<int4*>(s_geo + MB * GRP);              // [MB][GRP]
-    const float** s_src = reinterpret_cast<const float**>(s_meta + MB * GRP);  // [MB][GRP]
+    ulonglong2* s_dx = reinterpret_cast<ulonglong2*>(s_meta + MB * GRP);   // [MB][GRP][KV / 4]
+    const float** s_src = reinterpret_cast<const float**>(s_dx + MB * GRP * (KV / 4));  // [MB][GRP]
     int* s_cnt = reinterpret_cast<int*>(s_src + MB * GRP);                 // [MB][GRP]
     int2* s_group = reinterpret_cast<int2*>(s_cnt + MB * GRP);             // [MB] (points kept, guarded)
     float* s_sums = reinterpret_cast<float*>(smem_raw + P::kMeta);         // [2 KV][NT]
@@ -71,42 +82,38 @@ __global__ void __launch_bounds__(DepthTileParams::kThreads, YONLY ? 3 : 2) dept
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t rank = blockIdx.x % p.chains, tile = blockIdx.x / p.chains;
-    // This thread's scan point.
+    // This thread's scan point (unless the tile is a lattice).
+    const uint32_t cx = (warp & 1) * 8 + (lane & 7), cz = (warp >> 1) * 4 + (lane >> 3), sx = (p.side + 15) / 16;
     uint32_t c = tile * NT + tid;
     bool ok = c < p.L;
     if (p.side) {
-        const uint32_t tiles = (p.side + 15) / 16;
-        const uint32_t ix = tile % tiles * 16 + (warp & 1) * 8 + (lane & 7);
-        const uint32_t iz = tile / tiles * 16 + (warp >> 1) * 4 + (lane >> 3);
+        const uint32_t ix = tile % sx * 16 + cx, iz = tile / sx * 16 + cz;
         ok = ix < p.side && iz < p.side;
         c = min(iz, p.side - 1) * p.side + min(ix, p.side - 1);
     }
     c = min(c, p.L - 1);
     const uint32_t d0 = blockIdx.y * KV;
-    const bool warp_ok = __any_sync(0xffffffffu, ok);
 
+    if (tid < KV) s_df[tid] = (float)p.depths[min(d0 + tid, p.D - 1)];
+    __syncthreads();
     // Test points (transient_reconstruction.cuh:51) and their box.
     const float lx = p.xyz[3 * (size_t)c], ly = p.xyz[3 * (size_t)c + 1], lz = p.xyz[3 * (size_t)c + 2];
-    float px[YONLY ? 1 : KV], pz[YONLY ? 1 : KV];
-    f32x2_t pyp[KV / 2];
     float box[6] = {INFINITY, -INFINITY, INFINITY, -INFINITY, INFINITY, -INFINITY};
     bool finite = true;
-#pragma unroll
-    for (int k = 0; k < KV; k += 2) {
-        float y[2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const float df = (float)p.depths[min(d0 + k + h, p.D - 1)];
-            const float x = fma_rn(p.nx, df, lx), z = fma_rn(p.nz, df, lz);
-            y[h] = YONLY && !isfinite(df) ? NAN : fma_rn(p.ny, df, ly);  // (0 * df is NaN in x and z)
-            px[YONLY ? 0 : k + h] = x;
-            pz[YONLY ? 0 : k + h] = z;
-            finite = finite && isfinite(x) && isfinite(y[h]) && isfinite(z);
-            box[0] = fminf(box[0], x); box[1] = fmaxf(box[1], x);
-            box[2] = fminf(box[2], y[h]); box[3] = fmaxf(box[3], y[h]);
-            box[4] = fminf(box[4], z); box[5] = fmaxf(box[5], z);
-        }
-        pyp[k / 2] = pack2(y[0], y[1]);
+    // (0 * depth is NaN in x and z where the depth is not finite.)
+    auto point = [&](int k, float& x, float& y, float& z) {
+        const float df = s_df[k];
+        x = fma_rn(p.nx, df, lx);
+        y = YONLY && !isfinite(df) ? NAN : fma_rn(p.ny, df, ly);
+        z = fma_rn(p.nz, df, lz);
+    };
+    for (int k = 0; k < KV; ++k) {
+        float x, y, z;
+        point(k, x, y, z);
+        finite = finite && isfinite(x) && isfinite(y) && isfinite(z);
+        box[0] = fminf(box[0], x); box[1] = fmaxf(box[1], x);
+        box[2] = fminf(box[2], y); box[3] = fmaxf(box[3], y);
+        box[4] = fminf(box[4], z); box[5] = fmaxf(box[5], z);
     }
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
@@ -126,7 +133,16 @@ __global__ void __launch_bounds__(DepthTileParams::kThreads, YONLY ? 3 : 2) dept
     }
 #pragma unroll
     for (int k = 0; k < 2 * KV; ++k) s_sums[k * NT + tid] = 0.f;
+    if (cz == 0) s_lat[cx] = lx;
+    if (cx == 0) s_lat[16 + cz] = lz;
+    if (tid == 0) s_lat[32] = ly;
     const bool odd = __syncthreads_or(!finite);
+    const bool lattice = __syncthreads_and(YONLY && p.side > 0 && !odd && lx == s_lat[cx] && lz == s_lat[16 + cz] &&
+                                           ly == s_lat[32]);
+    // On a lattice: this thread's depth and row.
+    const uint32_t ld = d0 + (lane & 15), lr = (uint32_t)warp * 2 + (lane >> 4);
+    if (lattice) ok = ld < p.D && tile / sx * 16 + lr < p.side;
+    const bool warp_ok = __any_sync(0xffffffffu, ok);
 #pragma unroll
     for (int i = 0; i < 6; ++i)
         for (int w = 0; w < NW; ++w) box[i] = i & 1 ? fmaxf(box[i], s_box[i][w]) : fminf(box[i], s_box[i][w]);
@@ -197,6 +213,11 @@ __global__ void __launch_bounds__(DepthTileParams::kThreads, YONLY ? 3 : 2) dept
             }
             s_geo[gb + pos] = g;
             s_meta[gb + pos] = make_int4(bias, bias, (int)slot, 0);
+            if (lattice) {
+                float* dx = reinterpret_cast<float*>(s_dx + (gb + pos) * (KV / 4));
+#pragma unroll
+                for (int k = 0; k < KV; ++k) dx[k] = sub_rn(s_lat[k], g.x);
+            }
             s_cnt[gb + pos] = cnt;
             s_src[gb + pos] = p.rows + (size_t)l * p.pitch + a;
         }
@@ -228,35 +249,61 @@ __global__ void __launch_bounds__(DepthTileParams::kThreads, YONLY ? 3 : 2) dept
     f32x2_t accp[KV / 2];
 #pragma unroll
     for (int j = 0; j < KV / 2; ++j) accp[j] = 0ull;
-    const bool plain = !BOUNCE && p.t0 == 0.f;  // x = (2 d) rcp = d (2 rcp), exactly
-    const f32x2_t xs = plain ? pack2(2.f * rcp_dt, 2.f * rcp_dt) : pack2(rcp_dt, rcp_dt);
+    const f32x2_t xs = PLAIN ? pack2(2.f * rcp_dt, 2.f * rcp_dt) : pack2(rcp_dt, rcp_dt);  // (2 d) rcp = d (2 rcp)
     const f32x2_t two = pack2(2.f, 2.f), nt0p = pack2(neg_t0, neg_t0);
-    // Squared distances of depths (2 j, 2 j + 1) to scan point g.
-    auto square = [&](int j, const float4& g, f32x2_t dxc, f32x2_t dzc) -> f32x2_t {
-        const f32x2_t dy = sub_rn2(pyp[j], pack2(g.y, g.y));
-        if (!YONLY) {
-            dxc = sub_rn2(pack2(px[YONLY ? 0 : 2 * j], px[YONLY ? 0 : 2 * j + 1]), pack2(g.x, g.x));
-            dzc = sub_rn2(pack2(pz[YONLY ? 0 : 2 * j], pz[YONLY ? 0 : 2 * j + 1]), pack2(g.z, g.z));
+    // Path ratio of a packed pair of squared distances.
+    auto ratio = [&](f32x2_t q, float bounce) -> f32x2_t {
+        float q0, q1;
+        unpack2(q, q0, q1);
+        f32x2_t d = pack2(sqrt_approx(q0), sqrt_approx(q1));
+        if (!PLAIN) {
+            d = fma_rn2(d, two, nt0p);
+            if (BOUNCE) d = add_rn2(d, pack2(bounce, bounce));
         }
-        return fma_rn2(dzc, dzc, fma_rn2(dxc, dxc, mul_rn2(dy, dy)));
+        return mul_rn2(d, xs);
     };
-    auto walk = [&](uint32_t o, int n, auto&& sample) {
+    const float lpy = fma_rn(p.ny, s_df[lane & 15], s_lat[32]), lpz = s_lat[16 + lr];
+    auto walk_lattice = [&](uint32_t o, int n, auto&& sample) {
+#pragma unroll 4
+        for (int i = 0; i < n; ++i) {
+            const float4 g = s_geo[o + i];
+            const int4 m = s_meta[o + i];
+            const float dy = sub_rn(lpy, g.y), dz = sub_rn(lpz, g.z);
+            const float dy2 = mul_rn(dy, dy);
+            const f32x2_t dy2p = pack2(dy2, dy2), dzp = pack2(dz, dz);
+#pragma unroll
+            for (int j = 0; j < KV / 4; ++j) {
+                const ulonglong2 dx = s_dx[(o + i) * (KV / 4) + j];
+                accp[2 * j] = add_rn2(accp[2 * j], sample(ratio(fma_rn2(dzp, dzp, fma_rn2(dx.x, dx.x, dy2p)), g.w), m));
+                accp[2 * j + 1] =
+                    add_rn2(accp[2 * j + 1], sample(ratio(fma_rn2(dzp, dzp, fma_rn2(dx.y, dx.y, dy2p)), g.w), m));
+            }
+        }
+    };
+    auto walk_points = [&](uint32_t o, int n, auto&& sample) {
+        float px[YONLY ? 1 : KV], pz[YONLY ? 1 : KV];  // (made per stage: they would hold the lattice's registers)
+        f32x2_t pyp[KV / 2];
+#pragma unroll
+        for (int k = 0; k < KV; k += 2) {
+            float y0, y1;
+            point(k, px[YONLY ? 0 : k], y0, pz[YONLY ? 0 : k]);
+            point(k + 1, px[YONLY ? 0 : k + 1], y1, pz[YONLY ? 0 : k + 1]);
+            pyp[k / 2] = pack2(y0, y1);
+        }
 #pragma unroll 2
         for (int i = 0; i < n; ++i) {
             const float4 g = s_geo[o + i];
             const int4 m = s_meta[o + i];
             const float dx = sub_rn(px[0], g.x), dz = sub_rn(pz[0], g.z);
-            const f32x2_t dxc = pack2(dx, dx), dzc = pack2(dz, dz);
 #pragma unroll
             for (int j = 0; j < KV / 2; ++j) {
-                float q0, q1;
-                unpack2(square(j, g, dxc, dzc), q0, q1);
-                f32x2_t d = pack2(sqrt_approx(q0), sqrt_approx(q1));
-                if (!plain) {
-                    d = fma_rn2(d, two, nt0p);
-                    if (BOUNCE) d = add_rn2(d, pack2(g.w, g.w));
+                const f32x2_t dy = sub_rn2(pyp[j], pack2(g.y, g.y));
+                f32x2_t dxp = pack2(dx, dx), dzp = pack2(dz, dz);
+                if (!YONLY) {
+                    dxp = sub_rn2(pack2(px[YONLY ? 0 : 2 * j], px[YONLY ? 0 : 2 * j + 1]), pack2(g.x, g.x));
+                    dzp = sub_rn2(pack2(pz[YONLY ? 0 : 2 * j], pz[YONLY ? 0 : 2 * j + 1]), pack2(g.z, g.z));
                 }
-                accp[j] = add_rn2(accp[j], sample(mul_rn2(d, xs), m));
+                accp[j] = add_rn2(accp[j], sample(ratio(fma_rn2(dzp, dzp, fma_rn2(dxp, dxp, mul_rn2(dy, dy))), g.w), m));
             }
         }
     };
@@ -298,9 +345,12 @@ __global__ void __launch_bounds__(DepthTileParams::kThreads, YONLY ? 3 : 2) dept
             const int n = min((int)CH, grp.x - (int)(h * CH));
             if (warp_ok && !dead) {
                 const uint32_t o = gb + h * CH;
-                if (grp.y) walk(o, n, converted);
-                else if (whole) walk(o, n, clamped);
-                else walk(o, n, fast);
+                if (YONLY && lattice && !whole && !grp.y) walk_lattice(o, n, fast);
+                else if (YONLY && lattice && !grp.y) walk_lattice(o, n, clamped);
+                else if (YONLY && lattice) walk_lattice(o, n, converted);
+                else if (grp.y) walk_points(o, n, converted);
+                else if (whole) walk_points(o, n, clamped);
+                else walk_points(o, n, fast);
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_empty + 8 * buf);
@@ -321,16 +371,21 @@ __global__ void __launch_bounds__(DepthTileParams::kThreads, YONLY ? 3 : 2) dept
         }
     }
 
-    float* out = p.act + (size_t)c * p.D + d0;
-    if (p.chains == 1) {
-        if (ok) {
-#pragma unroll
-            for (int k = 0; k < KV; ++k)
-                if (d0 + k < p.D) out[k] = s_sums[(2 * k) * NT + tid];
+    // Sum k of this thread to its place.
+    auto store = [&](uint32_t k, float v) {
+        if (!ok) return;
+        if (lattice) {
+            const uint32_t ix = tile % sx * 16 + k, iz = tile / sx * 16 + lr;
+            if (ix < p.side) p.act[((size_t)iz * p.side + ix) * p.D + ld] = v;
+        } else if (d0 + k < p.D) {
+            p.act[(size_t)c * p.D + d0 + k] = v;
         }
+    };
+    if (p.chains == 1) {
+        for (uint32_t k = 0; k < (uint32_t)KV; ++k) store(k, s_sums[(2 * k) * NT + tid]);
         return;
     }
-    // The chains' sums, folded in order; CTA `rank` stores every chains-th depth.
+    // The chains' sums, folded in order; CTA `rank` stores every chains-th one.
     cluster_arrive();
     cluster_wait();
     const uint32_t kb = (uint32_t)__cvta_generic_to_shared(s_sums + tid);
@@ -341,15 +396,15 @@ __global__ void __launch_bounds__(DepthTileParams::kThreads, YONLY ? 3 : 2) dept
             fold(cluster_load(from), sum, comp);
             fold(-cluster_load(from + NT * 4u), sum, comp);
         }
-        if (ok && d0 + k < p.D) out[k] = sum;
+        store(k, sum);
     }
     cluster_arrive();
     cluster_wait();  // the others are through with this CTA's sums
 }
 
-template <bool YONLY, bool BOUNCE>
+template <bool YONLY, bool BOUNCE, bool PLAIN>
 fbp_status go_depth_tiles(fbp_context* ctx, const DepthTileParams& p, dim3 grid, cudaStream_t stream) {
-    auto kernel = depth_tile_kernel<YONLY, BOUNCE>;
+    auto kernel = depth_tile_kernel<YONLY, BOUNCE, PLAIN>;
     const size_t smem = DepthTileParams::kMeta + DepthTileParams::kSums + DepthTileParams::kWindowFloats * sizeof(float);
     FBP_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     if (p.chains == 1) {
@@ -406,13 +461,16 @@ fbp_status launch_depth_tiles(fbp_context* ctx, const fbp_recon_info& in, const 
     const uint64_t tiles = p.side ? (uint64_t)cdiv(side, 16) * cdiv(side, 16) : cdiv(L, DepthTileParams::kThreads);
     const dim3 grid((unsigned)tiles, cdiv(D, DepthTileParams::kDepths));
     const bool yonly = p.nx == 0.f && p.nz == 0.f, bounce = in.discard_first_last_bounces == 0;
-    p.chains = split_chains(ctx, tiles * grid.y, cdiv(L, DepthTileParams::kGroup), yonly ? 3 : 2);
+    p.chains = split_chains(ctx, tiles * grid.y, cdiv(L, DepthTileParams::kGroup), yonly ? 3 : 2, 0.8);
+    const bool plain = !bounce && p.t0 == 0.f;
     if (yonly) {
-        if (bounce) return go_depth_tiles<true, true>(ctx, p, grid, stream);
-        return go_depth_tiles<true, false>(ctx, p, grid, stream);
+        if (bounce) return go_depth_tiles<true, true, false>(ctx, p, grid, stream);
+        if (plain) return go_depth_tiles<true, false, true>(ctx, p, grid, stream);
+        return go_depth_tiles<true, false, false>(ctx, p, grid, stream);
     }
-    if (bounce) return go_depth_tiles<false, true>(ctx, p, grid, stream);
-    return go_depth_tiles<false, false>(ctx, p, grid, stream);
+    if (bounce) return go_depth_tiles<false, true, false>(ctx, p, grid, stream);
+    if (plain) return go_depth_tiles<false, false, true>(ctx, p, grid, stream);
+    return go_depth_tiles<false, false, false>(ctx, p, grid, stream);
 }
 
 template <typename S>
