@@ -45,22 +45,6 @@ __device__ __forceinline__ bool mbar_wait_parity(uint32_t bar, uint32_t parity) 
     return false;
 }
 
-// ---------------------------------------------------------------- cluster --
-
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-// Shared address of this CTA's `addr` in CTA `rank` of the cluster.
-__device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t rank) {
-    uint32_t r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ float cluster_load(uint32_t addr) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-    return v;
-}
-
 // One FP32 element of shared memory at a shared-state-space byte address.
 __device__ __forceinline__ float lds_f32(uint32_t addr) {
     float v;
@@ -130,6 +114,7 @@ struct ConfocalGatherParams {
     uint32_t slot_w;     // window width in elements (the sentinel zero sits at slot_w)
     int ch;              // scan points per window stage (a power of two <= 32)
     uint32_t chains;     // contiguous ranges of scan-point groups with compensated sums of their own
+    float* chain_sums;   // split tiles: [chains][sum, compensation][volume]
     const void* rows;    // [L][row_pitch] FP32
     SampleParams smp;    // used by the sampled (MIS) variant only
     float vs[3];         // voxel size (the voxel-scattering variant's extent)
@@ -175,9 +160,17 @@ fbp_status plan_window(const fbp_context* ctx, double ex, double ey, double ez, 
 // volume, whatever part of it a launch computes, so that slabs and batches sum
 // like the single call).
 uint32_t gather_chains(const fbp_context* ctx, const fbp_recon_info& in, size_t smem);
-// Chains for a launch of `tiles` voxel tiles that each walk `groups` groups,
-// occ CTAs to an SM, a CTA's set-up worth `setup` groups.
-uint32_t split_chains(const fbp_context* ctx, uint64_t tiles, uint64_t groups, int occ, double setup = 0.3);
+// Chains for a launch of `tiles` tiles (whose warps are `busy` to that part)
+// that each walk `groups` groups of `group_us` microseconds (at an SM's full
+// rate) into n outputs, occ CTAs to an SM.
+uint32_t split_chains(const fbp_context* ctx, uint64_t tiles, double busy, uint64_t groups, int occ, double group_us,
+                      uint64_t n);
+// Part of the warps of 16 x 16 (rows, slices) tiles that own voxels of a volume.
+double busy_warps(const uint32_t res[3]);
+constexpr double kGatherGroupUs = 6.3;  // 32 scan points x 4096 voxels
+// out[i] = the chains' sums [chains][sum, compensation][n], folded in order.
+fbp_status chain_sums(fbp_context* ctx, uint32_t chains, uint64_t n, cudaStream_t stream, float** sums);
+fbp_status fold_chains(fbp_context* ctx, const float* sums, uint32_t chains, uint64_t n, float* out, cudaStream_t stream);
 // CTAs of `smem` bytes of dynamic shared memory an SM holds, at most `most`.
 inline int resident_ctas(size_t smem, int most) {
     const size_t n = kSmSharedBytes / (smem + kCtaReservedShared);

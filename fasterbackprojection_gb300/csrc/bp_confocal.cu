@@ -216,11 +216,11 @@ fbp_status launch_confocal(fbp_context* ctx, const fbp_recon_info& in, const voi
         const bool free_walk = (sp - 1) * step + 1e-4 < vdiag;
         // ... and where none takes more (sp steps already pass the far end).
         p.scat_exact = free_walk && sp * step > vdiag + 1e-4;
-        if (p.chains > 1) return gather_scatter_cluster(ctx, p, grid, wp.smem, stream, sp, free_walk, bounce, wp.capped);
+        if (p.chains > 1) return gather_scatter_split(ctx, p, grid, wp.smem, stream, sp, free_walk, bounce, wp.capped);
         return gather_scatter(ctx, p, grid, wp.smem, stream, sp, free_walk, bounce, wp.capped);
     }
     if (smp) return gather_sampled(ctx, p, grid, wp.smem, stream, bounce, in.time_offset, wp.capped);
-    if (p.chains > 1) return gather_full_cluster(ctx, p, grid, wp.smem, stream, bounce, in.time_offset, wp.capped);
+    if (p.chains > 1) return gather_full_split(ctx, p, grid, wp.smem, stream, bounce, in.time_offset, wp.capped);
     return gather_full(ctx, p, grid, wp.smem, stream, bounce, in.time_offset, wp.capped);
 }
 
@@ -228,23 +228,28 @@ fbp_status launch_confocal(fbp_context* ctx, const fbp_recon_info& in, const voi
 
 // Chains (CTAs per tile) of a gather: 1 where the tiles alone keep every SM
 // busy, else as many as a model of the launch asks for.  The model, in units of
-// one group of scan points at an SM's full rate: the busiest SM's CTAs, each
-// with its share of the groups and 0.3 groups of set-up, at the rate of the
-// CTAs resident together (one or two reach 0.68 and 0.88 of three), and 0.3
-// CTAs for the uneven end.  Larger clusters only where they gain 2 %: clusters
-// of 7, 8, 14 and 16 CTAs leave part of a GPC's slots empty (128^2 x 1024 ->
-// 128^3: 12.2 ms with 2, 12.1 with 6, 12.9 with 8, 15.3 with 16; 14.3 with one
-// CTA per tile).  One CTA per tile against this rule: 32^2 x 256 -> 32^3 291
-// -> 48 us (12 chains), 64^2 x 512 -> 64^3 1133 -> 482 us (6).
-uint32_t split_chains(const fbp_context* ctx, uint64_t tiles, uint64_t groups, int occ, double setup) {
+// one group at an SM's full rate: the busiest SM's CTAs, each with its share of
+// the groups and half a group of set-up, at the rate of the CTAs resident
+// together (one or two reach 0.68 and 0.88 of three), the uneven end (a whole
+// CTA where tiles differ in their idle warps), and the sums' way through memory
+// and the fold's launch.  One CTA per tile against this rule: 32^2 x 256 ->
+// 32^3 328 -> 45 us (16 chains), 64^2 x 512 -> 64^3 1264 -> 432 us (7), 90^2 x
+// 700 -> 75 x 101 x 83 4028 -> 2189 us (16), 128^2 x 1024 -> 128^3 14.2 -> 11.5
+// ms (5), 8^2 x 16^2 x 512 -> 48^3 2251 -> 666 us (14).  The sums through the
+// shared memory of a cluster instead (at most 16 chains, and clusters leave
+// part of a GPC's slots empty): 48, 483, 2596 us, 11.9 ms, 728 us.
+uint32_t split_chains(const fbp_context* ctx, uint64_t tiles, double busy, uint64_t groups, int occ, double group_us,
+                      uint64_t n) {
     constexpr double kRate[kGatherCtasPerSm] = {0.68, 0.88, 1.0};
+    constexpr uint32_t kMaxChains = 32;
     uint32_t best = 1;
     double best_t = 0.0;
-    for (uint32_t c : {1u, 2u, 4u, 6u, 12u}) {
-        if (c > groups) break;
+    for (uint32_t c = 1; c <= std::min<uint64_t>(kMaxChains, groups); ++c) {
         const uint64_t per_sm = cdiv(tiles * c, (uint64_t)ctx->sm_count);
         const double rate = kRate[std::min<uint64_t>(per_sm, (uint64_t)occ) - 1] / kRate[occ - 1];
-        const double t = ((double)per_sm + 0.3) * ((double)groups / c + setup) / rate * (c == 12 ? 1.05 : 1.0);
+        const double ctas = busy < 1.0 ? (double)(tiles * c) * busy / ctx->sm_count + 1.0 : (double)per_sm + 0.3;
+        double t = ctas * ((double)((groups + c - 1) / c) + 0.5) / rate;
+        if (c > 1) t += (3.0 + 0.2 * c + (double)c * (double)n * 16.0 / 5.0e6) / group_us;  // 5 TB/s
         if (c == 1 || t < 0.98 * best_t) {
             best = c;
             best_t = t;
@@ -253,11 +258,45 @@ uint32_t split_chains(const fbp_context* ctx, uint64_t tiles, uint64_t groups, i
     return best;
 }
 
+double busy_warps(const uint32_t res[3]) {
+    return (double)cdiv(res[1], 8) * cdiv(res[2], 4) / ((double)cdiv(res[1], 16) * 2 * cdiv(res[2], 16) * 4);
+}
+
 uint32_t gather_chains(const fbp_context* ctx, const fbp_recon_info& in, size_t smem) {
+    static_assert(kWY == 2 && kWZ == 4, "busy_warps counts warps of 8 x 4 in tiles of 16 x 16");
     const uint64_t tiles = (uint64_t)cdiv(in.voxel_res[0], kKVFull) * cdiv(in.voxel_res[1], 8 * kWY) *
                            cdiv(in.voxel_res[2], 4 * kWZ);
-    return split_chains(ctx, tiles, cdiv(in.num_laser_targets, ConfocalGatherParams::kGroup),
-                        resident_ctas(smem, kGatherCtasPerSm));
+    return split_chains(ctx, tiles, busy_warps(in.voxel_res),
+                        cdiv(in.num_laser_targets, ConfocalGatherParams::kGroup), resident_ctas(smem, kGatherCtasPerSm),
+                        kGatherGroupUs, (uint64_t)in.voxel_res[0] * in.voxel_res[1] * in.voxel_res[2]);
+}
+
+fbp_status chain_sums(fbp_context* ctx, uint32_t chains, uint64_t n, cudaStream_t stream, float** sums) {
+    void* ws = nullptr;
+    FBP_TRY(workspace(ctx, WS_CHAIN_SUMS, (size_t)2 * chains * n * sizeof(float), stream, &ws));
+    *sums = static_cast<float*>(ws);
+    return FBP_OK;
+}
+
+__global__ void fold_chains_kernel(const float* __restrict__ sums, uint32_t chains, uint64_t n, float* __restrict__ out) {
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        float sum = 0.f, comp = 0.f;
+#pragma unroll 4
+        for (uint32_t c = 0; c < chains; ++c) {
+            const float s = sums[2 * c * n + i], e = -sums[(2 * c + 1) * n + i];
+            kahan_add(s, sum, comp);
+            kahan_add(e, sum, comp);
+        }
+        out[i] = sum;
+    }
+}
+
+fbp_status fold_chains(fbp_context* ctx, const float* sums, uint32_t chains, uint64_t n, float* out,
+                       cudaStream_t stream) {
+    const unsigned blocks = (unsigned)std::min<uint64_t>(cdiv(n, 256), (uint64_t)ctx->sm_count * 8);
+    fold_chains_kernel<<<blocks, 256, 0, stream>>>(sums, chains, n, out);
+    FBP_CHECK_LAUNCH(ctx, "fold_chains_kernel");
+    return FBP_OK;
 }
 
 // Tile grid of the confocal gather (also the MIS sampling tiles).

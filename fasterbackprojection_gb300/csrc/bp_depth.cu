@@ -26,7 +26,8 @@ struct DepthTileParams {
     uint32_t L, D, T, pitch;
     uint32_t side;           // > 0: the scan points are a side x side grid (tiles of 16 x 16), else runs of 256
     float nx, ny, nz, t0, dt;
-    uint32_t chains;
+    uint32_t chains;         // CTAs per tile, one per range of scan-point groups
+    float* chain_sums;       // chains > 1: [chains][sum, compensation][L][D]
 
     static constexpr int kGroup = 32, kPlanBufs = 4, kThreads = 256, kDepths = 16;
     static constexpr uint32_t kSlot = 256;           // widest window that is not the whole row
@@ -41,7 +42,7 @@ struct DepthTileParams {
     static constexpr uint32_t kMaxBins = (kWindowFloats / 2 - 8) / 4 * 4;
 };
 
-// A CTA (or a cluster of p.chains, one per range of scan-point groups) owns 256
+// A CTA (or p.chains of them, one per range of scan-point groups) owns 256
 // scan points' test points at 16 consecutive depths.  Pipeline, groups and
 // folds as in the confocal gather; the window width is the CTA's own, from the
 // box of its points (the host does not know the positions), and windows wider
@@ -57,7 +58,7 @@ struct DepthTileParams {
 // Bound by the issue port (a packed FP32 instruction holds it two cycles):
 // about 20 cycles per packed pair on a lattice, 30 otherwise.  64^2 x 512, 200
 // planes: one thread per point with rows in global memory 2867 us, a thread
-// per scan point 1200 us, the lattice 979 us.
+// per scan point 1200 us, the lattice 898 us.
 // PLAIN: no time offset and no bounces.
 template <bool YONLY, bool BOUNCE, bool PLAIN>
 __global__ void __launch_bounds__(DepthTileParams::kThreads, YONLY ? 3 : 2) depth_tile_kernel(DepthTileParams p) {
@@ -83,7 +84,7 @@ __global__ void __launch_bounds__(DepthTileParams::kThreads, YONLY ? 3 : 2) dept
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t rank = blockIdx.x % p.chains, tile = blockIdx.x / p.chains;
     // This thread's scan point (unless the tile is a lattice).
-    const uint32_t cx = (warp & 1) * 8 + (lane & 7), cz = (warp >> 1) * 4 + (lane >> 3), sx = (p.side + 15) / 16;
+    const uint32_t cx = (warp & 1) * 8 + (lane & 7), cz = (warp >> 1) * 4 + (lane >> 3), sx = p.side ? (p.side + 15) / 16 : 1;
     uint32_t c = tile * NT + tid;
     bool ok = c < p.L;
     if (p.side) {
@@ -323,12 +324,6 @@ __global__ void __launch_bounds__(DepthTileParams::kThreads, YONLY ? 3 : 2) dept
         return pack2(lds_f32((uint32_t)m.z + (min((uint32_t)(__float2int_rz(x0) - m.x), slot_w) << 2)),
                      lds_f32((uint32_t)m.z + (min((uint32_t)(__float2int_rz(x1) - m.x), slot_w) << 2)));
     };
-    auto fold = [](float part, float& sum, float& comp) {  // compensated (Kahan) addition
-        const float y = sub_rn(part, comp);
-        const float t = add_rn(sum, y);
-        comp = sub_rn(sub_rn(t, sum), y);
-        sum = t;
-    };
 
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();  // sentinels written
@@ -363,7 +358,7 @@ __global__ void __launch_bounds__(DepthTileParams::kThreads, YONLY ? 3 : 2) dept
             for (int h = 0; h < 2; ++h) {
                 float* s = s_sums + (2 * (2 * j + h)) * NT + tid;
                 float sum = s[0], comp = s[NT];
-                fold(part[h], sum, comp);
+                kahan_add(part[h], sum, comp);
                 s[0] = sum;
                 s[NT] = comp;
             }
@@ -371,61 +366,29 @@ __global__ void __launch_bounds__(DepthTileParams::kThreads, YONLY ? 3 : 2) dept
         }
     }
 
-    // Sum k of this thread to its place.
-    auto store = [&](uint32_t k, float v) {
-        if (!ok) return;
-        if (lattice) {
-            const uint32_t ix = tile % sx * 16 + k, iz = tile / sx * 16 + lr;
-            if (ix < p.side) p.act[((size_t)iz * p.side + ix) * p.D + ld] = v;
-        } else if (d0 + k < p.D) {
-            p.act[(size_t)c * p.D + d0 + k] = v;
-        }
-    };
-    if (p.chains == 1) {
-        for (uint32_t k = 0; k < (uint32_t)KV; ++k) store(k, s_sums[(2 * k) * NT + tid]);
-        return;
+    if (!ok) return;
+    const size_t n = (size_t)p.L * p.D;
+    float* out = p.chains == 1 ? p.act : p.chain_sums + (size_t)rank * 2 * n;
+    for (uint32_t k = 0; k < (uint32_t)KV; ++k) {
+        const uint32_t ix = tile % sx * 16 + k, iz = tile / sx * 16 + lr;
+        if (lattice ? ix >= p.side : d0 + k >= p.D) continue;
+        const size_t at = lattice ? ((size_t)iz * p.side + ix) * p.D + ld : (size_t)c * p.D + d0 + k;
+        out[at] = s_sums[(2 * k) * NT + tid];
+        if (p.chains > 1) out[n + at] = s_sums[(2 * k + 1) * NT + tid];
     }
-    // The chains' sums, folded in order; CTA `rank` stores every chains-th one.
-    cluster_arrive();
-    cluster_wait();
-    const uint32_t kb = (uint32_t)__cvta_generic_to_shared(s_sums + tid);
-    for (uint32_t k = rank; k < (uint32_t)KV; k += p.chains) {
-        float sum = 0.f, comp = 0.f;
-        for (uint32_t r = 0; r < p.chains; ++r) {
-            const uint32_t from = cluster_map(kb, r) + k * (2 * NT * 4u);
-            fold(cluster_load(from), sum, comp);
-            fold(-cluster_load(from + NT * 4u), sum, comp);
-        }
-        store(k, sum);
-    }
-    cluster_arrive();
-    cluster_wait();  // the others are through with this CTA's sums
 }
 
 template <bool YONLY, bool BOUNCE, bool PLAIN>
-fbp_status go_depth_tiles(fbp_context* ctx, const DepthTileParams& p, dim3 grid, cudaStream_t stream) {
+fbp_status go_depth_tiles(fbp_context* ctx, DepthTileParams p, dim3 grid, cudaStream_t stream) {
     auto kernel = depth_tile_kernel<YONLY, BOUNCE, PLAIN>;
     const size_t smem = DepthTileParams::kMeta + DepthTileParams::kSums + DepthTileParams::kWindowFloats * sizeof(float);
     FBP_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    if (p.chains == 1) {
-        kernel<<<grid, DepthTileParams::kThreads, smem, stream>>>(p);
-    } else {
-        FBP_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        cudaLaunchAttribute attr{};
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = p.chains;
-        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(grid.x * p.chains, grid.y, 1);
-        cfg.blockDim = dim3(DepthTileParams::kThreads);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = stream;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        FBP_TRY_CUDA(cudaLaunchKernelEx(&cfg, kernel, p));
-    }
+    const uint64_t n = (uint64_t)p.L * p.D;
+    if (p.chains > 1) FBP_TRY(chain_sums(ctx, p.chains, n, stream, &p.chain_sums));
+    grid.x *= p.chains;
+    kernel<<<grid, DepthTileParams::kThreads, smem, stream>>>(p);
     FBP_CHECK_LAUNCH(ctx, "depth_tile_kernel");
-    return FBP_OK;
+    return p.chains > 1 ? fold_chains(ctx, p.chain_sums, p.chains, n, p.act, stream) : FBP_OK;
 }
 
 // The confocal planes by tiles of 256 scan points x 16 depths.
@@ -461,7 +424,7 @@ fbp_status launch_depth_tiles(fbp_context* ctx, const fbp_recon_info& in, const 
     const uint64_t tiles = p.side ? (uint64_t)cdiv(side, 16) * cdiv(side, 16) : cdiv(L, DepthTileParams::kThreads);
     const dim3 grid((unsigned)tiles, cdiv(D, DepthTileParams::kDepths));
     const bool yonly = p.nx == 0.f && p.nz == 0.f, bounce = in.discard_first_last_bounces == 0;
-    p.chains = split_chains(ctx, tiles * grid.y, cdiv(L, DepthTileParams::kGroup), yonly ? 3 : 2, 0.8);
+    p.chains = split_chains(ctx, tiles * grid.y, 1.0, cdiv(L, DepthTileParams::kGroup), yonly ? 3 : 2, 5.0, (uint64_t)L * D);
     const bool plain = !bounce && p.t0 == 0.f;
     if (yonly) {
         if (bounce) return go_depth_tiles<true, true, false>(ctx, p, grid, stream);

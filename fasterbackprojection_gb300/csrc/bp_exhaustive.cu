@@ -2,8 +2,7 @@
 //
 // Replaces Laser::reconstructAABBExhaustive (Laser.cu:500-516) and
 // backprojectExhaustiveVoxel (transient_reconstruction.cuh:138-166).  Same
-// structure as the confocal gather: a CTA, or a cluster of them, per voxel
-// tile, the (laser, SPAD) pairs walked in groups, each pair's reachable
+// structure as the confocal gather: a CTA, or several, per voxel tile, the (laser, SPAD) pairs walked in groups, each pair's reachable
 // time-bin window copied to shared memory.  The pair index splits as l = ls / S, s = ls % S; the
 // reference splits by L (transient_reconstruction.cuh:147-148), which is the
 // same only when L == S and reads past the laser table otherwise.
@@ -29,6 +28,7 @@ struct ExhaustiveGatherParams {
     uint32_t row_pitch, slot_w;
     int ch;             // pairs per window stage (a power of two, 4..32)
     uint32_t chains;    // contiguous ranges of pair groups with compensated sums of their own, one CTA each
+    float* chain_sums;  // chains > 1: [chains][sum, compensation][volume]
     int exact_weights;  // 1: every weight by its own rcp.approx (FBP_WEIGHTS_REFERENCE)
 
     // Shared memory in front of the windows: the pipeline's barriers, then per
@@ -57,8 +57,8 @@ struct ExhaustiveGatherParams {
 // otherwise the planner guarantees that every bin lies inside its window.
 enum { EX_T0ZERO = 0, EX_FAST = 1, EX_EXACT = 2 };
 
-// One CTA of 32*WY*WZ threads (or a cluster of p.chains of them, one per range
-// of pair groups) owns a tile of KV x 8*WY x 4*WZ voxels, like the confocal
+// One CTA of 32*WY*WZ threads (or p.chains of them, one per range of pair
+// groups, their sums folded afterwards) owns a tile of KV x 8*WY x 4*WZ voxels, like the confocal
 // gather, with its pipeline: plans two groups ahead, windows by bulk copies,
 // no barrier across the CTA.
 // LB = 4: pairs are walked as (laser block of 4, SPAD, laser in block), so
@@ -216,7 +216,7 @@ exhaustive_gather_kernel(ExhaustiveGatherParams p) {
     };
 
     // A wait that ran out of polls (status FBP_ERR_TIMEOUT): the warp walks on
-    // to the cluster's barriers but touches nothing else.
+    // but touches nothing else.
     bool dead = false;
     auto wait = [&](uint32_t bar, uint32_t parity) {
         if (!dead && !mbar_wait_parity(bar, parity)) {
@@ -253,12 +253,6 @@ exhaustive_gather_kernel(ExhaustiveGatherParams p) {
         for (int j = 0; j < KV / 2; ++j) dlp[li][j] = 0ull;
     uint32_t cur_l = 0xFFFFFFFFu;
     const f32x2_t rdp = pack2(rcp_dt, rcp_dt), t0p = pack2(p.t0, p.t0);
-    auto fold = [](float part, float& sum, float& comp) {  // compensated (Kahan) addition
-        const float y = sub_rn(part, comp);
-        const float t = add_rn(sum, y);
-        comp = sub_rn(sub_rn(t, sum), y);
-        sum = t;
-    };
 
     // Distances of a point with the given x differences.
     auto point_dist = [&](float gy, float gz, auto&& dx, f32x2_t (&d)[KV / 2]) {
@@ -383,42 +377,21 @@ exhaustive_gather_kernel(ExhaustiveGatherParams p) {
         for (int j = 0; j < KV / 2; ++j) {
             float a0, a1;
             unpack2(accp[j], a0, a1);
-            fold(a0, ksum[2 * j], kcomp[2 * j]);
-            fold(a1, ksum[2 * j + 1], kcomp[2 * j + 1]);
+            kahan_add(a0, ksum[2 * j], kcomp[2 * j]);
+            kahan_add(a1, ksum[2 * j + 1], kcomp[2 * j + 1]);
             accp[j] = 0ull;
         }
     }
 
-    float* out = p.volume + ((size_t)vz * p.Vy + vy) * p.Vx + tx0;
-    if (p.chains == 1) {
-        if (row_ok) {
+    if (!row_ok) return;
+    const size_t at = ((size_t)vz * p.Vy + vy) * p.Vx + tx0, n = (size_t)p.Vx * p.Vy * p.Vz;
+    float* out = p.chains == 1 ? p.volume + at : p.chain_sums + (size_t)rank * 2 * n + at;
 #pragma unroll
-            for (int k = 0; k < KV; ++k)
-                if (tx0 + k < p.Vx) out[k] = ksum[k];
+    for (int k = 0; k < KV; ++k)
+        if (tx0 + k < p.Vx) {
+            out[k] = ksum[k];
+            if (p.chains > 1) out[n + k] = kcomp[k];
         }
-        return;
-    }
-    // The chains' sums, folded in order; CTA `rank` stores every chains-th voxel.
-    __syncthreads();  // every warp is through with the windows: their memory takes the sums, [2 KV][NT]
-#pragma unroll
-    for (int k = 0; k < KV; ++k) {
-        s_slots[(2 * k) * NT + tid] = ksum[k];
-        s_slots[(2 * k + 1) * NT + tid] = kcomp[k];
-    }
-    cluster_arrive();
-    cluster_wait();
-    const uint32_t kb = (uint32_t)__cvta_generic_to_shared(s_slots + tid);
-    for (uint32_t k = rank; k < (uint32_t)KV; k += p.chains) {
-        float sum = 0.f, comp = 0.f;
-        for (uint32_t c = 0; c < p.chains; ++c) {
-            const uint32_t from = cluster_map(kb, c) + k * (2 * NT * 4u);
-            fold(cluster_load(from), sum, comp);
-            fold(-cluster_load(from + NT * 4u), sum, comp);
-        }
-        if (row_ok && tx0 + k < p.Vx) out[k] = sum;
-    }
-    cluster_arrive();
-    cluster_wait();  // the others are through with this CTA's sums
 }
 
 namespace {
@@ -445,29 +418,15 @@ __global__ void pair_rows_kernel(float* __restrict__ rows, const S* __restrict__
 }
 
 template <int MODE, bool BOUNCE, bool CLAMP, int LB>
-fbp_status go_exhaustive(fbp_context* ctx, const ExhaustiveGatherParams& p, dim3 grid, size_t smem,
-                         cudaStream_t stream) {
+fbp_status go_exhaustive(fbp_context* ctx, ExhaustiveGatherParams p, dim3 grid, size_t smem, cudaStream_t stream) {
     auto kernel = exhaustive_gather_kernel<kKV, kWY, kWZ, MODE, BOUNCE, CLAMP, LB>;
     FBP_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    if (p.chains == 1) {
-        kernel<<<grid, 32 * kWY * kWZ, smem, stream>>>(p);
-    } else {
-        FBP_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        cudaLaunchAttribute attr{};
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = p.chains;
-        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(grid.x * p.chains, grid.y, grid.z);
-        cfg.blockDim = dim3(32 * kWY * kWZ);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = stream;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        FBP_TRY_CUDA(cudaLaunchKernelEx(&cfg, kernel, p));
-    }
+    const uint64_t n = (uint64_t)p.Vx * p.Vy * p.Vz;
+    if (p.chains > 1) FBP_TRY(chain_sums(ctx, p.chains, n, stream, &p.chain_sums));
+    grid.x *= p.chains;
+    kernel<<<grid, 32 * kWY * kWZ, smem, stream>>>(p);
     FBP_CHECK_LAUNCH(ctx, "exhaustive_gather_kernel");
-    return FBP_OK;
+    return p.chains > 1 ? fold_chains(ctx, p.chain_sums, p.chains, n, p.volume, stream) : FBP_OK;
 }
 
 template <int MODE, int LB>
@@ -547,16 +506,14 @@ fbp_status launch_exhaustive(fbp_context* ctx, const fbp_recon_info& in, const v
     const bool blocks = wp.ch % 4 == 0 && (L + 3) / 4 * 4 * 3 <= L * 4;
     const uint64_t groups = ((uint64_t)(blocks ? (L + 3) / 4 * 4 : L) * Sn + ExhaustiveGatherParams::kGroup - 1) /
                             ExhaustiveGatherParams::kGroup;
-    size_t smem = wp.smem;
-    p.chains = split_chains(ctx, (uint64_t)cdiv(Vx, kKV) * cdiv(Vy, 8 * kWY) * cdiv(Vz, 4 * kWZ), groups,
-                            resident_ctas(smem, kExhaustiveCtasPerSm));
-    if (p.chains > 1)  // the chains' sums take the windows' memory at the end
-        smem = std::max(smem, ExhaustiveGatherParams::meta_bytes(kKV) + (size_t)2 * kKV * 32 * kWY * kWZ * sizeof(float));
+    p.chains = split_chains(ctx, (uint64_t)cdiv(Vx, kKV) * cdiv(Vy, 8 * kWY) * cdiv(Vz, 4 * kWZ),
+                            busy_warps(in.voxel_res), groups,
+                            resident_ctas(wp.smem, kExhaustiveCtasPerSm), 3.2, (uint64_t)Vx * Vy * Vz);
     p.exact_weights = ctx->weight_mode == FBP_WEIGHTS_REFERENCE;
     dim3 grid(cdiv(Vx, kKV), cdiv(Vy, 8 * kWY), cdiv(Vz, 4 * kWZ));
     const bool bounce = in.discard_first_last_bounces == 0;
-    if (blocks) return dispatch_exhaustive<4>(ctx, p, grid, smem, stream, bounce, in.time_offset, wp.capped);
-    return dispatch_exhaustive<1>(ctx, p, grid, smem, stream, bounce, in.time_offset, wp.capped);
+    if (blocks) return dispatch_exhaustive<4>(ctx, p, grid, wp.smem, stream, bounce, in.time_offset, wp.capped);
+    return dispatch_exhaustive<1>(ctx, p, grid, wp.smem, stream, bounce, in.time_offset, wp.capped);
 }
 
 }  // namespace

@@ -288,7 +288,7 @@ __device__ __forceinline__ void confocal_stage(const ScanPlan pl, int nl, float 
     }
 }
 
-// The main kernel.  One CTA of 32*WY*WZ threads (or a cluster of CS of them)
+// The main kernel.  One CTA of 32*WY*WZ threads (or several, one per chain)
 // owns a tile of KV (x) x 8*WY (rows) x 4*WZ (depth slices) voxels; a warp
 // covers 8 rows x 4 slices, a thread KV consecutive voxels along x.  Scan
 // points (or, SAMPLED, K scan points drawn per tile) are taken in groups of 32:
@@ -303,12 +303,11 @@ __device__ __forceinline__ void confocal_stage(const ScanPlan pl, int nl, float 
 //
 // Chains: the groups are cut into p.chains contiguous ranges, each with its
 // own compensated sums; the chains' sums are folded, compensated, in order.
-// CLUSTER: one CTA of a cluster of p.chains per chain, the fold at the end
-// through distributed shared memory (every CTA folds and stores its share of
-// the tile's voxels).  Otherwise one CTA walks the chains one after the other
-// with the totals in `totals` (global, [2 KV][threads] per CTA): the same
-// operations in the same order, so the volume is the same bit for bit.
-template <int KV, int WY, int WZ, int PATH, bool BOUNCE, bool SAMPLED, bool CLAMP, bool CLUSTER>
+// SPLIT: one CTA per chain, which leaves its sums in p.chain_sums for
+// fold_chains.  Otherwise one CTA walks the chains one after the other with the
+// totals in `totals` (global, [2 KV][threads] per CTA): the same operations in
+// the same order, so the volume is the same bit for bit.
+template <int KV, int WY, int WZ, int PATH, bool BOUNCE, bool SAMPLED, bool CLAMP, bool SPLIT>
 __device__ __forceinline__ void confocal_tile(const ConfocalGatherParams& p, uint32_t bx, uint32_t by, uint32_t bz,
                                               unsigned long long tile_id, float* totals = nullptr) {
     constexpr int NT = 32 * WY * WZ, NW = WY * WZ;
@@ -357,7 +356,7 @@ __device__ __forceinline__ void confocal_tile(const ConfocalGatherParams& p, uin
     const float scat_ext = is_scatter(PATH) ? mul_rn(0.5f, sqrt_approx(ref_dot3(p.vs[0], p.vs[1], p.vs[2]))) : 0.f;
     const float scat_step = is_scatter(PATH) ? add_rn(p.dt, FBP_EPS) : 0.f;
 
-    const uint32_t rank = CLUSTER ? blockIdx.x % p.chains : 0;  // this CTA's place in the cluster (along x)
+    const uint32_t rank = SPLIT ? blockIdx.x % p.chains : 0;  // this CTA's chain
     if (tid == 0) {
         for (uint32_t b = 0; b < NB; ++b) {
             mbar_init(bar_full + 8 * b, 1);
@@ -431,8 +430,8 @@ __device__ __forceinline__ void confocal_tile(const ConfocalGatherParams& p, uin
     const uint32_t ngroups = (nitems + GRP - 1) / GRP;
     // Chain k: groups [k ngroups / chains, (k + 1) ngroups / chains).
     auto chain_begin = [&](uint32_t k) { return (uint32_t)((uint64_t)k * ngroups / p.chains); };
-    const uint32_t g0 = CLUSTER ? chain_begin(rank) : 0;
-    const uint32_t mine = CLUSTER ? chain_begin(rank + 1) - g0 : ngroups;  // groups of this CTA, from g0
+    const uint32_t g0 = SPLIT ? chain_begin(rank) : 0;
+    const uint32_t mine = SPLIT ? chain_begin(rank + 1) - g0 : ngroups;  // groups of this CTA, from g0
     const uint32_t sub = GRP / CH;                                 // stages per group
     const uint32_t nstages = mine * sub;
     const bool warp_ok = __any_sync(0xffffffffu, row_ok);          // the warp owns voxels of the volume
@@ -581,7 +580,7 @@ __device__ __forceinline__ void confocal_tile(const ConfocalGatherParams& p, uin
     // memory behind the zero slot, [2 KV][NT] so a warp's accesses are
     // consecutive words.
     constexpr bool KSMEM = kahan_smem_bytes(KV, NT) > 0;
-    static_assert(!CLUSTER || KSMEM, "the cluster folds compensated sums in shared memory");
+    static_assert(!SPLIT || KSMEM, "a split tile keeps its compensated sums in shared memory");
     float* s_kahan = reinterpret_cast<float*>(
         smem_raw + ((slots_off + (size_t)NB * CH * slot_stride * sizeof(float) + 15) & ~size_t(15)));
     float acc[KV], ksum[KSMEM ? 1 : KV], kcomp[KSMEM ? 1 : KV];
@@ -594,13 +593,6 @@ __device__ __forceinline__ void confocal_tile(const ConfocalGatherParams& p, uin
 #pragma unroll
         for (int k = 0; k < KV; ++k) ksum[k] = kcomp[k] = 0.f;
     }
-    // Compensated (Kahan) addition of a group's sum.
-    auto fold = [](float part, float& sum, float& comp) {
-        const float y = sub_rn(part, comp);
-        const float t = add_rn(sum, y);
-        comp = sub_rn(sub_rn(t, sum), y);
-        sum = t;
-    };
     // A previous tile's writes to this memory before the bulk copies' writes.
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();  // barriers initialised, sentinels written
@@ -637,22 +629,22 @@ __device__ __forceinline__ void confocal_tile(const ConfocalGatherParams& p, uin
         for (int k = 0; k < KV; ++k) {
             if constexpr (KSMEM) {
                 float sk = s_kahan[(2 * k) * NT + tid], ck = s_kahan[(2 * k + 1) * NT + tid];
-                fold(mul_rn(acc[k], scale), sk, ck);
+                kahan_add(mul_rn(acc[k], scale), sk, ck);
                 s_kahan[(2 * k) * NT + tid] = sk;
                 s_kahan[(2 * k + 1) * NT + tid] = ck;
             } else {
-                fold(mul_rn(acc[k], scale), ksum[k], kcomp[k]);
+                kahan_add(mul_rn(acc[k], scale), ksum[k], kcomp[k]);
             }
             acc[k] = 0.f;
         }
-        if constexpr (KSMEM && !CLUSTER) {
+        if constexpr (KSMEM && !SPLIT) {
             // The end of a chain, of several: its sums to the totals.
             while (p.chains > 1 && chain < p.chains && gi + 1 == chain_begin(chain + 1)) {
                 for (int k = 0; k < KV; ++k) {
                     float* t = totals + ((size_t)blockIdx.x * KV + k) * (2 * NT) + tid;
                     float sum = chain ? t[0] : 0.f, comp = chain ? t[NT] : 0.f;
-                    fold(s_kahan[(2 * k) * NT + tid], sum, comp);
-                    fold(-s_kahan[(2 * k + 1) * NT + tid], sum, comp);
+                    kahan_add(s_kahan[(2 * k) * NT + tid], sum, comp);
+                    kahan_add(-s_kahan[(2 * k + 1) * NT + tid], sum, comp);
                     t[0] = sum;
                     t[NT] = comp;
                     s_kahan[(2 * k) * NT + tid] = s_kahan[(2 * k + 1) * NT + tid] = 0.f;
@@ -662,22 +654,17 @@ __device__ __forceinline__ void confocal_tile(const ConfocalGatherParams& p, uin
         }
     }
 
-    if constexpr (CLUSTER) {
-        cluster_arrive();
-        cluster_wait();  // every chain's sums are in their CTA's shared memory
-        const uint32_t kb = (uint32_t)__cvta_generic_to_shared(s_kahan + tid);
-        float* out = p.volume + ((size_t)vz * p.Vy + vy) * p.Vx + tx0;
-        for (uint32_t k = rank; k < (uint32_t)KV; k += p.chains) {
-            float sum = 0.f, comp = 0.f;
-            for (uint32_t c = 0; c < p.chains; ++c) {
-                const uint32_t src = cluster_map(kb, c) + k * (2 * NT * 4u);
-                fold(cluster_load(src), sum, comp);
-                fold(-cluster_load(src + NT * 4u), sum, comp);
-            }
-            if (row_ok && tx0 + k < p.Vx) out[k] = sum;
+    if constexpr (SPLIT) {
+        if (row_ok) {
+            const size_t n = (size_t)p.Vx * p.Vy * p.Vz;
+            float* sums = p.chain_sums + (size_t)rank * 2 * n + ((size_t)vz * p.Vy + vy) * p.Vx + tx0;
+#pragma unroll
+            for (int k = 0; k < KV; ++k)
+                if (tx0 + k < p.Vx) {
+                    sums[k] = s_kahan[(2 * k) * NT + tid];
+                    sums[n + k] = s_kahan[(2 * k + 1) * NT + tid];
+                }
         }
-        cluster_arrive();
-        cluster_wait();  // the others are through with this CTA's sums
     } else if (row_ok) {
         float* out = p.volume + ((size_t)vz * p.Vy + vy) * p.Vx + tx0;
 #pragma unroll
@@ -695,12 +682,12 @@ __device__ __forceinline__ void confocal_tile(const ConfocalGatherParams& p, uin
 // Registers for three CTAs of 256 threads (80 each).
 constexpr int gather_ctas(int threads) { return threads > 256 ? 1 : kGatherCtasPerSm; }
 
-template <int KV, int WY, int WZ, int PATH, bool BOUNCE, bool SAMPLED, bool CLAMP, bool CLUSTER = false>
+template <int KV, int WY, int WZ, int PATH, bool BOUNCE, bool SAMPLED, bool CLAMP, bool SPLIT = false>
 __global__ void __launch_bounds__(32 * WY * WZ, gather_ctas(32 * WY * WZ))
 confocal_gather_kernel(ConfocalGatherParams p) {
-    const uint32_t cs = CLUSTER ? p.chains : 1, bx = blockIdx.x / cs;
+    const uint32_t cs = SPLIT ? p.chains : 1, bx = blockIdx.x / cs;
     const unsigned long long tile_id = ((unsigned long long)blockIdx.z * gridDim.y + blockIdx.y) * (gridDim.x / cs) + bx;
-    confocal_tile<KV, WY, WZ, PATH, BOUNCE, SAMPLED, CLAMP, CLUSTER>(p, bx, blockIdx.y, blockIdx.z, tile_id);
+    confocal_tile<KV, WY, WZ, PATH, BOUNCE, SAMPLED, CLAMP, SPLIT>(p, bx, blockIdx.y, blockIdx.z, tile_id);
 }
 
 // Persistent form for a batch of captures: CTAs pull (capture, tile) work items

@@ -88,6 +88,7 @@ enum WorkspaceSlot {
     WS_MLP_PROFILES,    // learned proposal: pooled cluster profiles, centres, scale
     WS_MLP_PARTIALS,    // learned proposal: per-CTA gradient partials
     WS_MIS_VIRTUAL,     // cluster MIS control variate: virtual capture + two partial volumes
+    WS_CHAIN_SUMS,      // split gathers: the chains' sums and compensations
     WS_NUM_SLOTS
 };
 
@@ -194,6 +195,13 @@ __device__ __forceinline__ float sub_rn(float a, float b) {
     float r;
     asm("sub.rn.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
     return r;
+}
+// Compensated (Kahan) addition.
+__device__ __forceinline__ void kahan_add(float part, float& sum, float& comp) {
+    const float y = sub_rn(part, comp);
+    const float t = add_rn(sum, y);
+    comp = sub_rn(sub_rn(t, sum), y);
+    sum = t;
 }
 // a + p (round to nearest) where x < y, else a unchanged: one compare and a
 // predicated add.

@@ -1,6 +1,5 @@
-"""The confocal gather's chains: small volumes split the scan points of a voxel
-tile over the CTAs of a cluster (1, 2, 4, 6 or 12 chains), each with its own
-compensated sums.
+"""The gathers' chains: small volumes split the scan points (or pairs) of a voxel
+tile over several CTAs (1 to 32 chains), each with its own compensated sums.
 
   * against the FP64 oracle with the GPU's bins: 1e-6 relative L2, the bound of
     the unsplit gather (FP32 sums of at most 32 terms and compensated folds:
