@@ -13,15 +13,19 @@
 // No FFT, no host round trip, the filter runs in place on device data.
 #include "fbp_internal.cuh"
 
+#include <algorithm>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 namespace fbp {
 
 constexpr int kMaxTaps = 2048;
-// Taps by value (kernel parameters): concurrent calls share no state.
+// Taps by value (kernel parameters, no longer than the kernel needs): concurrent
+// calls share no state.
+template <int N>
 struct FilterTaps {
-    float w[kMaxTaps];
+    float w[N];
 };
 
 // One CTA filters one series at a time (grid-stride over series).  Shared
@@ -37,13 +41,13 @@ struct FilterTaps {
 // are zero-padded to a multiple of 2Q (zero terms), and S is preceded by F
 // zero slots (3Q <= F < 4Q, making S-index + F of every window start a
 // multiple of Q) so the last, unused window loads stay in bounds.
-// Rows of S are 8 floats; the two 16-byte halves of row k trade places when
-// bit 2 of k is set, so the 16-byte loads of 8 consecutive threads (8
-// consecutive rows) fall in 8 different bank groups.
-constexpr int kFilterQ = 8;
+// Rows of S are 8 floats, 12 apart, so the 16-byte loads of 8 consecutive
+// threads (8 consecutive rows) fall in 8 different bank groups and every load
+// of a thread is an immediate offset from its first row (swapping the halves of
+// rows 8 floats apart cost 12 integer instructions per bin).
+constexpr int kFilterQ = 8, kFilterRow = 12;
 
-// 8k + 4 (half ^ bit 2 of k): bit 2 of 8k is clear, so OR and XOR compose.
-__device__ __forceinline__ int srow_addr(int k, int half) { return ((k << 3) | (k & 4)) ^ (half << 2); }
+__device__ __forceinline__ int srow_addr(int k, int half) { return k * kFilterRow + half * 4; }
 
 __device__ __forceinline__ void srow_load(const float* sh, int k, float (&v)[kFilterQ]) {
     const float4 a = *reinterpret_cast<const float4*>(sh + srow_addr(k, 0));
@@ -77,40 +81,82 @@ __device__ __forceinline__ void filter_block_shared(const float* s_taps, int J, 
 // NJ > 0: exactly NJ blocks of 2Q taps, unrolled, each FMA reading its tap
 // from the kernel parameters (constant bank; zero past the last tap).
 // NJ == 0: any tap count, taps from the shared copy.
-template <int NJ>
-__global__ void __launch_bounds__(128) filter_h_kernel(float* __restrict__ data, uint64_t nseries, uint32_t T, int n,
+// Bound by the FMA issue: 112 taps per bin.  The fill used to take a fifth of
+// the instructions (circular index, clamp and border per sample); now a thread
+// works out the slots of its first kPrefetch half rows once, and loads the next
+// series' samples before this one is filtered.
+// 65536 x 1024: 371 -> 298 us (FMA pipe 69 %, issue
+// 85 %).
+constexpr int kFilterThreads = 128, kPrefetch = 3;
+constexpr int filter_taps(int nj) { return nj > 0 ? 2 * kFilterQ * nj : kMaxTaps; }
+
+template <int NJ, int nt>
+__global__ void __launch_bounds__(nt, 1024 / nt) filter_h_kernel(float* __restrict__ data, uint64_t nseries, uint32_t T, int n,
                                                        int R, int pad, int edge, int F, int ntp, int rows,
-                                                       const __grid_constant__ FilterTaps taps) {
+                                                       const __grid_constant__ FilterTaps<filter_taps(NJ)> taps) {
     constexpr int Q = kFilterQ;
     extern __shared__ __align__(16) float sh[];  // taps (ntp, zero-padded), then `rows` rows of S
     const int E = n + 2 * R;
-    const int ntaps = 2 * R + 1;
     float* s_taps = sh;
     float* sser = sh + ntp;
-    for (int j = threadIdx.x; j < ntp; j += blockDim.x) s_taps[j] = j < ntaps ? taps.w[j] : 0.f;
+    if (NJ == 0)
+        for (int j = threadIdx.x; j < ntp; j += nt) s_taps[j] = taps.w[j];
+    // Slot i of S (S index): the sample it takes and whether it does.  Slots
+    // before S[0] and past S[E - 1] are zero; a slot whose signal index falls
+    // outside [0, T) takes the clamped border sample (edge) or zero.
+    auto slot = [&](int i, bool& keep) -> uint32_t {
+        int k = i - R;  // circular index: -R <= k < n + R for i in [0, E), R < n
+        k += k < 0 ? n : 0;
+        k -= k >= n ? n : 0;
+        const int u = k - pad;  // signal index
+        keep = i >= 0 && i < E && (edge || (u >= 0 && u < (int)T));
+        return (uint32_t)min(max(u, 0), (int)T - 1);
+    };
+    // The slots of this thread's first kPrefetch half rows (the same for every
+    // series): half row g holds slots 4 g - F and on.
+    uint32_t from[kPrefetch][4], kept = 0;
+#pragma unroll
+    for (int u = 0; u < kPrefetch; ++u)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            bool keep;
+            from[u][b] = slot(4 * ((int)threadIdx.x + u * nt) + b - F, keep);
+            kept |= (uint32_t)keep << (4 * u + b);
+        }
+    auto store_half = [&](int g, const float (&v)[4]) {
+        *reinterpret_cast<float4*>(sser + srow_addr(g >> 1, g & 1)) = make_float4(v[0], v[1], v[2], v[3]);
+    };
+    float pre[kPrefetch][4];
+    auto prefetch = [&](const float* h) {
+#pragma unroll
+        for (int u = 0; u < kPrefetch; ++u)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) pre[u][b] = h[from[u][b]];
+    };
+    if (blockIdx.x < nseries) prefetch(data + (uint64_t)blockIdx.x * T);
     for (uint64_t s = blockIdx.x; s < nseries; s += gridDim.x) {
         float* h = data + s * T;
-        // Fill one 16-byte half row (four consecutive slots) per thread and
-        // step.  Slots before S[0] and past S[E - 1] are zero; a slot whose
-        // signal index falls outside [0, T) takes the clamped border sample
-        // (edge) or zero, so every load is in bounds and unconditional.
-        for (int g = threadIdx.x; g < 2 * rows; g += blockDim.x) {
+#pragma unroll
+        for (int u = 0; u < kPrefetch; ++u) {
+            const int g = threadIdx.x + u * nt;
+            float v[4];
+#pragma unroll
+            for (int b = 0; b < 4; ++b) v[b] = kept >> (4 * u + b) & 1 ? pre[u][b] : 0.f;
+            if (g < 2 * rows) store_half(g, v);
+        }
+        for (int g = threadIdx.x + kPrefetch * nt; g < 2 * rows; g += nt) {
             float v[4];
 #pragma unroll
             for (int b = 0; b < 4; ++b) {
-                const int i = 4 * g + b - F;  // S index
-                int k = i - R;                // circular index: -R <= k < n + R for i in [0, E), R < n
-                k += k < 0 ? n : 0;
-                k -= k >= n ? n : 0;
-                const int u = k - pad;  // signal index
-                const float x = h[min(max(u, 0), (int)T - 1)];
-                const bool keep = i >= 0 && i < E && (edge || (u >= 0 && u < (int)T));
-                v[b] = keep ? x : 0.f;
+                bool keep;
+                const uint32_t u = slot(4 * g + b - F, keep);
+                v[b] = keep ? h[u] : 0.f;
             }
-            *reinterpret_cast<float4*>(sser + srow_addr(g >> 1, g & 1)) = make_float4(v[0], v[1], v[2], v[3]);
+            store_half(g, v);
         }
+        if (s + gridDim.x < nseries) prefetch(data + (s + gridDim.x) * T);
         __syncthreads();
-        for (int t0 = threadIdx.x * Q; t0 < (int)T; t0 += blockDim.x * Q) {
+        for (int t0 = threadIdx.x * Q; t0 < (int)T; t0 += nt * Q) {
             // out[t0 + q] = sum_j taps[j] * S[b0 - j + q], b0 = t0 + pad + 2R; in slots
             // b = b0 + F (a multiple of Q), window of block J: slots b - J - Q .. b - J + Q.
             const int kb = (t0 + pad + 2 * R + F) >> 3;  // row of slot b
@@ -193,8 +239,6 @@ fbp_status filter_h_device(fbp_context* ctx, float* data, uint64_t nseries, uint
     std::vector<float> taps;
     int R = 0, pad = 0, n = 0;
     FBP_TRY(filter_h_taps(T, delta_t, wl_mean, wl_sigma, taps, R, pad, n));
-    FilterTaps tp{};
-    for (size_t j = 0; j < taps.size(); ++j) tp.w[j] = taps[j];
     constexpr int Q = kFilterQ;
     const int ntp = (2 * R + 1 + 2 * Q - 1) / (2 * Q) * (2 * Q);
     if (ntp > kMaxTaps) return set_error(FBP_ERR_UNSUPPORTED, "filter_H: filter longer than the tap table");
@@ -202,30 +246,46 @@ fbp_status filter_h_device(fbp_context* ctx, float* data, uint64_t nseries, uint
     const int F = 3 * Q + (Q - (pad + 2 * R + 3 * Q) % Q) % Q;
     // Highest slot read: t0 + pad + 2R + F + Q - 1 with t0 <= T - 1 (< E + F + Q).
     const int rows = (n + 2 * R + F + Q) / Q + 1;
-    const size_t smem = ((size_t)ntp + (size_t)Q * rows) * sizeof(float);
+    const size_t smem = ((size_t)ntp + (size_t)kFilterRow * rows) * sizeof(float);
     if (smem > (size_t)ctx->smem_optin) return set_error(FBP_ERR_UNSUPPORTED, "filter_H: series too long for one CTA");
-    const unsigned blocks = (unsigned)std::min<uint64_t>(nseries, (uint64_t)ctx->sm_count * 16);
-    auto go = [&](auto kernel) -> fbp_status {
+    taps.resize((size_t)ntp, 0.f);
+    auto launch = [&](auto nj, auto nt) -> fbp_status {
+        constexpr int NJ = decltype(nj)::value, threads = decltype(nt)::value;
+        auto kernel = filter_h_kernel<NJ, threads>;
+        FilterTaps<filter_taps(NJ)> tp;
+        std::copy(taps.begin(), taps.end(), tp.w);
         FBP_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kernel<<<blocks, 128, smem, stream>>>(data, nseries, T, n, R, pad, border == FBP_BORDER_EDGE, F, ntp, rows, tp);
+        // One CTA per resident slot (64 registers a thread), or twice as many
+        // where that leaves each only a few series.
+        const size_t fit = std::min<size_t>(std::min<size_t>(32, 1024 / threads), kSmSharedBytes / (smem + kCtaReservedShared));
+        const uint64_t slots = (uint64_t)ctx->sm_count * std::max<size_t>(1, fit);
+        const unsigned blocks = (unsigned)std::min<uint64_t>(nseries, nseries < 8 * slots ? 2 * slots : slots);
+        kernel<<<blocks, threads, smem, stream>>>(data, nseries, T, n, R, pad, border == FBP_BORDER_EDGE, F, ntp, rows, tp);
         FBP_CHECK_LAUNCH(ctx, "filter_h_kernel");
         return FBP_OK;
+    };
+    // Threads for one pass over a series (8 bins each): 65536 x 128 with 128
+    // threads 65.7 us, with 32 38.7 us.
+    auto go = [&](auto nj) -> fbp_status {
+        if (T <= 32 * Q) return launch(nj, std::integral_constant<int, 32>{});
+        if (T <= 64 * Q) return launch(nj, std::integral_constant<int, 64>{});
+        return launch(nj, std::integral_constant<int, kFilterThreads>{});
     };
     // Unrolled forms for 2 .. 12 blocks of 16 taps (wavelengths of about 2
     // to 20 bins; 10 bins, the reference's default, gives 107 taps = 7 blocks).
     switch (ntp / (2 * Q)) {
-        case 2: return go(filter_h_kernel<2>);
-        case 3: return go(filter_h_kernel<3>);
-        case 4: return go(filter_h_kernel<4>);
-        case 5: return go(filter_h_kernel<5>);
-        case 6: return go(filter_h_kernel<6>);
-        case 7: return go(filter_h_kernel<7>);
-        case 8: return go(filter_h_kernel<8>);
-        case 9: return go(filter_h_kernel<9>);
-        case 10: return go(filter_h_kernel<10>);
-        case 11: return go(filter_h_kernel<11>);
-        case 12: return go(filter_h_kernel<12>);
-        default: return go(filter_h_kernel<0>);
+        case 2: return go(std::integral_constant<int, 2>{});
+        case 3: return go(std::integral_constant<int, 3>{});
+        case 4: return go(std::integral_constant<int, 4>{});
+        case 5: return go(std::integral_constant<int, 5>{});
+        case 6: return go(std::integral_constant<int, 6>{});
+        case 7: return go(std::integral_constant<int, 7>{});
+        case 8: return go(std::integral_constant<int, 8>{});
+        case 9: return go(std::integral_constant<int, 9>{});
+        case 10: return go(std::integral_constant<int, 10>{});
+        case 11: return go(std::integral_constant<int, 11>{});
+        case 12: return go(std::integral_constant<int, 12>{});
+        default: return go(std::integral_constant<int, 0>{});
     }
 }
 
