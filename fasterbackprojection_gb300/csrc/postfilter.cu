@@ -71,27 +71,43 @@ __global__ void minmax_partial_kernel(const float* __restrict__ v, uint64_t n, f
     }
 }
 
-// Pass 2: one block folds the partials into mm[0] = min, mm[1] = max.
-__global__ void minmax_final_kernel(const float* __restrict__ partials, int nblocks, float* __restrict__ mm) {
-    float mn = INFINITY, mx = -INFINITY;
-    for (int i = threadIdx.x; i < nblocks; i += blockDim.x) {
-        mn = fminf(mn, partials[2 * i]);
-        mx = fmaxf(mx, partials[2 * i + 1]);
+// Pass 2: normalizeReconstruction, v = (v - min) * safeRCP(max - min), every
+// block folding the partials by itself (a launch less than a fold of its own).
+__global__ void normalize_apply_kernel(float* __restrict__ v, uint64_t n, const float* __restrict__ partials, int nparts) {
+    __shared__ float s_mm[2];
+    {
+        float mn = INFINITY, mx = -INFINITY;
+        for (int i = threadIdx.x; i < nparts; i += blockDim.x) {
+            const float2 p = reinterpret_cast<const float2*>(partials)[i];
+            mn = fminf(mn, p.x);
+            mx = fmaxf(mx, p.y);
+        }
+        block_minmax(mn, mx);
+        if (threadIdx.x == 0) {
+            s_mm[0] = mn;
+            s_mm[1] = mx;
+        }
+        __syncthreads();
     }
-    block_minmax(mn, mx);
-    if (threadIdx.x == 0) {
-        mm[0] = mn;
-        mm[1] = mx;
-    }
-}
-
-// Pass 3: normalizeReconstruction, v = (v - min) * safeRCP(max - min).
-__global__ void normalize_apply_kernel(float* __restrict__ v, uint64_t n, const float* __restrict__ mm) {
-    const float mn = mm[0];
-    const float r = ref_safe_rcp(sub_rn(mm[1], mn));
+    const float mn = s_mm[0];
+    const float r = ref_safe_rcp(sub_rn(s_mm[1], mn));
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += stride)
-        v[i] = mul_rn(sub_rn(v[i], mn), r);
+    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    uint64_t tail = 0;
+    if ((reinterpret_cast<uintptr_t>(v) & 15) == 0) {
+        float4* v4 = reinterpret_cast<float4*>(v);
+        const uint64_t n4 = n / 4;
+        for (uint64_t j = i; j < n4; j += stride) {
+            float4 a = v4[j];
+            a.x = mul_rn(sub_rn(a.x, mn), r);
+            a.y = mul_rn(sub_rn(a.y, mn), r);
+            a.z = mul_rn(sub_rn(a.z, mn), r);
+            a.w = mul_rn(sub_rn(a.w, mn), r);
+            v4[j] = a;
+        }
+        tail = n4 * 4;
+    }
+    for (uint64_t j = tail + i; j < n; j += stride) v[j] = mul_rn(sub_rn(v[j], mn), r);
 }
 
 int minmax_blocks(const fbp_context* ctx, uint64_t n) {
@@ -100,27 +116,17 @@ int minmax_blocks(const fbp_context* ctx, uint64_t n) {
     return (int)std::max<uint64_t>(1, std::min<uint64_t>(want, cap));
 }
 
-// Runs the three passes with caller-provided scratch: partials must hold
-// 2*minmax_blocks(n) floats and mm two floats.
-fbp_status normalize_with_scratch(fbp_context* ctx, float* v, uint64_t n, float* partials, float* mm,
-                                  cudaStream_t stream) {
-    const int nb = minmax_blocks(ctx, n);
-    minmax_partial_kernel<<<nb, kReduceThreads, 0, stream>>>(v, n, partials);
-    FBP_CHECK_LAUNCH(ctx, "minmax_partial_kernel");
-    minmax_final_kernel<<<1, kReduceThreads, 0, stream>>>(partials, nb, mm);
-    FBP_CHECK_LAUNCH(ctx, "minmax_final_kernel");
-    const unsigned ab = (unsigned)std::min<uint64_t>(cdiv(n, 256), (uint64_t)ctx->sm_count * 8);
-    normalize_apply_kernel<<<ab, 256, 0, stream>>>(v, n, mm);
-    FBP_CHECK_LAUNCH(ctx, "normalize_apply_kernel");
-    return FBP_OK;
-}
-
 fbp_status normalize_device(fbp_context* ctx, float* v, uint64_t n, cudaStream_t stream) {
     const int nb = minmax_blocks(ctx, n);
     void* ws = nullptr;
-    FBP_TRY(workspace(ctx, WS_PARTIALS, (size_t)(2 * nb + 2) * sizeof(float), stream, &ws));
+    FBP_TRY(workspace(ctx, WS_PARTIALS, (size_t)2 * nb * sizeof(float), stream, &ws));
     float* partials = static_cast<float*>(ws);
-    return normalize_with_scratch(ctx, v, n, partials, partials + 2 * nb, stream);
+    minmax_partial_kernel<<<nb, kReduceThreads, 0, stream>>>(v, n, partials);
+    FBP_CHECK_LAUNCH(ctx, "minmax_partial_kernel");
+    const unsigned ab = (unsigned)std::min<uint64_t>(cdiv(n, 4 * 256), (uint64_t)ctx->sm_count * 8);
+    normalize_apply_kernel<<<ab, 256, 0, stream>>>(v, n, partials, nb);
+    FBP_CHECK_LAUNCH(ctx, "normalize_apply_kernel");
+    return FBP_OK;
 }
 
 // ------------------------------------------------------------- LoG filter --
@@ -178,85 +184,112 @@ __global__ void __launch_bounds__(512) log_filter_kernel(const float* __restrict
 }
 
 
-// The same filter for odd ksize = 2H+1 with H <= 2, register-blocked along
-// z: a thread walks the input planes of its columns once, keeping the K = 2H+1
-// outputs a plane reaches in a rotating window of accumulators (output
-// zo = pl - 2H + k sits in acc[k] and takes tap kz = 2H - k of plane pl;
-// after the plane acc[0] is complete and the window shifts).  Each thread
-// owns two columns, x and x + 16, as the halves of packed FP32 pairs: the
-// tile holds (v[x], v[x + 16]) pairs, the taps (w, w), and one fma.rn.f32x2
-// applies a tap to both outputs with the scalar rounding on each half.
-// Every output still receives its terms in the reference's order (plane =
-// kz ascending, then ky, then kx), so the result is bitwise that of
-// log_filter_kernel at half an issue slot per tap and output.  Tile
-// 32 x 8 x 16 outputs, 128 threads, 38 KB of shared memory.
+// The same filter for odd ksize = 2H+1 with H <= 2, streaming along z: a thread
+// walks the input planes of its columns once, keeping the K = 2H+1 outputs a
+// plane reaches in a rotating window of accumulators (plane pl adds tap
+// kz = 2H - k to output pl - 2H + k; the loop is unrolled over K planes, so the
+// rotation is in the register names).  Each thread owns two columns, x and
+// x + 16, as the halves of packed FP32 pairs: one fma.rn.f32x2 applies a tap to
+// both outputs with the scalar rounding on each half, and every output receives
+// its terms in the reference's order (plane = kz ascending, then ky, then kx),
+// so the result is bitwise that of log_filter_kernel.
+// The taps of a LoG depend on kx^2 + ky^2 + kz^2 alone (4 values for K = 3, 10
+// for K = 5; the host checks their bits), so they stay in registers.  The
+// planes pass through a ring in shared memory, asynchronous copies three ahead.
+// Bound by the FMA issue (a packed instruction holds the port two cycles): 125
+// FMAs per voxel are 52 us at 256^3.  89 us there; one plane ahead
+// through registers 97, and with the whole tile in shared memory first, slabs of
+// 16 planes and taps from the constant bank 125.
 template <int H>
 struct LogTaps2 {
-    unsigned long long w2[(2 * H + 1) * (2 * H + 1) * (2 * H + 1)];
+    unsigned long long w2[3 * H * H + 1];  // (w, w) by squared distance
 };
 
+constexpr int kLogTX = 32, kLogTY = 8;
+
+// Four bytes from global to shared memory, asynchronously.
+__device__ __forceinline__ void copy_async4(float* dst, const float* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+
 template <int H>
-__global__ void __launch_bounds__(128) log_filter_zpair_kernel(const float* __restrict__ in, float* __restrict__ out,
-                                                               uint32_t nx, uint32_t ny, uint32_t nz,
-                                                               const __grid_constant__ LogTaps2<H> taps) {
-    constexpr int K = 2 * H + 1, TX = 32, HX = 16, TY = 8, TZ = 16;
-    constexpr int EX = HX + 2 * H, EY = TY + 2 * H, EZ = TZ + 2 * H;
-    __shared__ f32x2_t tile[EZ][EY][EX];
-    const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY, z0 = blockIdx.z * TZ;
-    const int tid = threadIdx.x + HX * threadIdx.y;
-    constexpr int NT = HX * TY, NE = EX * EY * EZ, B = 8;
-    for (int i0 = tid; i0 < NE; i0 += B * NT) {
-        float va[B], vb[B];
+__global__ void __launch_bounds__(128, 7) log_filter_stream_kernel(const float* __restrict__ in, float* __restrict__ out,
+                                                                   uint32_t nx, uint32_t ny, uint32_t nz, uint32_t tz,
+                                                                   const LogTaps2<H> taps) {
+    constexpr int K = 2 * H + 1, HX = kLogTX / 2, TY = kLogTY, EX = HX + 2 * H, EY = TY + 2 * H, NT = HX * TY;
+    constexpr int NE = EX * EY, PER = (NE + NT - 1) / NT;
+    constexpr int RING = 4;
+    __shared__ f32x2_t tile[RING][EY][EX];
+    const int x0 = blockIdx.x * kLogTX, y0 = blockIdx.y * TY, z0 = blockIdx.z * tz;
+    const int z1 = min(z0 + (int)tz, (int)nz);
+    const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + HX * ty;
+    f32x2_t w[3 * H * H + 1];
 #pragma unroll
-        for (int u = 0; u < B; ++u) {
-            const int i = i0 + u * NT;
-            if (i < NE) {
-                const int lx = i % EX, ly = (i / EX) % EY, lz = i / (EX * EY);
-                const int ga = min(max(x0 + lx - H, 0), (int)nx - 1);
-                const int gb = min(max(x0 + lx + HX - H, 0), (int)nx - 1);
-                const int gy = min(max(y0 + ly - H, 0), (int)ny - 1);
-                const int gz = min(max(z0 + lz - H, 0), (int)nz - 1);
-                const size_t row = ((size_t)gz * ny + gy) * nx;
-                va[u] = in[row + ga];
-                vb[u] = in[row + gb];
-            }
-        }
+    for (int i = 0; i <= 3 * H * H; ++i) w[i] = taps.w2[i];
+    // This thread's samples of a plane (borders clamped).
+    uint32_t oa[PER], ob[PER];
 #pragma unroll
-        for (int u = 0; u < B; ++u)
-            if (i0 + u * NT < NE) (&tile[0][0][0])[i0 + u * NT] = pack2(va[u], vb[u]);
+    for (int u = 0; u < PER; ++u) {
+        const int e = min(tid + u * NT, NE - 1), lx = e % EX, gy = min(max(y0 + e / EX - H, 0), (int)ny - 1);
+        oa[u] = (uint32_t)gy * nx + min(max(x0 + lx - H, 0), (int)nx - 1);
+        ob[u] = (uint32_t)gy * nx + min(max(x0 + lx + HX - H, 0), (int)nx - 1);
     }
-    __syncthreads();
-    const int tx = threadIdx.x, ty = threadIdx.y;
+    const size_t plane = (size_t)nx * ny;
+    const int planes = z1 - z0 + 2 * H;
+    auto load = [&](int pl) {  // input plane z0 - H + pl into its place in the ring (a group even past the last)
+        if (pl < planes) {
+            const float* src = in + (size_t)min(max(z0 + pl - H, 0), (int)nz - 1) * plane;
+#pragma unroll
+            for (int u = 0; u < PER; ++u)
+                if (tid + u * NT < NE) {
+                    float* dst = reinterpret_cast<float*>(&tile[pl % RING][0][0] + tid + u * NT);
+                    copy_async4(dst, src + oa[u]);
+                    copy_async4(dst + 1, src + ob[u]);
+                }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
     const int xa = x0 + tx, xb = xa + HX, y = y0 + ty;
     const bool ok_a = xa < (int)nx && y < (int)ny, ok_b = xb < (int)nx && y < (int)ny;
+    const size_t row = (size_t)y * nx;
     f32x2_t acc[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) acc[k] = 0ull;
+    for (int pl = 0; pl < RING - 1; ++pl) load(pl);
 #pragma unroll 1
-    for (int pl = 0; pl < EZ; ++pl) {
+    for (int p0 = 0; p0 < planes; p0 += K) {
 #pragma unroll
-        for (int ky = 0; ky < K; ++ky) {
-            f32x2_t r[K];
+        for (int u = 0; u < K; ++u) {
+            const int pl = p0 + u;
+            if (pl >= planes) break;
+            asm volatile("cp.async.wait_group %0;" ::"n"(RING - 2) : "memory");  // this thread's part of plane pl
+            __syncthreads();  // everyone's; and all are through with plane pl - 1
+            load(pl + RING - 1);
+            const f32x2_t(*t)[EX] = tile[pl % RING];
 #pragma unroll
-            for (int kx = 0; kx < K; ++kx) r[kx] = tile[pl][ty + ky][tx + kx];
+            for (int ky = 0; ky < K; ++ky) {
+                f32x2_t r[K];
 #pragma unroll
-            for (int k = 0; k < K; ++k) {
-                const int kz = 2 * H - k;
+                for (int kx = 0; kx < K; ++kx) r[kx] = t[ty + ky][tx + kx];
 #pragma unroll
-                for (int kx = 0; kx < K; ++kx) acc[k] = fma_rn2(r[kx], taps.w2[(kz * K + ky) * K + kx], acc[k]);
+                for (int k = 0; k < K; ++k) {
+                    const int dz = H - k, dy = ky - H;  // kz = 2H - k
+                    f32x2_t& a = acc[(u + 1 + k) % K];
+#pragma unroll
+                    for (int kx = 0; kx < K; ++kx) a = fma_rn2(r[kx], w[dz * dz + dy * dy + (kx - H) * (kx - H)], a);
+                }
             }
+            f32x2_t& done = acc[(u + 1) % K];  // output plane pl - 2H
+            if (pl >= 2 * H) {
+                float a, b;
+                unpack2(done, a, b);
+                float* o = out + (size_t)(z0 + pl - 2 * H) * plane + row;
+                if (ok_a) o[xa] = a;
+                if (ok_b) o[xb] = b;
+            }
+            done = 0ull;
         }
-        const int zo = pl - 2 * H;  // acc[0] is complete
-        if (zo >= 0 && z0 + zo < (int)nz) {
-            float a, b;
-            unpack2(acc[0], a, b);
-            const size_t row = ((size_t)(z0 + zo) * ny + y) * nx;
-            if (ok_a) out[row + xa] = a;
-            if (ok_b) out[row + xb] = b;
-        }
-#pragma unroll
-        for (int k = 0; k < K - 1; ++k) acc[k] = acc[k + 1];
-        acc[K - 1] = 0ull;
     }
 }
 
@@ -409,16 +442,38 @@ static fbp_status log_h(fbp_context* ctx, const float* in, float* out, uint32_t 
     for (int i = 0; i < ksize * ksize * ksize; ++i) taps.w[i] = w[i];
     if constexpr (H >= 1 && H <= 2) {
         if (ksize == 2 * H + 1) {
+            // The taps by squared distance, if they depend on nothing else.
             LogTaps2<H> taps2{};
+            bool radial = (uint64_t)nx * ny < (1ull << 32), seen[3 * H * H + 1] = {};
             for (int i = 0; i < ksize * ksize * ksize; ++i) {
+                const int x = i % ksize - H, y = i / ksize % ksize - H, z = i / (ksize * ksize) - H;
                 uint32_t b;
                 std::memcpy(&b, &w[i], 4);
-                taps2.w2[i] = ((unsigned long long)b << 32) | b;  // (w, w)
+                const int d = x * x + y * y + z * z;
+                const unsigned long long v = ((unsigned long long)b << 32) | b;  // (w, w)
+                radial = radial && (!seen[d] || taps2.w2[d] == v);
+                seen[d] = true;
+                taps2.w2[d] = v;
             }
-            dim3 grid(cdiv(nx, 32), cdiv(ny, 8), cdiv(nz, 16));
-            log_filter_zpair_kernel<H><<<grid, dim3(16, 8), 0, stream>>>(in, out, nx, ny, nz, taps2);
-            FBP_CHECK_LAUNCH(ctx, "log_filter_zpair_kernel");
-            return FBP_OK;
+            if (radial) {
+                // Planes per CTA: the fewest plane steps on the busiest SM
+                // (seven CTAs resident; two steps' worth of set-up).
+                uint32_t tz = 8;
+                uint64_t least = ~0ull;
+                const uint64_t columns = (uint64_t)cdiv(nx, kLogTX) * cdiv(ny, kLogTY);
+                for (uint32_t c = 8; c <= 256; c *= 2) {
+                    const uint64_t ctas = columns * cdiv(nz, c), rounds = cdiv(ctas, (uint64_t)ctx->sm_count);
+                    const uint64_t steps = rounds * (std::min(c, nz) + 2 * H + 2);
+                    if (steps < least) {
+                        least = steps;
+                        tz = c;
+                    }
+                }
+                dim3 grid(cdiv(nx, kLogTX), cdiv(ny, kLogTY), cdiv(nz, tz));
+                log_filter_stream_kernel<H><<<grid, dim3(kLogTX / 2, kLogTY), 0, stream>>>(in, out, nx, ny, nz, tz, taps2);
+                FBP_CHECK_LAUNCH(ctx, "log_filter_stream_kernel");
+                return FBP_OK;
+            }
         }
     }
     constexpr int E = 8 + 2 * H;
@@ -509,11 +564,11 @@ extern "C" fbp_status fbp_normalize_minmax(fbp_context* ctx, float* v, uint64_t 
 
 // ------------------------------------------ allocation-free normalisation --
 //
-// fbp_normalize_minmax_noalloc: the same three passes as fbp_normalize_minmax,
-// but its scratch (one min/max pair per reduction block plus the final pair)
-// lives in this file-scope array instead of context workspace, so the call
-// allocates nothing and needs no fbp_context.  Every device that loads the
-// library holds the array (8 KiB) until the process exits.  The partial pass
+// fbp_normalize_minmax_noalloc: the same two passes as fbp_normalize_minmax,
+// but its scratch (one min/max pair per reduction block) lives in this
+// file-scope array instead of context workspace, so the call allocates nothing
+// and needs no fbp_context.  Every device that loads the library holds the array
+// (8 KiB) until the process exits.  The partial pass
 // strides over the input with up to 1024 blocks (4 per SM, like the context
 // entry point), one partial slot each; inputs are limited to 2^30 elements.
 // All calls on a device share the array: each call overwrites every slot it
@@ -522,7 +577,7 @@ extern "C" fbp_status fbp_normalize_minmax(fbp_context* ctx, float* v, uint64_t 
 namespace fbp {
 constexpr int kNoAllocMaxBlocks = 1024;
 constexpr uint64_t kNoAllocMaxElems = 1ull << 30;
-static __device__ __align__(256) float g_noalloc_scratch[2 * kNoAllocMaxBlocks + 2];
+static __device__ __align__(256) float g_noalloc_scratch[2 * kNoAllocMaxBlocks];
 
 // Device address of g_noalloc_scratch on the current device, looked up on
 // every call (the first call on a device loads the module; later lookups are
@@ -566,13 +621,10 @@ extern "C" fbp_status fbp_normalize_minmax_noalloc(float* v, uint64_t n, void* s
         const uint64_t want = (n + 4ull * kReduceThreads - 1) / (4ull * kReduceThreads);
         const uint64_t cap = std::min<uint64_t>(kNoAllocMaxBlocks, 4ull * (uint64_t)std::max(sms, 1));
         const int nb = (int)std::max<uint64_t>(1, std::min(want, cap));
-        float* mm = scratch + 2 * kNoAllocMaxBlocks;
         minmax_partial_kernel<<<nb, kReduceThreads, 0, s>>>(v, n, scratch);
         FBP_TRY_CUDA(cudaGetLastError());
-        minmax_final_kernel<<<1, kReduceThreads, 0, s>>>(scratch, nb, mm);
-        FBP_TRY_CUDA(cudaGetLastError());
-        const unsigned ab = (unsigned)std::min<uint64_t>(cdiv(n, 256), 1216);
-        normalize_apply_kernel<<<ab, 256, 0, s>>>(v, n, mm);
+        const unsigned ab = (unsigned)std::min<uint64_t>(cdiv(n, 4 * 256), 1216);
+        normalize_apply_kernel<<<ab, 256, 0, s>>>(v, n, scratch, nb);
         FBP_TRY_CUDA(cudaGetLastError());
         return FBP_OK;
     });
