@@ -102,12 +102,8 @@ fbp_status launch_any(fbp_context* ctx, const BatchLaunch& l, int ctas, cudaStre
 fbp_status rows_any(fbp_context* ctx, int dtype, const fbp_capture_desc& c, uint32_t pitch, void* dst,
                     cudaStream_t s) {
     const uint32_t L = c.info.num_laser_targets, T = c.info.num_time_bins;
-    float* rows = static_cast<float*>(dst);
-    switch (dtype) {
-        case FBP_F32: return prepare_rows_into<float>(ctx, c.cube, c.layout, L, T, pitch, rows, s);
-        case FBP_BF16: return prepare_rows_into<__nv_bfloat16>(ctx, c.cube, c.layout, L, T, pitch, rows, s);
-        default: return prepare_rows_into<__half>(ctx, c.cube, c.layout, L, T, pitch, rows, s);
-    }
+    return prepare_gather(ctx, dtype, PrepRows{c.cube, static_cast<float*>(dst), L, T, pitch, c.layout == FBP_LAYOUT_TIME_MAJOR},
+                          PrepTables{}, s);
 }
 
 // (Re)plan windows, parameters and work items for tile configuration `cfg`.

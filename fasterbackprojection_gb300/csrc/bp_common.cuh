@@ -189,11 +189,33 @@ fbp_status confocal_gather(fbp_context* ctx, const fbp_recon_info& in, const voi
                            const float* laser_xyz, float* volume, cudaStream_t s, const SampleParams* smp);
 void confocal_tile_grid(const fbp_recon_info& in, uint32_t out[3]);
 
-// Padded, thresholded FP32 rows [L][pitch] of a confocal cube of storage type
-// S (16-bit values widened exactly), written to dst.
-template <typename S>
-fbp_status prepare_rows_into(fbp_context* ctx, const void* cube, int layout, uint32_t L, uint32_t T, uint32_t pitch,
-                             float* dst, cudaStream_t stream);
+// The gathers' inputs, made by one launch (prepare_gather).
+// Rows [count][pitch] FP32 (pitch a multiple of 4), time innermost, values
+// <= 1e-5 replaced by 0 (the reference skips them), zeros in [T, pitch); 16-bit
+// captures are widened exactly.
+struct PrepRows {
+    const void* cube;
+    float* rows;
+    uint64_t count;
+    uint32_t T, pitch;
+    int time_major;  // cube[t][row] instead of cube[row][t]
+};
+// Scan tables (x, y, z, bounce distances) and voxel-centre coordinates
+// [Vx + Vz + Vy]; zero counts leave a table out.
+struct PrepTables {
+    const float *laser_xyz, *sensor_xyz;
+    float4 *lasers, *sensors;
+    float* axes;
+    uint32_t num_lasers, num_sensors;  // no sensors: confocal, both bounces with the lasers
+    int discard;
+    float laser_pos[3], sensor_pos[3], min[3], size[3];
+    uint32_t res[3];
+};
+fbp_status prepare_gather(fbp_context* ctx, int dtype, const PrepRows& rows, const PrepTables& tables, cudaStream_t stream);
+// The tables' part of the request, in the context's scratch (sensor_xyz null:
+// confocal).
+fbp_status table_buffers(fbp_context* ctx, const fbp_recon_info& in, const float* laser_xyz, const float* sensor_xyz,
+                         cudaStream_t stream, PrepTables* t);
 
 __global__ void axis_tables_kernel(float* __restrict__ xs, float* __restrict__ ys, float* __restrict__ zs,
                                    uint32_t Vx, uint32_t Vy, uint32_t Vz, float mnx, float mny, float mnz, float sx,

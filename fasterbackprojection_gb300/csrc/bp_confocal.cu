@@ -56,102 +56,13 @@ __global__ void scan_table_kernel(float4* __restrict__ out, const float* __restr
     out[i] = make_float4(x, y, z, b);
 }
 
-// Rows from a time-innermost cube: copy (widened to FP32), threshold, pad.
-template <typename S>
-__global__ void rows_from_time_inner_kernel(float* __restrict__ rows, const S* __restrict__ cube, uint32_t L,
-                                            uint32_t T, uint32_t pitch) {
-    const uint64_t n = (uint64_t)L * pitch;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t l = (uint32_t)(i / pitch), t = (uint32_t)(i % pitch);
-        float v = 0.f;
-        if (t < T) {
-            const float c = to_f32(cube[(uint64_t)l * T + t]);
-            if (c > FBP_EPS) v = c;
-        }
-        rows[i] = v;
-    }
-}
-
-// Rows from a time-major cube (cube[t*L + l]): tiled transpose through shared
-// memory so both the read and the write are coalesced.
-template <typename S>
-__global__ void rows_from_time_major_kernel(float* __restrict__ rows, const S* __restrict__ cube, uint32_t L,
-                                            uint32_t T, uint32_t pitch) {
-    __shared__ float tile[32][33];
-    const uint32_t l0 = blockIdx.x * 32, t0 = blockIdx.y * 32;
-    for (int j = threadIdx.y; j < 32; j += blockDim.y) {
-        const uint32_t t = t0 + j, l = l0 + threadIdx.x;
-        float v = 0.f;
-        if (t < T && l < L) {
-            v = to_f32(cube[(uint64_t)t * L + l]);
-            if (!(v > FBP_EPS)) v = 0.f;
-        }
-        tile[j][threadIdx.x] = v;
-    }
-    __syncthreads();
-    for (int j = threadIdx.y; j < 32; j += blockDim.y) {
-        const uint32_t l = l0 + j, t = t0 + threadIdx.x;
-        if (l < L && t < pitch) rows[(uint64_t)l * pitch + t] = tile[threadIdx.x][j];
-    }
-}
-
-// Zero the padding columns [roundup(T,32), pitch) the transpose grid does not cover.
-__global__ void rows_zero_tail_kernel(float* __restrict__ rows, uint32_t L, uint32_t from, uint32_t pitch) {
-    const uint32_t w = pitch - from;
-    const uint64_t n = (uint64_t)L * w;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        rows[(i / w) * pitch + from + (i % w)] = 0.f;
-}
-
-// ------------------------------------------------------------ host driver --
-
-template <typename S>
-fbp_status prepare_rows_into(fbp_context* ctx, const void* cube, int layout, uint32_t L, uint32_t T, uint32_t pitch,
-                             float* r, cudaStream_t stream) {
-    const S* c = static_cast<const S*>(cube);
-    if (layout == FBP_LAYOUT_TIME_INNER) {
-        const uint64_t n = (uint64_t)L * pitch;
-        const unsigned blocks = (unsigned)std::min<uint64_t>(cdiv(n, 256), (uint64_t)ctx->sm_count * 16);
-        rows_from_time_inner_kernel<S><<<blocks, 256, 0, stream>>>(r, c, L, T, pitch);
-        FBP_CHECK_LAUNCH(ctx, "rows_from_time_inner_kernel");
-    } else {
-        const uint32_t tcover = std::min<uint32_t>(pitch, (T + 31) / 32 * 32);
-        dim3 grid(cdiv(L, 32), cdiv(tcover, 32));
-        rows_from_time_major_kernel<S><<<grid, dim3(32, 8), 0, stream>>>(r, c, L, T, pitch);
-        FBP_CHECK_LAUNCH(ctx, "rows_from_time_major_kernel");
-        if (tcover < pitch) {
-            const uint64_t n = (uint64_t)L * (pitch - tcover);
-            const unsigned blocks = (unsigned)std::min<uint64_t>(cdiv(n, 256), (uint64_t)ctx->sm_count * 16);
-            rows_zero_tail_kernel<<<blocks, 256, 0, stream>>>(r, L, tcover, pitch);
-            FBP_CHECK_LAUNCH(ctx, "rows_zero_tail_kernel");
-        }
-    }
-    return FBP_OK;
-}
-template fbp_status prepare_rows_into<float>(fbp_context*, const void*, int, uint32_t, uint32_t, uint32_t, float*,
-                                             cudaStream_t);
-template fbp_status prepare_rows_into<__nv_bfloat16>(fbp_context*, const void*, int, uint32_t, uint32_t, uint32_t,
-                                                     float*, cudaStream_t);
-template fbp_status prepare_rows_into<__half>(fbp_context*, const void*, int, uint32_t, uint32_t, uint32_t, float*,
-                                              cudaStream_t);
-
 namespace {
-
-template <typename S>
-fbp_status prepare_rows(fbp_context* ctx, const void* cube, int layout, uint32_t L, uint32_t T, uint32_t pitch,
-                        cudaStream_t stream, float** rows_out) {
-    void* rows = nullptr;
-    FBP_TRY(workspace(ctx, WS_CUBE_ROWS, (size_t)L * pitch * sizeof(float), stream, &rows));
-    *rows_out = static_cast<float*>(rows);
-    return prepare_rows_into<S>(ctx, cube, layout, L, T, pitch, *rows_out, stream);
-}
 
 // Depth slices [z_begin, z_end) of the volume (the whole volume by default)
 // into `volume` ([z_end - z_begin][Vy][Vx]).  The window plan and the voxel
 // tables are those of the whole volume, so with z_begin a multiple of the
 // tile depth a slab is bitwise the same rows of the full result.
-template <typename S>
-fbp_status launch_confocal(fbp_context* ctx, const fbp_recon_info& in, const void* cube, int layout,
+fbp_status launch_confocal(fbp_context* ctx, const fbp_recon_info& in, const void* cube, int dtype, int layout,
                            const float* laser_xyz, float* volume, cudaStream_t stream, const SampleParams* smp,
                            uint32_t z_begin = 0, uint32_t z_end = 0xFFFFFFFFu, bool scatter = false) {
     const uint32_t L = in.num_laser_targets, T = in.num_time_bins;
@@ -182,11 +93,18 @@ fbp_status launch_confocal(fbp_context* ctx, const fbp_recon_info& in, const voi
                         ConfocalGatherParams::kWindowBufs));
     if (smp) wp.smem -= kSampledStaticSmem;
 
-    float* rows = nullptr;
-    FBP_TRY(prepare_rows<S>(ctx, cube, layout, L, T, wp.pitch, stream, &rows));
+    void* rows = nullptr;
+    FBP_TRY(workspace(ctx, WS_CUBE_ROWS, (size_t)L * wp.pitch * sizeof(float), stream, &rows));
+    PrepTables tables{};
+    FBP_TRY(table_buffers(ctx, in, laser_xyz, nullptr, stream, &tables));
+    FBP_TRY(prepare_gather(ctx, dtype, PrepRows{cube, static_cast<float*>(rows), L, T, wp.pitch, layout == FBP_LAYOUT_TIME_MAJOR},
+                           tables, stream));
 
     ConfocalGatherParams p{};
-    FBP_TRY(build_tables(ctx, in, laser_xyz, stream, &p.scan, &p.xs, &p.ys, &p.zs));
+    p.scan = tables.lasers;
+    p.xs = tables.axes;
+    p.ys = p.xs + Vx;
+    p.zs = p.ys + Vz;
     p.rows = rows;
     p.volume = volume;
     p.status = ctx->status_dev;
@@ -308,36 +226,18 @@ void confocal_tile_grid(const fbp_recon_info& in, uint32_t out[3]) {
 
 fbp_status confocal_gather(fbp_context* ctx, const fbp_recon_info& in, const void* cube, int dtype, int layout,
                            const float* laser_xyz, float* volume, cudaStream_t s, const SampleParams* smp) {
-    switch (dtype) {
-        case FBP_F32: return launch_confocal<float>(ctx, in, cube, layout, laser_xyz, volume, s, smp);
-        case FBP_BF16: return launch_confocal<__nv_bfloat16>(ctx, in, cube, layout, laser_xyz, volume, s, smp);
-        case FBP_F16: return launch_confocal<__half>(ctx, in, cube, layout, laser_xyz, volume, s, smp);
-        default: return set_error(FBP_ERR_INVALID_ARG, "unknown dtype");
-    }
+    return launch_confocal(ctx, in, cube, dtype, layout, laser_xyz, volume, s, smp);
 }
 
 fbp_status confocal_gather_scatter(fbp_context* ctx, const fbp_recon_info& in, const void* cube, int dtype,
                                    int layout, const float* laser_xyz, float* volume, cudaStream_t s) {
-    const uint32_t all = 0xFFFFFFFFu;
-    switch (dtype) {
-        case FBP_F32: return launch_confocal<float>(ctx, in, cube, layout, laser_xyz, volume, s, nullptr, 0, all, true);
-        case FBP_BF16:
-            return launch_confocal<__nv_bfloat16>(ctx, in, cube, layout, laser_xyz, volume, s, nullptr, 0, all, true);
-        case FBP_F16: return launch_confocal<__half>(ctx, in, cube, layout, laser_xyz, volume, s, nullptr, 0, all, true);
-        default: return set_error(FBP_ERR_INVALID_ARG, "unknown dtype");
-    }
+    return launch_confocal(ctx, in, cube, dtype, layout, laser_xyz, volume, s, nullptr, 0, 0xFFFFFFFFu, true);
 }
 
 fbp_status confocal_gather_slab(fbp_context* ctx, const fbp_recon_info& in, const void* cube, int dtype, int layout,
                                 const float* laser_xyz, uint32_t z_begin, uint32_t z_end, float* volume,
                                 cudaStream_t s) {
-    switch (dtype) {
-        case FBP_F32: return launch_confocal<float>(ctx, in, cube, layout, laser_xyz, volume, s, nullptr, z_begin, z_end);
-        case FBP_BF16:
-            return launch_confocal<__nv_bfloat16>(ctx, in, cube, layout, laser_xyz, volume, s, nullptr, z_begin, z_end);
-        case FBP_F16: return launch_confocal<__half>(ctx, in, cube, layout, laser_xyz, volume, s, nullptr, z_begin, z_end);
-        default: return set_error(FBP_ERR_INVALID_ARG, "unknown dtype");
-    }
+    return launch_confocal(ctx, in, cube, dtype, layout, laser_xyz, volume, s, nullptr, z_begin, z_end);
 }
 
 fbp_status build_tables(fbp_context* ctx, const fbp_recon_info& in, const float* laser_xyz, cudaStream_t stream,

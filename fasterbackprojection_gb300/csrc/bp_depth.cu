@@ -392,24 +392,21 @@ fbp_status go_depth_tiles(fbp_context* ctx, DepthTileParams p, dim3 grid, cudaSt
 }
 
 // The confocal planes by tiles of 256 scan points x 16 depths.
-template <typename S>
-fbp_status launch_depth_tiles(fbp_context* ctx, const fbp_recon_info& in, const void* cube, int layout,
+fbp_status launch_depth_tiles(fbp_context* ctx, const fbp_recon_info& in, const void* cube, int dtype, int layout,
                               const float* laser_xyz, const double* depths, uint32_t D, float* act,
                               cudaStream_t stream) {
     const uint32_t L = in.num_laser_targets, T = in.num_time_bins;
     DepthTileParams p{};
     p.pitch = (T + 3) / 4 * 4 + DepthTileParams::kSlot;
-    void *rows = nullptr, *sp = nullptr;
+    void* rows = nullptr;
     FBP_TRY(workspace(ctx, WS_CUBE_ROWS, (size_t)L * p.pitch * sizeof(float), stream, &rows));
-    FBP_TRY(prepare_rows_into<S>(ctx, cube, layout, L, T, p.pitch, static_cast<float*>(rows), stream));
-    FBP_TRY(workspace(ctx, WS_SCAN_TABLE, (size_t)L * sizeof(float4), stream, &sp));
-    scan_table_kernel<<<cdiv(L, 256), 256, 0, stream>>>(static_cast<float4*>(sp), laser_xyz, L,
-                                                       (int)in.discard_first_last_bounces, in.laser_position[0],
-                                                       in.laser_position[1], in.laser_position[2],
-                                                       in.sensor_position[0], in.sensor_position[1],
-                                                       in.sensor_position[2], 1);
-    FBP_CHECK_LAUNCH(ctx, "scan_table_kernel");
-    p.scan = static_cast<const float4*>(sp);
+    PrepTables tables{};
+    FBP_TRY(table_buffers(ctx, in, laser_xyz, nullptr, stream, &tables));
+    for (uint32_t& r : tables.res) r = 0;  // no volume
+    FBP_TRY(prepare_gather(ctx, dtype,
+                           PrepRows{cube, static_cast<float*>(rows), L, T, p.pitch, layout == FBP_LAYOUT_TIME_MAJOR}, tables,
+                           stream));
+    p.scan = tables.lasers;
     p.xyz = laser_xyz;
     p.depths = depths;
     p.rows = static_cast<const float*>(rows);
@@ -536,7 +533,7 @@ fbp_status launch_depths(fbp_context* ctx, const fbp_recon_info& in, const void*
                          float* act, cudaStream_t stream) {
     const bool exhaustive = in.capture_system == FBP_EXHAUSTIVE;
     if (!exhaustive && in.num_time_bins <= DepthTileParams::kMaxBins && cdiv(D, DepthTileParams::kDepths) <= 65535)
-        return launch_depth_tiles<S>(ctx, in, cube, layout, laser_xyz, depths, D, act, stream);
+        return launch_depth_tiles(ctx, in, cube, dtype_of<S>(), layout, laser_xyz, depths, D, act, stream);
     const uint32_t L = in.num_laser_targets, Sn = exhaustive ? in.num_sensor_targets : 1, T = in.num_time_bins;
     const uint32_t pitch = (T + 7) / 8 * 8;
     const uint64_t R = (uint64_t)L * Sn;

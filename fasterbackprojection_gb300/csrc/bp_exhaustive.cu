@@ -399,24 +399,6 @@ namespace {
 constexpr int kKV = 8, kWY = 2, kWZ = 4;
 constexpr int kExhaustiveCtasPerSm = 2;  // 256 threads of up to 128 registers
 
-// Padded, thresholded FP32 rows [L*S][pitch] of the cube (16-bit storage
-// widened exactly, so the triple loop reads FP32 with no conversion).
-template <typename S>
-__global__ void pair_rows_kernel(float* __restrict__ rows, const S* __restrict__ cube, uint64_t npairs, uint32_t T,
-                                 uint32_t pitch) {
-    const uint64_t n = npairs * pitch;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t r = i / pitch;
-        const uint32_t t = (uint32_t)(i % pitch);
-        float v = 0.f;
-        if (t < T) {
-            const float c = to_f32(cube[r * T + t]);
-            if (c > FBP_EPS) v = c;
-        }
-        rows[i] = v;
-    }
-}
-
 template <int MODE, bool BOUNCE, bool CLAMP, int LB>
 fbp_status go_exhaustive(fbp_context* ctx, ExhaustiveGatherParams p, dim3 grid, size_t smem, cudaStream_t stream) {
     auto kernel = exhaustive_gather_kernel<kKV, kWY, kWZ, MODE, BOUNCE, CLAMP, LB>;
@@ -448,8 +430,7 @@ fbp_status dispatch_exhaustive(fbp_context* ctx, const ExhaustiveGatherParams& p
     return go_exhaustive<EX_FAST, LB>(ctx, p, grid, smem, s, bounce, capped);
 }
 
-template <typename S>
-fbp_status launch_exhaustive(fbp_context* ctx, const fbp_recon_info& in, const void* cube, const float* laser_xyz,
+fbp_status launch_exhaustive(fbp_context* ctx, const fbp_recon_info& in, const void* cube, int dtype, const float* laser_xyz,
                              const float* sensor_xyz, float* volume, cudaStream_t stream) {
     const uint32_t L = in.num_laser_targets, Sn = in.num_sensor_targets, T = in.num_time_bins;
     const uint32_t Vx = in.voxel_res[0], Vy = in.voxel_res[1], Vz = in.voxel_res[2];
@@ -465,33 +446,16 @@ fbp_status launch_exhaustive(fbp_context* ctx, const fbp_recon_info& in, const v
 
     void* rows = nullptr;
     FBP_TRY(workspace(ctx, WS_CUBE_ROWS, npairs * pitch * sizeof(float), stream, &rows));
-    {
-        const uint64_t n = npairs * pitch;
-        const unsigned blocks = (unsigned)std::min<uint64_t>(cdiv(n, 256), (uint64_t)ctx->sm_count * 16);
-        pair_rows_kernel<S><<<blocks, 256, 0, stream>>>(static_cast<float*>(rows), static_cast<const S*>(cube), npairs,
-                                                        T, pitch);
-        FBP_CHECK_LAUNCH(ctx, "pair_rows_kernel");
-    }
+    PrepTables tables{};
+    FBP_TRY(table_buffers(ctx, in, laser_xyz, sensor_xyz, stream, &tables));
+    FBP_TRY(prepare_gather(ctx, dtype, PrepRows{cube, static_cast<float*>(rows), npairs, T, pitch, 0}, tables, stream));
 
     ExhaustiveGatherParams p{};
-    const float4* lscan = nullptr;
-    FBP_TRY(build_tables(ctx, in, laser_xyz, stream, &lscan, &p.xs, &p.ys, &p.zs));
-    // build_tables stores |l-laser| + |l-sensor|; the exhaustive kernel needs
-    // |l - laserPos| and |s - sensorPos| separately, so rebuild both tables.
-    void* lp = nullptr;
-    void* sp = nullptr;
-    FBP_TRY(workspace(ctx, WS_SCAN_TABLE, (size_t)L * sizeof(float4), stream, &lp));
-    FBP_TRY(workspace(ctx, WS_SENSOR_TABLE, (size_t)Sn * sizeof(float4), stream, &sp));
-    scan_table_kernel<<<cdiv(L, 256), 256, 0, stream>>>(static_cast<float4*>(lp), laser_xyz, L,
-                                                       (int)in.discard_first_last_bounces, in.laser_position[0],
-                                                       in.laser_position[1], in.laser_position[2], 0.f, 0.f, 0.f, 0);
-    FBP_CHECK_LAUNCH(ctx, "scan_table_kernel");
-    scan_table_kernel<<<cdiv(Sn, 256), 256, 0, stream>>>(static_cast<float4*>(sp), sensor_xyz, Sn,
-                                                        (int)in.discard_first_last_bounces, in.sensor_position[0],
-                                                        in.sensor_position[1], in.sensor_position[2], 0.f, 0.f, 0.f, 0);
-    FBP_CHECK_LAUNCH(ctx, "scan_table_kernel");
-    p.lscan = static_cast<const float4*>(lp);
-    p.sscan = static_cast<const float4*>(sp);
+    p.lscan = tables.lasers;
+    p.sscan = tables.sensors;
+    p.xs = tables.axes;
+    p.ys = p.xs + Vx;
+    p.zs = p.ys + Vz;
     p.volume = volume;
     p.status = ctx->status_dev;
     p.rows = static_cast<const float*>(rows);
@@ -531,11 +495,8 @@ extern "C" fbp_status fbp_backproject_exhaustive(fbp_context* ctx, const fbp_rec
         if (!cube || !laser_xyz || !sensor_xyz || !volume)
             return set_error(FBP_ERR_INVALID_ARG, "fbp_backproject_exhaustive: null buffer");
         cudaStream_t s = (cudaStream_t)stream;
-        switch (dtype) {
-            case FBP_F32: return launch_exhaustive<float>(ctx, *info, cube, laser_xyz, sensor_xyz, volume, s);
-            case FBP_BF16: return launch_exhaustive<__nv_bfloat16>(ctx, *info, cube, laser_xyz, sensor_xyz, volume, s);
-            case FBP_F16: return launch_exhaustive<__half>(ctx, *info, cube, laser_xyz, sensor_xyz, volume, s);
-            default: return set_error(FBP_ERR_INVALID_ARG, "fbp_backproject_exhaustive: unknown dtype");
-        }
+        if (dtype != FBP_F32 && dtype != FBP_BF16 && dtype != FBP_F16)
+            return set_error(FBP_ERR_INVALID_ARG, "fbp_backproject_exhaustive: unknown dtype");
+        return launch_exhaustive(ctx, *info, cube, dtype, laser_xyz, sensor_xyz, volume, s);
     });
 }
