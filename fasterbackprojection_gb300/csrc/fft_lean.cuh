@@ -43,7 +43,10 @@ __device__ __forceinline__ void lean_dft(float2 (&v)[R]) {
 // HALF_IN (first pass only): inputs N/2 .. N-1 are zero, i.e. the inputs
 // r >= R/2 of every butterfly, and are not read.  HALF_OUT (last pass only):
 // outputs N/2 .. N-1, the outputs k >= R/2 of every butterfly, are not
-// stored.  Stage tables hold R entries per jm (64-byte aligned for R >= 8).
+// stored.  Stage tables hold the Ns entries of r = 0, then those of r = 1, ...:
+// the butterflies of a warp have consecutive jm and read consecutive entries
+// (with the R entries of a jm together, 16-byte loads 64 or 128 bytes apart took
+// four times the data's share of the shared-memory pipe).
 template <int LOG2N, int DONE, int NLINES, int NT, bool INV, bool COLS, bool HALF_IN, bool HALF_OUT>
 __device__ __forceinline__ void lean_pass(float2* x, const float2* tw, int rs) {
     constexpr int RB = stage_radix_bits(LOG2N, DONE), R = 1 << RB;
@@ -63,22 +66,12 @@ __device__ __forceinline__ void lean_pass(float2* x, const float2* tw, int rs) {
             for (int r = 0; r < R; ++r)
                 v[u][r] = r < RIN ? x[lean_addr<COLS>(line, j + r * NB, rs)] : make_float2(0.f, 0.f);
             if constexpr (DONE > 0) {
-                float2 w[R];
-                if constexpr (R >= 4) {
-                    const float4* t4 = reinterpret_cast<const float4*>(tws + (j & (NS - 1)) * R);
-#pragma unroll
-                    for (int q = 0; q < R / 2; ++q) {
-                        const float4 t = t4[q];
-                        w[2 * q] = make_float2(t.x, t.y);
-                        w[2 * q + 1] = make_float2(t.z, t.w);
-                    }
-                } else {
-                    w[1] = tws[(j & (NS - 1)) * R + 1];
-                }
+                const float2* t = tws + (j & (NS - 1));
 #pragma unroll
                 for (int r = 1; r < R; ++r) {
-                    if (INV) w[r].y = -w[r].y;
-                    v[u][r] = cmul(v[u][r], w[r]);
+                    float2 w = t[r * NS];
+                    if (INV) w.y = -w.y;
+                    v[u][r] = cmul(v[u][r], w);
                 }
             }
             lean_dft<R, INV>(v[u]);

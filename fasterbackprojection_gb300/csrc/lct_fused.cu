@@ -55,22 +55,26 @@ struct LctFusedParams {
     int magnitude;                // 1: |vol| (lct_2.py), 0: max(real(vol), 0) (lct.py)
 };
 
-constexpr int kZThreads = 512;
-
-// Real lines per CTA of the z kernels (even: lines j and j + C/2 share one
-// complex transform): 64 KiB of line buffers at most, at most 8.
-constexpr int z_lines(int log2z) { return log2z <= 10 ? 8 : (log2z == 11 ? 4 : 2); }
-
-template <int LOG2Z>
-constexpr size_t zfwd_smem() {
-    constexpr int Z = 1 << LOG2Z, C = z_lines(LOG2Z);
-    return ((size_t)(C / 2) * line_stride(Z) + stage_table_size(LOG2Z)) * sizeof(float2) +
-           (size_t)C * (Z / 2) * sizeof(float);
+// Real lines per CTA of the z kernels (even: lines 2j and 2j + 1 share one
+// complex transform): at most 8 and 70 KB of line buffers.  16 values of a
+// complex line per thread, so every pass is one radix-16 or two radix-8
+// butterflies of each thread; four CTAs (two of the two longest) share an SM.
+// (Half the lines for the two longest, 35 KB, halves the width of the strided
+// accesses: 64^2 x 2048 in 450 against 347 us.)
+constexpr int z_lines(int log2z) { return log2z <= 11 ? 8 : 4; }
+constexpr int z_threads(int log2z) {
+    return (z_lines(log2z) / 2 << log2z) / 16 < 64 ? 64 : (z_lines(log2z) / 2 << log2z) / 16;
 }
+constexpr int z_ctas(int log2z) { return log2z <= 10 ? 4 : 2; }
+
+// The lines' stride and the two raw lines' within one: the 32 (line, bin) pairs of
+// a warp's strided accesses fall into different banks.
+constexpr int z_skew(int log2z) { return 32 / z_lines(log2z); }
+constexpr int z_stride(int log2z) { return (1 << log2z) + (1 << log2z) / 16 + z_skew(log2z); }
+
 template <int LOG2Z>
-constexpr size_t zinv_smem() {
-    constexpr int Z = 1 << LOG2Z, C = z_lines(LOG2Z);
-    return ((size_t)C * line_stride(Z) + stage_table_size(LOG2Z)) * sizeof(float2);
+constexpr size_t z_smem() {
+    return ((size_t)(z_lines(LOG2Z) / 2) * z_stride(LOG2Z) + stage_table_size(LOG2Z)) * sizeof(float2);
 }
 template <int LOG2X>
 constexpr size_t plane_smem() {
@@ -80,57 +84,88 @@ constexpr size_t plane_smem() {
 template <int LOG2X>
 constexpr int plane_threads() { return LOG2X >= 7 ? 512 : 256; }
 
+// Latency-bound: loads, resample, three FFT passes and the store follow one
+// another, so what counts is how many lines an SM holds and how little of the
+// shared-memory pipe they take (now 46 %).  64^2 x 512: 31.6 us with 512 threads
+// on as many lines, every element walking its own row of mtx; 20.7 with these
+// lines, threads and shared rows; 17.4 with the skews and the stage tables by r.
 template <int LOG2Z>
-__global__ void __launch_bounds__(kZThreads, 2) lct_zfwd_kernel(LctFusedParams p) {
-    constexpr int Z = 1 << LOG2Z, M = Z / 2, C = z_lines(LOG2Z), H = C / 2, LS = line_stride(Z),
-                  TWN = stage_table_size(LOG2Z);
+__global__ void __launch_bounds__(z_threads(LOG2Z), z_ctas(LOG2Z)) lct_zfwd_kernel(LctFusedParams p) {
+    constexpr int Z = 1 << LOG2Z, M = Z / 2, C = z_lines(LOG2Z), H = C / 2, LS = z_stride(LOG2Z),
+                  TWN = stage_table_size(LOG2Z), NT = z_threads(LOG2Z);
     extern __shared__ __align__(16) float2 sm[];
-    float2* lines = sm;  // [H] complex lines: line j in the real part, line j + H in the imaginary part
+    float2* lines = sm;  // [H] complex lines: real line 2j in the real part, 2j + 1 in the imaginary part
     float2* tw = lines + H * LS;
-    float* raw = reinterpret_cast<float*>(tw + TWN);  // [C][M], scaled capture
-    for (int i = threadIdx.x; i < TWN; i += kZThreads) tw[i] = p.tw_z[i];
     const int N = p.N, y = blockIdx.y, x0 = blockIdx.x * C;
-    const bool time_inner = p.sz == 1;
+    constexpr int PZ = (M + NT - 1) / NT;
+    int begin[PZ], end[PZ];  // this thread's rows of mtx
+#pragma unroll
+    for (int q = 0; q < PZ; ++q) {
+        const int zp = min((int)threadIdx.x + q * NT, M - 1);
+        begin[q] = p.rp[zp];
+        end[q] = p.rp[zp + 1];
+    }
+    // The capture of real line i: in the half of its complex line that the padding leaves free.
+    auto raw = [&](int i) { return reinterpret_cast<float*>(lines + (i / 2) * LS + (M + M / 16)) + (i & 1) * (M + z_skew(LOG2Z)); };
     {
-        // All of a thread's loads in flight together; consecutive threads read
+        // Rounds of 8 loads in flight per thread; consecutive threads read
         // consecutive addresses in either layout.
-        constexpr int PL = (C * M + kZThreads - 1) / kZThreads;
-        float val[PL];
+        const bool time_inner = p.sz == 1;
+        const float* src = p.src + y * p.sy + (long long)x0 * p.sx;
+        constexpr int PL = (C * M + NT - 1) / NT, RL = PL < 8 ? PL : 8;
+        static_assert(PL % RL == 0, "whole rounds");
+        for (int i = threadIdx.x; i < TWN; i += NT) tw[i] = p.tw_z[i];
 #pragma unroll
-        for (int u = 0; u < PL; ++u) {
-            const int e = threadIdx.x + u * kZThreads;
-            const int i = time_inner ? e / M : e % C, z = time_inner ? e % M : e / C;
-            val[u] = (e < C * M && x0 + i < N) ? p.src[z * p.sz + y * p.sy + (long long)(x0 + i) * p.sx] : 0.f;
-        }
+        for (int r = 0; r < PL; r += RL) {
+            float val[RL];
 #pragma unroll
-        for (int u = 0; u < PL; ++u) {
-            const int e = threadIdx.x + u * kZThreads;
-            if (e >= C * M) break;
-            const int i = time_inner ? e / M : e % C, z = time_inner ? e % M : e / C;
-            float g = 1.f;
-            if (p.power > 0) g = p.gtab[p.tiled ? (z * N + y) % M : z];
-            raw[i * M + z] = val[u] * g;
+            for (int u = 0; u < RL; ++u) {
+                const int e = threadIdx.x + (r + u) * NT;
+                const int i = time_inner ? e / M : e % C, z = time_inner ? e % M : e / C;
+                val[u] = (C * M) % NT == 0 || e < C * M ? src[z * p.sz + i * p.sx] : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < RL; ++u) {
+                const int e = threadIdx.x + (r + u) * NT;
+                const int i = time_inner ? e / M : e % C, z = time_inner ? e % M : e / C;
+                if ((C * M) % NT == 0 || e < C * M) raw(i)[z] = val[u];
+            }
         }
     }
     __syncthreads();
     // z' < M only: the first FFT pass treats z' >= M as zero without reading it.
-    for (int e = threadIdx.x; e < C * M; e += kZThreads) {
-        const int i = e / M, zp = e % M;
-        float acc = 0.f;
-        for (int k = p.rp[zp]; k < p.rp[zp + 1]; ++k) acc = fmaf(p.v[k], raw[i * M + p.ci[k]], acc);
-        reinterpret_cast<float*>(lines + (i % H) * LS + pidx(zp))[i / H] = acc;
+    // A row's weights, and a bin's radiometric scale, are read once for all lines.
+#pragma unroll
+    for (int q = 0; q < PZ; ++q) {
+        const int zp = threadIdx.x + q * NT;
+        if (zp >= M) break;
+        float acc[C];
+#pragma unroll
+        for (int i = 0; i < C; ++i) acc[i] = 0.f;
+#pragma unroll 2
+        for (int k = begin[q]; k < end[q]; ++k) {
+            const float w = p.v[k];
+            const int c = p.ci[k];
+            const float g = p.power > 0 ? p.gtab[p.tiled ? (c * N + y) % M : c] : 1.f;
+#pragma unroll
+            for (int i = 0; i < C; ++i) acc[i] = fmaf(w, raw(i)[c] * g, acc[i]);
+        }
+#pragma unroll
+        for (int j = 0; j < H; ++j) lines[j * LS + pidx(zp)] = make_float2(acc[2 * j], acc[2 * j + 1]);
     }
     __syncthreads();
-    lean_fft<LOG2Z, 0, H, kZThreads, false, false, true, false>(lines, tw, LS);  // inputs z' >= M are zero
+    lean_fft<LOG2Z, 0, H, NT, false, false, true, false>(lines, tw, LS);  // inputs z' >= M are zero
     // P = FFT(a + i b) of two real lines: A[k] = (P[k] + conj(P[Z - k])) / 2,
     // B[k] = (P[k] - conj(P[Z - k])) / 2i; kz = 0..M stored.
-    for (int e = threadIdx.x; e < C * (M + 1); e += kZThreads) {
-        const int i = e % C, kz = e / C;
-        if (x0 + i >= N) continue;
-        const float2* l = lines + (i % H) * LS;
+    float4* out = reinterpret_cast<float4*>(p.buf + (size_t)y * N + x0);  // x0 and N are even
+    const size_t plane = (size_t)N * N / 2;
+#pragma unroll 4
+    for (int e = threadIdx.x; e < H * (M + 1); e += NT) {
+        const int j = e % H, kz = e / H;
+        const float2* l = lines + j * LS;
         const float2 pk = l[pidx(kz)], pm = l[pidx((Z - kz) & (Z - 1))];
-        p.buf[((size_t)kz * N + y) * N + x0 + i] = i < H ? make_float2(0.5f * (pk.x + pm.x), 0.5f * (pk.y - pm.y))
-                                                          : make_float2(0.5f * (pk.y + pm.y), 0.5f * (pm.x - pk.x));
+        out[kz * plane + j] = make_float4(0.5f * (pk.x + pm.x), 0.5f * (pk.y - pm.y),
+                                          0.5f * (pk.y + pm.y), 0.5f * (pm.x - pk.x));
     }
 }
 
@@ -221,7 +256,7 @@ __device__ __forceinline__ void fs128(float2 (&v)[16], float2* s, int n1, const 
     dft16<INV>(v);
 #pragma unroll
     for (int k1 = 1; k1 < 16; ++k1) {
-        float2 w = tw[16 + k1 * 8 + n1];  // second stage table: entry jm * 8 + k = w128^(jm k)
+        float2 w = tw[16 + k1 * 8 + n1];  // entry jm * 8 + k = w128^(jm k)
         if (INV) w.y = -w.y;
         v[k1] = cmul(v[k1], w);
     }
@@ -250,7 +285,8 @@ __global__ void __launch_bounds__(kP128Threads, 2) lct_plane128_kernel(LctFusedP
     float2* plane = sm;                              // [64][kP128Ps]
     float2* scratch = plane + 64 * kP128Ps;          // [kP128Lines][kP128ColLine]
     float2* tw = scratch + kP128Lines * kP128ColLine;
-    for (int i = threadIdx.x; i < kP128Tw; i += kP128Threads) tw[i] = p.tw_x[i];
+    // The second table by jm: a warp reads 8 or one of a jm's entries.
+    for (int i = threadIdx.x; i < kP128Tw; i += kP128Threads) tw[i] = p.tw_x[i < 16 ? i : 16 + (i - 16) % 8 * 16 + (i - 16) / 8];
     const size_t kz = blockIdx.x;
     float2* g = p.buf + kz * N * N;
     const int line = threadIdx.x >> 3, n1 = threadIdx.x & 7;
@@ -304,53 +340,81 @@ __global__ void __launch_bounds__(kP128Threads, 2) lct_plane128_kernel(LctFusedP
     }
 }
 
+// Bound like the forward pass; 27.9, 18.1 and 16.6 us by the same steps.
 template <int LOG2Z>
-__global__ void __launch_bounds__(kZThreads, 2) lct_zinv_kernel(LctFusedParams p) {
-    constexpr int Z = 1 << LOG2Z, M = Z / 2, C = z_lines(LOG2Z), H = C / 2, LS = line_stride(Z),
-                  TWN = stage_table_size(LOG2Z);
+__global__ void __launch_bounds__(z_threads(LOG2Z), z_ctas(LOG2Z)) lct_zinv_kernel(LctFusedParams p) {
+    constexpr int Z = 1 << LOG2Z, M = Z / 2, C = z_lines(LOG2Z), H = C / 2, LS = z_stride(LOG2Z),
+                  TWN = stage_table_size(LOG2Z), NT = z_threads(LOG2Z);
     extern __shared__ __align__(16) float2 sm[];
     float2* lines = sm;
-    float2* tw = lines + C * LS;
-    for (int i = threadIdx.x; i < TWN; i += kZThreads) tw[i] = p.tw_z[i];
+    float2* tw = lines + H * LS;
     const int N = p.N, y = blockIdx.y, x0 = blockIdx.x * C;
     {
-        constexpr int PL = (C * (M + 1) + kZThreads - 1) / kZThreads;
-        float2 t[PL];
+        // Q = A + i B over the whole period for the line pair (2j, 2j + 1), with
+        // A[Z - k] = conj(A[k]) and B[Z - k] = conj(B[k]) (and the real parts at
+        // k = 0 and M): IFFT(Q) = Re IFFT(A) + i Re IFFT(B).
+        const float4* in = reinterpret_cast<const float4*>(p.buf + (size_t)y * N + x0);  // x0 and N are even
+        const size_t plane = (size_t)N * N / 2;
+        constexpr int PL = (H * (M + 1) + NT - 1) / NT;
+        float4 t[PL];
 #pragma unroll
         for (int u = 0; u < PL; ++u) {
-            const int e = threadIdx.x + u * kZThreads;
-            const int i = e % C, kz = e / C;
-            t[u] = (e < C * (M + 1) && x0 + i < N) ? p.buf[((size_t)kz * N + y) * N + x0 + i] : make_float2(0.f, 0.f);
+            const int e = threadIdx.x + u * NT;
+            t[u] = e < H * (M + 1) ? in[(e / H) * plane + e % H] : make_float4(0.f, 0.f, 0.f, 0.f);
         }
+        for (int i = threadIdx.x; i < TWN; i += NT) tw[i] = p.tw_z[i];
 #pragma unroll
         for (int u = 0; u < PL; ++u) {
-            const int e = threadIdx.x + u * kZThreads;
-            if (e < C * (M + 1)) lines[(e % C) * LS + pidx(e / C)] = t[u];
+            const int e = threadIdx.x + u * NT, k = e / H;
+            float2* l = lines + (e % H) * LS;
+            const float4 q = t[u];
+            if (k == 0 || k == M) {
+                l[pidx(k)] = make_float2(q.x, q.z);
+            } else if (k < M) {
+                l[pidx(k)] = make_float2(q.x - q.w, q.y + q.z);
+                l[pidx(Z - k)] = make_float2(q.x + q.w, q.z - q.y);
+            }
         }
     }
     __syncthreads();
-    // Q = A + i B over the whole period for the line pair (j, j + H), with
-    // A[Z - k] = conj(A[k]) and B[Z - k] = conj(B[k]) (and the real parts at
-    // k = 0 and M): IFFT(Q) = Re IFFT(A) + i Re IFFT(B).
-    for (int e = threadIdx.x; e < H * (M + 1); e += kZThreads) {
-        const int j = e / (M + 1), k = e % (M + 1);
-        const float2 a = lines[j * LS + pidx(k)], b = lines[(j + H) * LS + pidx(k)];
-        if (k == 0 || k == M) {
-            lines[j * LS + pidx(k)] = make_float2(a.x, b.x);
+    constexpr int PZ = (M + NT - 1) / NT;
+    int begin[PZ], end[PZ];  // this thread's rows of mtx^T
+#pragma unroll
+    for (int q = 0; q < PZ; ++q) {
+        const int z = min((int)threadIdx.x + q * NT, M - 1);
+        begin[q] = p.rpt[z];
+        end[q] = p.rpt[z + 1];
+    }
+    lean_fft<LOG2Z, 0, H, NT, true, false, false, true>(lines, tw, LS);  // z < M kept
+    float* out = p.vol + (size_t)y * N + x0;
+    const bool vec = reinterpret_cast<uintptr_t>(p.vol) % 16 == 0;  // N and x0 are multiples of C
+#pragma unroll
+    for (int q = 0; q < PZ; ++q) {
+        const int z = threadIdx.x + q * NT;
+        if (z >= M) break;
+        float re[C];
+#pragma unroll
+        for (int i = 0; i < C; ++i) re[i] = 0.f;
+        for (int k = begin[q]; k < end[q]; ++k) {
+            const float w = p.vt[k];
+            const int at = pidx(p.cit[k]);
+#pragma unroll
+            for (int j = 0; j < H; ++j) {
+                const float2 c = lines[j * LS + at];
+                re[2 * j] = fmaf(w, c.x, re[2 * j]);
+                re[2 * j + 1] = fmaf(w, c.y, re[2 * j + 1]);
+            }
+        }
+        float* o = out + (size_t)z * N * N;
+#pragma unroll
+        for (int i = 0; i < C; ++i) re[i] = p.magnitude ? fabsf(re[i]) * p.scale : fmaxf(re[i] * p.scale, 0.f);
+        if (C >= 4 && vec) {
+#pragma unroll
+            for (int i = 0; i + 3 < C; i += 4) *reinterpret_cast<float4*>(o + i) = make_float4(re[i], re[i + 1], re[i + 2], re[i + 3]);
         } else {
-            lines[j * LS + pidx(k)] = make_float2(a.x - b.y, a.y + b.x);
-            lines[j * LS + pidx(Z - k)] = make_float2(a.x + b.y, b.x - a.y);
+#pragma unroll
+            for (int i = 0; i < C; ++i) o[i] = re[i];
         }
-    }
-    __syncthreads();
-    lean_fft<LOG2Z, 0, H, kZThreads, true, false, false, true>(lines, tw, LS);  // z < M kept
-    for (int e = threadIdx.x; e < C * M; e += kZThreads) {
-        const int i = e % C, z = e / C;
-        if (x0 + i >= N) continue;
-        const float* l = reinterpret_cast<const float*>(lines + (i % H) * LS) + i / H;  // a: real, b: imaginary
-        float re = 0.f;
-        for (int k = p.rpt[z]; k < p.rpt[z + 1]; ++k) re = fmaf(p.vt[k], l[2 * pidx(p.cit[k])], re);
-        p.vol[((size_t)z * N + y) * N + x0 + i] = p.magnitude ? fabsf(re) * p.scale : fmaxf(re * p.scale, 0.f);
     }
 }
 
@@ -482,22 +546,13 @@ fbp_status launch_rows_cols(fbp_context* ctx, const LctFusedParams& p, unsigned 
 
 template <int LOG2Z>
 fbp_status launch_z(fbp_context* ctx, const LctFusedParams& p, bool forward, cudaStream_t s) {
-    constexpr int C = z_lines(LOG2Z);
-    const dim3 grid(cdiv(p.N, C), p.N);
-    if (forward) {
-        constexpr size_t smem = zfwd_smem<LOG2Z>();
-        static_assert(smem <= 200 * 1024, "z-forward tile too large");
-        auto k = lct_zfwd_kernel<LOG2Z>;
-        FBP_TRY_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k<<<grid, kZThreads, smem, s>>>(p);
-        FBP_CHECK_LAUNCH(ctx, "lct_zfwd_kernel");
-    } else {
-        constexpr size_t smem = zinv_smem<LOG2Z>();
-        auto k = lct_zinv_kernel<LOG2Z>;
-        FBP_TRY_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k<<<grid, kZThreads, smem, s>>>(p);
-        FBP_CHECK_LAUNCH(ctx, "lct_zinv_kernel");
-    }
+    const dim3 grid(p.N / z_lines(LOG2Z), p.N);  // N is a power of two of at least 8
+    constexpr size_t smem = z_smem<LOG2Z>();
+    static_assert(smem * z_ctas(LOG2Z) <= 220 * 1024, "z tiles too large");
+    auto k = forward ? lct_zfwd_kernel<LOG2Z> : lct_zinv_kernel<LOG2Z>;
+    FBP_TRY_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k<<<grid, z_threads(LOG2Z), smem, s>>>(p);
+    FBP_CHECK_LAUNCH(ctx, forward ? "lct_zfwd_kernel" : "lct_zinv_kernel");
     return FBP_OK;
 }
 
@@ -558,8 +613,8 @@ fbp_status stage_twiddles(fbp_context* ctx, int log2n, cudaStream_t s, const flo
         for (int done = 0; done < log2n;) {
             const int rb = stage_radix_bits(log2n, done);
             const int ns = 1 << done, r = 1 << rb;
-            for (int jm = 0; jm < ns; ++jm)
-                for (int k = 0; k < r; ++k) {
+            for (int k = 0; k < r; ++k)
+                for (int jm = 0; jm < ns; ++jm) {
                     const double a = -2.0 * M_PI * (double)k * (double)jm / (double)(ns * r);
                     h.push_back(make_float2((float)std::cos(a), (float)std::sin(a)));
                 }
