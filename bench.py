@@ -180,9 +180,9 @@ def profiled_traffic():
 # Multi-function unit (XU) of an sm_100-class SM: 16 results per clock (4 per
 # SM sub-partition).  The confocal pair loop issues one sqrt.approx per pair
 # (the reference's bin, irreducible for bit-exact bins) and, with the batched
-# weights, one rcp.approx per two pairs.
+# weights, one rcp.approx per four pairs.
 XU_PER_CLK_SM = 16
-MUFU_PER_PAIR = 1.5
+MUFU_PER_PAIR = 1.25
 MUFU_PER_PAIR_FLOOR = 1.0
 
 
@@ -210,7 +210,7 @@ def gather_roofline(samples, bp_ms, clocks, hbm_peak, hbm_kind):
         "bound": "mufu", "achieved": per_clk_sm, "peak": peak, "unit": "voxel-samples/clk/SM",
         "frac": per_clk_sm / peak, "traffic": profiled_traffic(),
         "peak_basis": f"{XU_PER_CLK_SM} XU results/clk/SM / {MUFU_PER_PAIR} MUFU ops per pair (sqrt.approx + "
-                      f"rcp.approx per two pairs) at the sampled {mhz:.0f} MHz x {sms} SMs = "
+                      f"rcp.approx per four pairs) at the sampled {mhz:.0f} MHz x {sms} SMs = "
                       f"{peak * sms * mhz * 1e6:.3e} voxel-samples/s",
         "frac_of_bitwise_bin_floor": per_clk_sm / floor,
         "bitwise_bin_floor_note": f"{floor:.0f} voxel-samples/clk/SM: one sqrt.approx per pair, the least any "

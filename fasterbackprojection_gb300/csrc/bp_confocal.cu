@@ -5,9 +5,10 @@
 // reference launches one thread per (voxel, scan point) pair and adds each
 // contribution with a global FP32 atomic.  Here one CTA owns a tile of voxels
 // and walks all scan points; for every scan point it stages only the window
-// of time bins the tile can reach into shared memory (cp.async), so each
+// of time bins the tile can reach into shared memory (one bulk copy), so each
 // pair costs a shared-memory load instead of a global gather + atomic, and the
-// sum order is fixed (reproducible run to run).
+// sum order is fixed (reproducible run to run).  Volumes with few tiles walk
+// the scan points in several chains, one CTA each, folded afterwards.
 //
 // Data layout in HBM (per call, in the context's scratch):
 //   rows   [L][row_pitch] FP32: one padded row per scan point, time
@@ -281,7 +282,6 @@ fbp_status plan_window(const fbp_context* ctx, double ex, double ey, double ez, 
     out->capped = slot_w == cap;
     out->pitch = t_round + slot_w;
     const size_t per_stage = (size_t)window_bufs * (slot_w + align) * elem_bytes;  // per scan point of a stage
-    const size_t zero_slot = (size_t)(slot_w + align) * elem_bytes;
     // Points per stage: 32, halved down to 8 where that lets one more CTA share
     // the SM (at 128^2 x 1024 -> 128^3 a stage of 16 keeps three CTAs instead
     // of two), below 8 only where not even one CTA fits otherwise.
@@ -289,16 +289,16 @@ fbp_status plan_window(const fbp_context* ctx, double ex, double ey, double ez, 
     for (int n = ctas_per_sm; n >= 2 && !ch; --n) {
         const size_t room = kSmSharedBytes / n - kCtaReservedShared;
         for (int c = 32; c >= 8 && !ch; c >>= 1)
-            if (meta_bytes + (size_t)c * per_stage + zero_slot <= room) ch = c;
+            if (meta_bytes + (size_t)c * per_stage <= room) ch = c;
     }
     if (!ch) {
         ch = 32;
-        while (ch > 1 && meta_bytes + (size_t)ch * per_stage + zero_slot > (size_t)ctx->smem_optin) ch >>= 1;
+        while (ch > 1 && meta_bytes + (size_t)ch * per_stage > (size_t)ctx->smem_optin) ch >>= 1;
     }
-    if (meta_bytes + (size_t)ch * per_stage + zero_slot > (size_t)ctx->smem_optin)
+    if (meta_bytes + (size_t)ch * per_stage > (size_t)ctx->smem_optin)
         return set_error(FBP_ERR_UNSUPPORTED, std::string(who) + ": time-bin window too large for shared memory");
     out->ch = ch;
-    out->smem = meta_bytes + (size_t)ch * per_stage + zero_slot;
+    out->smem = meta_bytes + (size_t)ch * per_stage;
     return FBP_OK;
 }
 

@@ -577,7 +577,7 @@ __device__ __forceinline__ void confocal_tile(const ConfocalGatherParams& p, uin
     };
 
     // Compensated sums: in registers, or (16 voxels per thread) in shared
-    // memory behind the zero slot, [2 KV][NT] so a warp's accesses are
+    // memory behind the windows, [2 KV][NT] so a warp's accesses are
     // consecutive words.
     constexpr bool KSMEM = kahan_smem_bytes(KV, NT) > 0;
     static_assert(!SPLIT || KSMEM, "a split tile keeps its compensated sums in shared memory");
