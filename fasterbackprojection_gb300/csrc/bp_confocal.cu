@@ -151,10 +151,12 @@ fbp_status launch_confocal(fbp_context* ctx, const fbp_recon_info& in, const voi
 // the groups and half a group of set-up, at the rate of the CTAs resident
 // together (one or two reach 0.68 and 0.88 of three), the uneven end (a whole
 // CTA where tiles differ in their idle warps), and the sums' way through memory
-// and the fold's launch.  One CTA per tile against this rule: 32^2 x 256 ->
-// 32^3 328 -> 45 us (16 chains), 64^2 x 512 -> 64^3 1264 -> 432 us (7), 90^2 x
-// 700 -> 75 x 101 x 83 4028 -> 2189 us (16), 128^2 x 1024 -> 128^3 14.2 -> 11.5
-// ms (5), 8^2 x 16^2 x 512 -> 48^3 2251 -> 666 us (14).  The sums through the
+// and the fold's launch.  One CTA per tile against this rule (both with the
+// tables' launches of their own, which one launch for rows and tables has since
+// taken 8-28 us off): 32^2 x 256 -> 32^3 328 -> 45 us (16 chains), 64^2 x 512 ->
+// 64^3 1264 -> 432 us (7), 90^2 x 700 -> 75 x 101 x 83 4028 -> 2189 us (16),
+// 128^2 x 1024 -> 128^3 14.2 -> 11.5 ms (5), 8^2 x 16^2 x 512 -> 48^3 2251 ->
+// 666 us (14).  The sums through the
 // shared memory of a cluster instead (at most 16 chains, and clusters leave
 // part of a GPC's slots empty): 48, 483, 2596 us, 11.9 ms, 728 us.
 uint32_t split_chains(const fbp_context* ctx, uint64_t tiles, double busy, uint64_t groups, int occ, double group_us,

@@ -2,10 +2,11 @@
 //
 // Replaces Laser::reconstructAABBExhaustive (Laser.cu:500-516) and
 // backprojectExhaustiveVoxel (transient_reconstruction.cuh:138-166).  Same
-// structure as the confocal gather: a CTA, or several, per voxel tile, the (laser, SPAD) pairs walked in groups, each pair's reachable
-// time-bin window copied to shared memory.  The pair index splits as l = ls / S, s = ls % S; the
-// reference splits by L (transient_reconstruction.cuh:147-148), which is the
-// same only when L == S and reads past the laser table otherwise.
+// structure as the confocal gather: a CTA, or several, per voxel tile, the
+// (laser, SPAD) pairs walked in groups, each pair's reachable time-bin window
+// copied to shared memory.  The pair index splits as l = ls / S, s = ls % S;
+// the reference splits by L (transient_reconstruction.cuh:147-148), which is
+// the same only when L == S and reads past the laser table otherwise.
 #include "fbp_internal.cuh"
 #include "bp_common.cuh"
 
@@ -58,9 +59,9 @@ struct ExhaustiveGatherParams {
 enum { EX_T0ZERO = 0, EX_FAST = 1, EX_EXACT = 2 };
 
 // One CTA of 32*WY*WZ threads (or p.chains of them, one per range of pair
-// groups, their sums folded afterwards) owns a tile of KV x 8*WY x 4*WZ voxels, like the confocal
-// gather, with its pipeline: plans two groups ahead, windows by bulk copies,
-// no barrier across the CTA.
+// groups, their sums folded afterwards) owns a tile of KV x 8*WY x 4*WZ
+// voxels, like the confocal gather, with its pipeline: plans two groups ahead,
+// windows by bulk copies, no barrier across the CTA.
 // LB = 4: pairs are walked as (laser block of 4, SPAD, laser in block), so
 // the SPAD-to-voxel distance is computed once per SPAD for 4 lasers (the 4
 // laser distances are kept per block); a last block short of lasers reads
