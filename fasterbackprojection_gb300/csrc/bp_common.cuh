@@ -169,7 +169,9 @@ uint32_t split_chains(const fbp_context* ctx, uint64_t tiles, double busy, uint6
 double busy_warps(const uint32_t res[3]);
 constexpr double kGatherGroupUs = 6.3;  // 32 scan points x 4096 voxels
 // out[i] = the chains' sums [chains][sum, compensation][n], folded in order.
-fbp_status chain_sums(fbp_context* ctx, uint32_t chains, uint64_t n, cudaStream_t stream, float** sums);
+// Scratch for the chains' sums of n outputs; *chains becomes 1 where there is
+// none (no memory, or a stream under capture and too small a buffer).
+fbp_status chain_sums(fbp_context* ctx, uint32_t* chains, uint64_t n, cudaStream_t stream, float** sums);
 fbp_status fold_chains(fbp_context* ctx, const float* sums, uint32_t chains, uint64_t n, float* out, cudaStream_t stream);
 // CTAs of `smem` bytes of dynamic shared memory an SM holds, at most `most`.
 inline int resident_ctas(size_t smem, int most) {
@@ -213,9 +215,9 @@ struct PrepTables {
 };
 fbp_status prepare_gather(fbp_context* ctx, int dtype, const PrepRows& rows, const PrepTables& tables, cudaStream_t stream);
 // The tables' part of the request, in the context's scratch (sensor_xyz null:
-// confocal).
+// confocal; axes: a volume's coordinates too).
 fbp_status table_buffers(fbp_context* ctx, const fbp_recon_info& in, const float* laser_xyz, const float* sensor_xyz,
-                         cudaStream_t stream, PrepTables* t);
+                         bool axes, cudaStream_t stream, PrepTables* t);
 
 __global__ void axis_tables_kernel(float* __restrict__ xs, float* __restrict__ ys, float* __restrict__ zs,
                                    uint32_t Vx, uint32_t Vy, uint32_t Vz, float mnx, float mny, float mnz, float sx,

@@ -97,7 +97,7 @@ fbp_status launch_confocal(fbp_context* ctx, const fbp_recon_info& in, const voi
     void* rows = nullptr;
     FBP_TRY(workspace(ctx, WS_CUBE_ROWS, (size_t)L * wp.pitch * sizeof(float), stream, &rows));
     PrepTables tables{};
-    FBP_TRY(table_buffers(ctx, in, laser_xyz, nullptr, stream, &tables));
+    FBP_TRY(table_buffers(ctx, in, laser_xyz, nullptr, true, stream, &tables));
     FBP_TRY(prepare_gather(ctx, dtype, PrepRows{cube, static_cast<float*>(rows), L, T, wp.pitch, layout == FBP_LAYOUT_TIME_MAJOR},
                            tables, stream));
 
@@ -117,6 +117,7 @@ fbp_status launch_confocal(fbp_context* ctx, const fbp_recon_info& in, const voi
     p.slot_w = wp.slot_w;
     p.ch = wp.ch;
     p.chains = smp ? 1 : gather_chains(ctx, in, wp.smem);
+    FBP_TRY(chain_sums(ctx, &p.chains, (uint64_t)p.Vx * p.Vy * p.Vz, stream, &p.chain_sums));
     for (int k = 0; k < 3; ++k) p.vs[k] = in.voxel_size[k];
     p.exact_weights = ctx->weight_mode == FBP_WEIGHTS_REFERENCE;
     if (smp) p.smp = *smp;
@@ -145,6 +146,10 @@ fbp_status launch_confocal(fbp_context* ctx, const fbp_recon_info& in, const voi
 
 }  // namespace
 
+// The most scratch that chains may ask for (volumes beyond 16 M voxels have tiles
+// enough for every SM).
+constexpr size_t kChainSumBytes = (size_t)128 << 20;
+
 // Chains (CTAs per tile) of a gather: 1 where the tiles alone keep every SM
 // busy, else as many as a model of the launch asks for.  The model, in units of
 // one group at an SM's full rate: the busiest SM's CTAs, each with its share of
@@ -165,7 +170,8 @@ uint32_t split_chains(const fbp_context* ctx, uint64_t tiles, double busy, uint6
     constexpr uint32_t kMaxChains = 32;
     uint32_t best = 1;
     double best_t = 0.0;
-    for (uint32_t c = 1; c <= std::min<uint64_t>(kMaxChains, groups); ++c) {
+    const uint64_t most = std::min<uint64_t>(std::min<uint64_t>(kMaxChains, groups), kChainSumBytes / (8 * n));
+    for (uint32_t c = 1; c <= std::max<uint64_t>(most, 1); ++c) {
         const uint64_t per_sm = cdiv(tiles * c, (uint64_t)ctx->sm_count);
         const double rate = kRate[std::min<uint64_t>(per_sm, (uint64_t)occ) - 1] / kRate[occ - 1];
         const double ctas = busy < 1.0 ? (double)(tiles * c) * busy / ctx->sm_count + 1.0 : (double)per_sm + 0.3;
@@ -192,9 +198,33 @@ uint32_t gather_chains(const fbp_context* ctx, const fbp_recon_info& in, size_t 
                         kGatherGroupUs, (uint64_t)in.voxel_res[0] * in.voxel_res[1] * in.voxel_res[2]);
 }
 
-fbp_status chain_sums(fbp_context* ctx, uint32_t chains, uint64_t n, cudaStream_t stream, float** sums) {
-    void* ws = nullptr;
-    FBP_TRY(workspace(ctx, WS_CHAIN_SUMS, (size_t)2 * chains * n * sizeof(float), stream, &ws));
+fbp_status chain_sums(fbp_context* ctx, uint32_t* chains, uint64_t n, cudaStream_t stream, float** sums) {
+    if (*chains <= 1) return FBP_OK;
+    const size_t bytes = (size_t)2 * *chains * n * sizeof(float);
+    size_t& have = ctx->ws_bytes[WS_CHAIN_SUMS];
+    void*& ws = ctx->ws[WS_CHAIN_SUMS];
+    if (have < bytes) {
+        // A smaller volume may want more of this than a larger one, so a graph
+        // captured before must not lose its buffer to a later call: an outgrown
+        // one lives as long as the context, and each at least doubles the last
+        // (up to kChainSumBytes, which bounds them all together at twice that).
+        const size_t grown = std::max(bytes, std::min(2 * have, kChainSumBytes));
+        void* p = nullptr;
+        if (!workspace_ready(ctx, WS_CHAIN_SUMS, bytes, stream)) {
+            *chains = 1;
+            return FBP_OK;
+        }
+        const cudaError_t e = cudaMalloc(&p, grown);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            *chains = 1;
+            return FBP_OK;
+        }
+        FBP_TRY_CUDA(e);
+        if (ws) ctx->ws_outgrown.push_back(ws);
+        ws = p;
+        have = grown;
+    }
     *sums = static_cast<float*>(ws);
     return FBP_OK;
 }

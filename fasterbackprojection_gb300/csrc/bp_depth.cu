@@ -40,6 +40,10 @@ struct DepthTileParams {
     static constexpr uint32_t kWindowFloats = (uint32_t)((kSmem - kMeta - kSums) / sizeof(float));
     // Longest row whose whole-row windows fit, one scan point to a stage.
     static constexpr uint32_t kMaxBins = (kWindowFloats / 2 - 8) / 4 * 4;
+    static uint32_t pitch_of(uint32_t T) { return (T + 3) / 4 * 4 + kSlot; }
+    static size_t row_bytes(const fbp_recon_info& in) {
+        return (size_t)in.num_laser_targets * pitch_of(in.num_time_bins) * sizeof(float);
+    }
 };
 
 // A CTA (or p.chains of them, one per range of scan-point groups) owns 256
@@ -384,7 +388,7 @@ fbp_status go_depth_tiles(fbp_context* ctx, DepthTileParams p, dim3 grid, cudaSt
     const size_t smem = DepthTileParams::kMeta + DepthTileParams::kSums + DepthTileParams::kWindowFloats * sizeof(float);
     FBP_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const uint64_t n = (uint64_t)p.L * p.D;
-    if (p.chains > 1) FBP_TRY(chain_sums(ctx, p.chains, n, stream, &p.chain_sums));
+    FBP_TRY(chain_sums(ctx, &p.chains, n, stream, &p.chain_sums));
     grid.x *= p.chains;
     kernel<<<grid, DepthTileParams::kThreads, smem, stream>>>(p);
     FBP_CHECK_LAUNCH(ctx, "depth_tile_kernel");
@@ -397,12 +401,11 @@ fbp_status launch_depth_tiles(fbp_context* ctx, const fbp_recon_info& in, const 
                               cudaStream_t stream) {
     const uint32_t L = in.num_laser_targets, T = in.num_time_bins;
     DepthTileParams p{};
-    p.pitch = (T + 3) / 4 * 4 + DepthTileParams::kSlot;
+    p.pitch = DepthTileParams::pitch_of(T);
     void* rows = nullptr;
-    FBP_TRY(workspace(ctx, WS_CUBE_ROWS, (size_t)L * p.pitch * sizeof(float), stream, &rows));
+    FBP_TRY(workspace(ctx, WS_CUBE_ROWS, DepthTileParams::row_bytes(in), stream, &rows));
     PrepTables tables{};
-    FBP_TRY(table_buffers(ctx, in, laser_xyz, nullptr, stream, &tables));
-    for (uint32_t& r : tables.res) r = 0;  // no volume
+    FBP_TRY(table_buffers(ctx, in, laser_xyz, nullptr, false, stream, &tables));
     FBP_TRY(prepare_gather(ctx, dtype,
                            PrepRows{cube, static_cast<float*>(rows), L, T, p.pitch, layout == FBP_LAYOUT_TIME_MAJOR}, tables,
                            stream));
@@ -532,8 +535,13 @@ fbp_status launch_depths(fbp_context* ctx, const fbp_recon_info& in, const void*
                          const float* laser_xyz, const float* sensor_xyz, const double* depths, uint32_t D,
                          float* act, cudaStream_t stream) {
     const bool exhaustive = in.capture_system == FBP_EXHAUSTIVE;
-    if (!exhaustive && in.num_time_bins <= DepthTileParams::kMaxBins && cdiv(D, DepthTileParams::kDepths) <= 65535)
-        return launch_depth_tiles(ctx, in, cube, dtype_of<S>(), layout, laser_xyz, depths, D, act, stream);
+    if (!exhaustive && in.num_time_bins <= DepthTileParams::kMaxBins && cdiv(D, DepthTileParams::kDepths) <= 65535 &&
+        workspace_ready(ctx, WS_CUBE_ROWS, DepthTileParams::row_bytes(in), stream)) {
+        const fbp_status st = launch_depth_tiles(ctx, in, cube, dtype_of<S>(), layout, laser_xyz, depths, D, act, stream);
+        if (st != FBP_ERR_OOM) return st;
+        cudaGetLastError();  // no memory for FP32 rows: the kernel below needs the capture's own bytes
+        clear_error();
+    }
     const uint32_t L = in.num_laser_targets, Sn = exhaustive ? in.num_sensor_targets : 1, T = in.num_time_bins;
     const uint32_t pitch = (T + 7) / 8 * 8;
     const uint64_t R = (uint64_t)L * Sn;

@@ -405,7 +405,7 @@ fbp_status go_exhaustive(fbp_context* ctx, ExhaustiveGatherParams p, dim3 grid, 
     auto kernel = exhaustive_gather_kernel<kKV, kWY, kWZ, MODE, BOUNCE, CLAMP, LB>;
     FBP_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const uint64_t n = (uint64_t)p.Vx * p.Vy * p.Vz;
-    if (p.chains > 1) FBP_TRY(chain_sums(ctx, p.chains, n, stream, &p.chain_sums));
+    FBP_TRY(chain_sums(ctx, &p.chains, n, stream, &p.chain_sums));
     grid.x *= p.chains;
     kernel<<<grid, 32 * kWY * kWZ, smem, stream>>>(p);
     FBP_CHECK_LAUNCH(ctx, "exhaustive_gather_kernel");
@@ -448,7 +448,7 @@ fbp_status launch_exhaustive(fbp_context* ctx, const fbp_recon_info& in, const v
     void* rows = nullptr;
     FBP_TRY(workspace(ctx, WS_CUBE_ROWS, npairs * pitch * sizeof(float), stream, &rows));
     PrepTables tables{};
-    FBP_TRY(table_buffers(ctx, in, laser_xyz, sensor_xyz, stream, &tables));
+    FBP_TRY(table_buffers(ctx, in, laser_xyz, sensor_xyz, true, stream, &tables));
     FBP_TRY(prepare_gather(ctx, dtype, PrepRows{cube, static_cast<float*>(rows), npairs, T, pitch, 0}, tables, stream));
 
     ExhaustiveGatherParams p{};

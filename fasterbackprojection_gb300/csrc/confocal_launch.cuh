@@ -34,10 +34,7 @@ fbp_status go_confocal(fbp_context* ctx, ConfocalGatherParams p, dim3 grid, size
     auto kernel = confocal_gather_kernel<KV, kWY, kWZ, PATH, BOUNCE, SAMPLED, CLAMP, SPLIT>;
     FBP_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const uint64_t n = (uint64_t)p.Vx * p.Vy * p.Vz;
-    if (SPLIT) {
-        FBP_TRY(chain_sums(ctx, p.chains, n, stream, &p.chain_sums));
-        grid.x *= p.chains;
-    }
+    if (SPLIT) grid.x *= p.chains;
     kernel<<<grid, 32 * kWY * kWZ, smem, stream>>>(p);
     FBP_CHECK_LAUNCH(ctx, "confocal_gather_kernel");
     return SPLIT ? fold_chains(ctx, p.chain_sums, p.chains, n, p.volume, stream) : FBP_OK;

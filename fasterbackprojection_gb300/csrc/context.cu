@@ -76,6 +76,16 @@ fbp_status workspace(fbp_context* ctx, int slot, size_t bytes, cudaStream_t stre
     return FBP_OK;
 }
 
+bool workspace_ready(const fbp_context* ctx, int slot, size_t bytes, cudaStream_t stream) {
+    if (ctx->ws_bytes[slot] >= bytes) return true;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &st) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return st == cudaStreamCaptureStatusNone;
+}
+
 }  // namespace fbp
 
 using namespace fbp;
@@ -123,6 +133,7 @@ fbp_status fbp_destroy(fbp_context* ctx) {
         cudaDeviceSynchronize();
         for (int i = 0; i < WS_NUM_SLOTS; ++i)
             if (ctx->ws[i]) cudaFree(ctx->ws[i]);
+        for (void* t : ctx->ws_outgrown) cudaFree(t);
         for (void* t : ctx->twiddles)
             if (t) cudaFree(t);
         for (void* t : ctx->stage_twiddles)

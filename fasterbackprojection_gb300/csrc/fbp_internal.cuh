@@ -1,6 +1,7 @@
 // Internal declarations shared by the libfbp translation units.
 #pragma once
 
+#include <vector>
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -100,6 +101,7 @@ struct fbp_context {
     int smem_optin = 0;
     void* ws[fbp::WS_NUM_SLOTS] = {};
     size_t ws_bytes[fbp::WS_NUM_SLOTS] = {};
+    std::vector<void*> ws_outgrown;  // buffers of WS_CHAIN_SUMS that captured graphs may still use
     int* status_dev = nullptr;  // device status word: 0 ok, else an fbp_status
     int weight_mode = FBP_WEIGHTS_BATCHED;  // fbp_weight_mode of the gathers
     uint64_t launches = 0;
@@ -123,6 +125,9 @@ fbp_status check_ctx(fbp_context* ctx);
 fbp_status use_device(int device);
 // Returns a device buffer of at least `bytes` in slot `slot`.
 fbp_status workspace(fbp_context* ctx, int slot, size_t bytes, cudaStream_t stream, void** out);
+// Whether workspace(slot, bytes) can be had now: false where it would have to
+// allocate while the stream is being captured.
+bool workspace_ready(const fbp_context* ctx, int slot, size_t bytes, cudaStream_t stream);
 
 // Shared memory of an SM, and what each resident CTA takes beside its own.
 constexpr size_t kSmSharedBytes = 228 * 1024, kCtaReservedShared = 1024;

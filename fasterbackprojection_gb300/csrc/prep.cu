@@ -138,14 +138,15 @@ fbp_status prepare_gather(fbp_context* ctx, int dtype, const PrepRows& r, const 
 }
 
 fbp_status table_buffers(fbp_context* ctx, const fbp_recon_info& in, const float* laser_xyz, const float* sensor_xyz,
-                         cudaStream_t stream, PrepTables* t) {
+                         bool axes, cudaStream_t stream, PrepTables* t) {
     const uint32_t L = in.num_laser_targets, Sn = sensor_xyz ? in.num_sensor_targets : 0;
     void *lp = nullptr, *sp = nullptr, *ap = nullptr;
     FBP_TRY(workspace(ctx, WS_SCAN_TABLE, (size_t)L * sizeof(float4), stream, &lp));
     if (Sn) FBP_TRY(workspace(ctx, WS_SENSOR_TABLE, (size_t)Sn * sizeof(float4), stream, &sp));
-    size_t axes = 0;
-    for (int k = 0; k < 3; ++k) axes += in.voxel_res[k];
-    FBP_TRY(workspace(ctx, WS_AXIS_TABLES, axes * sizeof(float), stream, &ap));
+    if (axes) {
+        const size_t n = (size_t)in.voxel_res[0] + in.voxel_res[1] + in.voxel_res[2];
+        FBP_TRY(workspace(ctx, WS_AXIS_TABLES, n * sizeof(float), stream, &ap));
+    }
     t->laser_xyz = laser_xyz;
     t->sensor_xyz = sensor_xyz;
     t->num_lasers = L;
@@ -159,7 +160,7 @@ fbp_status table_buffers(fbp_context* ctx, const fbp_recon_info& in, const float
         t->sensor_pos[k] = in.sensor_position[k];
         t->min[k] = in.hidden_min[k];
         t->size[k] = in.voxel_size[k];
-        t->res[k] = in.voxel_res[k];
+        t->res[k] = axes ? in.voxel_res[k] : 0;
     }
     return FBP_OK;
 }

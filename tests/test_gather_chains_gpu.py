@@ -94,3 +94,72 @@ def test_exhaustive_chains_against_fp64(ctx, cuda, nl, ns, T, vres, bounce, t0):
     want = cpu.exhaustive_voxel(info, cap.cube, cap.laser_xyz, cap.sensor_xyz, bins=bins)
     assert (bins >= 0).any()
     assert rel_l2(vol.cpu().numpy(), want) < 1e-6
+
+
+def _capture(cuda, n, T, vres, seed):
+    import torch
+
+    from fasterbackprojection_gb300 import make_info, scenes
+
+    cap = scenes.confocal_points(n, T, 4.92 / T / scenes.LIGHT_SPEED, n_points=20, depth_range=(0.3, 1.3), seed=seed)
+    hmin, vs = scenes.volume_geometry(vres, depth_range=(0.0, 1.6))
+    info = make_info(num_laser_targets=n * n, num_time_bins=T, time_step=cap.time_step, voxel_res=vres,
+                     hidden_min=hmin, voxel_size=vs, discard_first_last_bounces=1)
+    return info, torch.from_numpy(cap.cube).to(cuda), torch.from_numpy(cap.laser_xyz).to(cuda)
+
+
+def _launches(ctx, call):
+    before = ctx.launches
+    out = call()
+    return ctx.launches - before, out
+
+
+@pytest.fixture()
+def own_ctx(cuda):
+    from fasterbackprojection_gb300 import Context
+
+    c = Context()
+    yield c
+    c.check_device_status()
+    c.close()
+
+
+def test_capture_without_chain_scratch_runs_one_chain(own_ctx, cuda):
+    """A context that has only run a volume too large for chains can be captured
+    with a smaller one, although its chains' sums would need an allocation: one
+    CTA per tile then, the same volume to FP32 rounding."""
+    import torch
+
+    ctx = own_ctx
+    big = _capture(cuda, 32, 1024, (256, 256, 256), 1)  # rows and tables as large as the small one needs
+    small = _capture(cuda, 32, 256, (32, 32, 32), 2)
+    assert _launches(ctx, lambda: ctx.backproject_confocal(*big))[0] == 2  # rows, gather
+    out = torch.empty((32, 32, 32), device=cuda)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        count, _ = _launches(ctx, lambda: ctx.backproject_confocal(*small, out=out))
+    assert count == 2
+    graph.replay()
+    count, eager = _launches(ctx, lambda: ctx.backproject_confocal(*small))
+    assert count == 3  # the chains' fold too
+    assert rel_l2(out.cpu().numpy(), eager.cpu().numpy()) < 1e-6
+
+
+def test_captured_chains_outlive_a_call_that_needs_more(own_ctx, cuda):
+    """A captured call keeps its chain scratch when a later call with fewer scan
+    points, but more voxels, outgrows it."""
+    import torch
+
+    ctx = own_ctx
+    first = _capture(cuda, 32, 512, (16, 16, 170), 3)
+    more = _capture(cuda, 20, 256, (64, 64, 72), 4)
+    want = ctx.backproject_confocal(*first)
+    out = torch.empty_like(want)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ctx.backproject_confocal(*first, out=out)
+    again = ctx.backproject_confocal(*more)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
+    assert torch.equal(ctx.backproject_confocal(*more), again)
