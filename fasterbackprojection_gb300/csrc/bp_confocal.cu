@@ -94,14 +94,15 @@ fbp_status launch_confocal(fbp_context* ctx, const fbp_recon_info& in, const voi
                         ConfocalGatherParams::kWindowBufs));
     if (smp) wp.smem -= kSampledStaticSmem;
 
-    void* rows = nullptr;
-    FBP_TRY(workspace(ctx, WS_CUBE_ROWS, (size_t)L * wp.pitch * sizeof(float), stream, &rows));
+    ConfocalGatherParams p{};
+    p.chains = smp ? 1 : gather_chains(ctx, in, wp.smem);
+    float* rows = nullptr;
+    FBP_TRY(gather_scratch(ctx, (size_t)L * wp.pitch * sizeof(float), &p.chains, (uint64_t)Vx * Vy * (z_end - z_begin), stream,
+                           &rows, &p.chain_sums));
     PrepTables tables{};
     FBP_TRY(table_buffers(ctx, in, laser_xyz, nullptr, true, stream, &tables));
-    FBP_TRY(prepare_gather(ctx, dtype, PrepRows{cube, static_cast<float*>(rows), L, T, wp.pitch, layout == FBP_LAYOUT_TIME_MAJOR},
-                           tables, stream));
+    FBP_TRY(prepare_gather(ctx, dtype, PrepRows{cube, rows, L, T, wp.pitch, layout == FBP_LAYOUT_TIME_MAJOR}, tables, stream));
 
-    ConfocalGatherParams p{};
     p.scan = tables.lasers;
     p.xs = tables.axes;
     p.ys = p.xs + Vx;
@@ -116,8 +117,6 @@ fbp_status launch_confocal(fbp_context* ctx, const fbp_recon_info& in, const voi
     p.row_pitch = wp.pitch;
     p.slot_w = wp.slot_w;
     p.ch = wp.ch;
-    p.chains = smp ? 1 : gather_chains(ctx, in, wp.smem);
-    FBP_TRY(chain_sums(ctx, &p.chains, (uint64_t)p.Vx * p.Vy * p.Vz, stream, &p.chain_sums));
     for (int k = 0; k < 3; ++k) p.vs[k] = in.voxel_size[k];
     p.exact_weights = ctx->weight_mode == FBP_WEIGHTS_REFERENCE;
     if (smp) p.smp = *smp;
@@ -198,11 +197,29 @@ uint32_t gather_chains(const fbp_context* ctx, const fbp_recon_info& in, size_t 
                         kGatherGroupUs, (uint64_t)in.voxel_res[0] * in.voxel_res[1] * in.voxel_res[2]);
 }
 
-fbp_status chain_sums(fbp_context* ctx, uint32_t* chains, uint64_t n, cudaStream_t stream, float** sums) {
-    if (*chains <= 1) return FBP_OK;
-    const size_t bytes = (size_t)2 * *chains * n * sizeof(float);
+fbp_status gather_scratch(fbp_context* ctx, size_t row_bytes, uint32_t* chains, uint64_t n, cudaStream_t stream,
+                          float** rows, float** sums) {
+    void* r = nullptr;
+    const size_t at = (row_bytes + 255) & ~size_t(255), bytes = *chains > 1 ? (size_t)2 * *chains * n * sizeof(float) : 0;
     size_t& have = ctx->ws_bytes[WS_CHAIN_SUMS];
     void*& ws = ctx->ws[WS_CHAIN_SUMS];
+    // A context's first call makes one allocation for both (each costs tens of
+    // microseconds); later ones use what is behind the rows where it is enough.
+    if (ctx->ws_bytes[WS_CUBE_ROWS] < row_bytes && have < bytes) {
+        const fbp_status st = workspace(ctx, WS_CUBE_ROWS, at + bytes, stream, &r);
+        if (st != FBP_OK && st != FBP_ERR_OOM) return st;
+        if (st == FBP_ERR_OOM) {
+            cudaGetLastError();
+            clear_error();
+        }
+    }
+    FBP_TRY(workspace(ctx, WS_CUBE_ROWS, row_bytes, stream, &r));
+    *rows = static_cast<float*>(r);
+    if (*chains <= 1) return FBP_OK;
+    if (ctx->ws_bytes[WS_CUBE_ROWS] >= at + bytes) {
+        *sums = reinterpret_cast<float*>(static_cast<char*>(r) + at);
+        return FBP_OK;
+    }
     if (have < bytes) {
         // A smaller volume may want more of this than a larger one, so a graph
         // captured before must not lose its buffer to a later call: an outgrown

@@ -388,7 +388,6 @@ fbp_status go_depth_tiles(fbp_context* ctx, DepthTileParams p, dim3 grid, cudaSt
     const size_t smem = DepthTileParams::kMeta + DepthTileParams::kSums + DepthTileParams::kWindowFloats * sizeof(float);
     FBP_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const uint64_t n = (uint64_t)p.L * p.D;
-    FBP_TRY(chain_sums(ctx, &p.chains, n, stream, &p.chain_sums));
     grid.x *= p.chains;
     kernel<<<grid, DepthTileParams::kThreads, smem, stream>>>(p);
     FBP_CHECK_LAUNCH(ctx, "depth_tile_kernel");
@@ -402,29 +401,28 @@ fbp_status launch_depth_tiles(fbp_context* ctx, const fbp_recon_info& in, const 
     const uint32_t L = in.num_laser_targets, T = in.num_time_bins;
     DepthTileParams p{};
     p.pitch = DepthTileParams::pitch_of(T);
-    void* rows = nullptr;
-    FBP_TRY(workspace(ctx, WS_CUBE_ROWS, DepthTileParams::row_bytes(in), stream, &rows));
-    PrepTables tables{};
-    FBP_TRY(table_buffers(ctx, in, laser_xyz, nullptr, false, stream, &tables));
-    FBP_TRY(prepare_gather(ctx, dtype,
-                           PrepRows{cube, static_cast<float*>(rows), L, T, p.pitch, layout == FBP_LAYOUT_TIME_MAJOR}, tables,
-                           stream));
-    p.scan = tables.lasers;
-    p.xyz = laser_xyz;
-    p.depths = depths;
-    p.rows = static_cast<const float*>(rows);
-    p.act = act;
-    p.status = ctx->status_dev;
-    p.L = L; p.D = D; p.T = T;
     const uint32_t side = (uint32_t)std::lround(std::sqrt((double)L));
     p.side = (uint64_t)side * side == L ? side : 0;
     p.nx = in.wall_normal[0]; p.ny = in.wall_normal[1]; p.nz = in.wall_normal[2];
-    p.t0 = in.time_offset;
-    p.dt = in.time_step;
     const uint64_t tiles = p.side ? (uint64_t)cdiv(side, 16) * cdiv(side, 16) : cdiv(L, DepthTileParams::kThreads);
     const dim3 grid((unsigned)tiles, cdiv(D, DepthTileParams::kDepths));
     const bool yonly = p.nx == 0.f && p.nz == 0.f, bounce = in.discard_first_last_bounces == 0;
     p.chains = split_chains(ctx, tiles * grid.y, 1.0, cdiv(L, DepthTileParams::kGroup), yonly ? 3 : 2, 5.0, (uint64_t)L * D);
+    float* rows = nullptr;
+    FBP_TRY(gather_scratch(ctx, DepthTileParams::row_bytes(in), &p.chains, (uint64_t)L * D, stream, &rows, &p.chain_sums));
+    PrepTables tables{};
+    FBP_TRY(table_buffers(ctx, in, laser_xyz, nullptr, false, stream, &tables));
+    FBP_TRY(prepare_gather(ctx, dtype,
+                           PrepRows{cube, rows, L, T, p.pitch, layout == FBP_LAYOUT_TIME_MAJOR}, tables, stream));
+    p.scan = tables.lasers;
+    p.xyz = laser_xyz;
+    p.depths = depths;
+    p.rows = rows;
+    p.act = act;
+    p.status = ctx->status_dev;
+    p.L = L; p.D = D; p.T = T;
+    p.t0 = in.time_offset;
+    p.dt = in.time_step;
     const bool plain = !bounce && p.t0 == 0.f;
     if (yonly) {
         if (bounce) return go_depth_tiles<true, true, false>(ctx, p, grid, stream);

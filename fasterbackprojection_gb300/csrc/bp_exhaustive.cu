@@ -405,7 +405,6 @@ fbp_status go_exhaustive(fbp_context* ctx, ExhaustiveGatherParams p, dim3 grid, 
     auto kernel = exhaustive_gather_kernel<kKV, kWY, kWZ, MODE, BOUNCE, CLAMP, LB>;
     FBP_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const uint64_t n = (uint64_t)p.Vx * p.Vy * p.Vz;
-    FBP_TRY(chain_sums(ctx, &p.chains, n, stream, &p.chain_sums));
     grid.x *= p.chains;
     kernel<<<grid, 32 * kWY * kWZ, smem, stream>>>(p);
     FBP_CHECK_LAUNCH(ctx, "exhaustive_gather_kernel");
@@ -445,13 +444,22 @@ fbp_status launch_exhaustive(fbp_context* ctx, const fbp_recon_info& in, const v
     const uint32_t slot_w = wp.slot_w, pitch = wp.pitch;
     const uint64_t npairs = (uint64_t)L * Sn;
 
-    void* rows = nullptr;
-    FBP_TRY(workspace(ctx, WS_CUBE_ROWS, npairs * pitch * sizeof(float), stream, &rows));
+    // Laser blocks of 4 where padding the lasers to whole blocks costs no more
+    // than a SPAD distance per pair would (about 8 of 21 issue cycles).
+    const bool blocks = wp.ch % 4 == 0 && (L + 3) / 4 * 4 * 3 <= L * 4;
+    const uint64_t groups = ((uint64_t)(blocks ? (L + 3) / 4 * 4 : L) * Sn + ExhaustiveGatherParams::kGroup - 1) /
+                            ExhaustiveGatherParams::kGroup;
+    ExhaustiveGatherParams p{};
+    p.chains = split_chains(ctx, (uint64_t)cdiv(Vx, kKV) * cdiv(Vy, 8 * kWY) * cdiv(Vz, 4 * kWZ),
+                            busy_warps(in.voxel_res), groups,
+                            resident_ctas(wp.smem, kExhaustiveCtasPerSm), 3.2, (uint64_t)Vx * Vy * Vz);
+    float* rows = nullptr;
+    FBP_TRY(gather_scratch(ctx, npairs * pitch * sizeof(float), &p.chains, (uint64_t)Vx * Vy * Vz, stream, &rows,
+                           &p.chain_sums));
     PrepTables tables{};
     FBP_TRY(table_buffers(ctx, in, laser_xyz, sensor_xyz, true, stream, &tables));
-    FBP_TRY(prepare_gather(ctx, dtype, PrepRows{cube, static_cast<float*>(rows), npairs, T, pitch, 0}, tables, stream));
+    FBP_TRY(prepare_gather(ctx, dtype, PrepRows{cube, rows, npairs, T, pitch, 0}, tables, stream));
 
-    ExhaustiveGatherParams p{};
     p.lscan = tables.lasers;
     p.sscan = tables.sensors;
     p.xs = tables.axes;
@@ -459,21 +467,13 @@ fbp_status launch_exhaustive(fbp_context* ctx, const fbp_recon_info& in, const v
     p.zs = p.ys + Vz;
     p.volume = volume;
     p.status = ctx->status_dev;
-    p.rows = static_cast<const float*>(rows);
+    p.rows = rows;
     p.Vx = Vx; p.Vy = Vy; p.Vz = Vz; p.L = L; p.S = Sn; p.T = T;
     p.t0 = in.time_offset;
     p.dt = in.time_step;
     p.row_pitch = pitch;
     p.slot_w = slot_w;
     p.ch = wp.ch;
-    // Laser blocks of 4 where padding the lasers to whole blocks costs no more
-    // than a SPAD distance per pair would (about 8 of 21 issue cycles).
-    const bool blocks = wp.ch % 4 == 0 && (L + 3) / 4 * 4 * 3 <= L * 4;
-    const uint64_t groups = ((uint64_t)(blocks ? (L + 3) / 4 * 4 : L) * Sn + ExhaustiveGatherParams::kGroup - 1) /
-                            ExhaustiveGatherParams::kGroup;
-    p.chains = split_chains(ctx, (uint64_t)cdiv(Vx, kKV) * cdiv(Vy, 8 * kWY) * cdiv(Vz, 4 * kWZ),
-                            busy_warps(in.voxel_res), groups,
-                            resident_ctas(wp.smem, kExhaustiveCtasPerSm), 3.2, (uint64_t)Vx * Vy * Vz);
     p.exact_weights = ctx->weight_mode == FBP_WEIGHTS_REFERENCE;
     dim3 grid(cdiv(Vx, kKV), cdiv(Vy, 8 * kWY), cdiv(Vz, 4 * kWZ));
     const bool bounce = in.discard_first_last_bounces == 0;

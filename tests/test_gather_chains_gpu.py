@@ -153,6 +153,7 @@ def test_captured_chains_outlive_a_call_that_needs_more(own_ctx, cuda):
     ctx = own_ctx
     first = _capture(cuda, 32, 512, (16, 16, 170), 3)
     more = _capture(cuda, 20, 256, (64, 64, 72), 4)
+    ctx.backproject_confocal(*_capture(cuda, 32, 2048, (256, 256, 256), 5))  # rows without room for sums behind them
     want = ctx.backproject_confocal(*first)
     out = torch.empty_like(want)
     graph = torch.cuda.CUDAGraph()
