@@ -227,13 +227,18 @@ __global__ void __launch_bounds__(128, 7) log_filter_stream_kernel(const float* 
     f32x2_t w[3 * H * H + 1];
 #pragma unroll
     for (int i = 0; i <= 3 * H * H; ++i) w[i] = taps.w2[i];
-    // This thread's samples of a plane (borders clamped).
+    // This thread's samples of a plane (borders clamped).  Samples that only
+    // outputs beyond the volume would use are left out: lanes that copy one
+    // clamped address into many places take a pass each.
+    constexpr uint32_t kNone = 0xFFFFFFFFu;
     uint32_t oa[PER], ob[PER];
 #pragma unroll
     for (int u = 0; u < PER; ++u) {
-        const int e = min(tid + u * NT, NE - 1), lx = e % EX, gy = min(max(y0 + e / EX - H, 0), (int)ny - 1);
-        oa[u] = (uint32_t)gy * nx + min(max(x0 + lx - H, 0), (int)nx - 1);
-        ob[u] = (uint32_t)gy * nx + min(max(x0 + lx + HX - H, 0), (int)nx - 1);
+        const int e = tid + u * NT, gx = x0 + e % EX - H, gy = y0 + e / EX - H;
+        const uint32_t row = (uint32_t)min(max(gy, 0), (int)ny - 1) * nx;
+        const bool used = e < NE && gy < (int)ny + H;
+        oa[u] = used && gx < (int)nx + H ? row + min(max(gx, 0), (int)nx - 1) : kNone;
+        ob[u] = used && gx + HX < (int)nx + H ? row + min(max(gx + HX, 0), (int)nx - 1) : kNone;
     }
     const size_t plane = (size_t)nx * ny;
     const int planes = z1 - z0 + 2 * H;
@@ -241,12 +246,11 @@ __global__ void __launch_bounds__(128, 7) log_filter_stream_kernel(const float* 
         if (pl < planes) {
             const float* src = in + (size_t)min(max(z0 + pl - H, 0), (int)nz - 1) * plane;
 #pragma unroll
-            for (int u = 0; u < PER; ++u)
-                if (tid + u * NT < NE) {
-                    float* dst = reinterpret_cast<float*>(&tile[pl % RING][0][0] + tid + u * NT);
-                    copy_async4(dst, src + oa[u]);
-                    copy_async4(dst + 1, src + ob[u]);
-                }
+            for (int u = 0; u < PER; ++u) {
+                float* dst = reinterpret_cast<float*>(&tile[pl % RING][0][0] + tid + u * NT);
+                if (oa[u] != kNone) copy_async4(dst, src + oa[u]);
+                if (ob[u] != kNone) copy_async4(dst + 1, src + ob[u]);
+            }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -457,16 +461,19 @@ static fbp_status log_h(fbp_context* ctx, const float* in, float* out, uint32_t 
             }
             if (radial) {
                 // Planes per CTA: the fewest plane steps on the busiest SM
-                // (seven CTAs resident; two steps' worth of set-up).
+                // (seven CTAs resident; two steps' worth of set-up), where
+                // fewer than five CTAs take as long as five (a step's latency):
+                // K = 3 at 128^3 7.8 us so, 12.1 by the steps alone.
                 uint32_t tz = 8;
                 uint64_t least = ~0ull;
                 const uint64_t columns = (uint64_t)cdiv(nx, kLogTX) * cdiv(ny, kLogTY);
                 for (uint32_t c = 8; c <= 256; c *= 2) {
-                    const uint64_t ctas = columns * cdiv(nz, c), rounds = cdiv(ctas, (uint64_t)ctx->sm_count);
-                    const uint64_t steps = rounds * (std::min(c, nz) + 2 * H + 2);
+                    const uint32_t slabs = cdiv(nz, c), planes = cdiv(nz, slabs);
+                    const uint64_t rounds = cdiv(columns * slabs, (uint64_t)ctx->sm_count);
+                    const uint64_t steps = std::max<uint64_t>(rounds, 5) * (planes + 2 * H + 2);
                     if (steps < least) {
                         least = steps;
-                        tz = c;
+                        tz = planes;
                     }
                 }
                 dim3 grid(cdiv(nx, kLogTX), cdiv(ny, kLogTY), cdiv(nz, tz));
