@@ -105,12 +105,13 @@ __global__ void __launch_bounds__(DepthTileParams::kThreads, YONLY ? 3 : 2) dept
     const float lx = p.xyz[3 * (size_t)c], ly = p.xyz[3 * (size_t)c + 1], lz = p.xyz[3 * (size_t)c + 2];
     float box[6] = {INFINITY, -INFINITY, INFINITY, -INFINITY, INFINITY, -INFINITY};
     bool finite = true;
-    // (0 * depth is NaN in x and z where the depth is not finite.)
+    // YONLY: x and z are the scan point's at every depth; 0 * depth, NaN where the
+    // depth is not finite, is put into y (any NaN makes the path one).
     auto point = [&](int k, float& x, float& y, float& z) {
         const float df = s_df[k];
-        x = fma_rn(p.nx, df, lx);
+        x = YONLY ? lx : fma_rn(p.nx, df, lx);
         y = YONLY && !isfinite(df) ? NAN : fma_rn(p.ny, df, ly);
-        z = fma_rn(p.nz, df, lz);
+        z = YONLY ? lz : fma_rn(p.nz, df, lz);
     };
     for (int k = 0; k < KV; ++k) {
         float x, y, z;
