@@ -251,9 +251,8 @@ __global__ void fold_chains_kernel(const float* __restrict__ sums, uint32_t chai
         float sum = 0.f, comp = 0.f;
 #pragma unroll 4
         for (uint32_t c = 0; c < chains; ++c) {
-            const float s = sums[2 * c * n + i], e = -sums[(2 * c + 1) * n + i];
-            kahan_add(s, sum, comp);
-            kahan_add(e, sum, comp);
+            const float s = sums[2 * c * n + i], e = sums[(2 * c + 1) * n + i];
+            kahan_fold(s, e, sum, comp);
         }
         out[i] = sum;
     }

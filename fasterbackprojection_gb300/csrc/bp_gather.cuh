@@ -643,8 +643,7 @@ __device__ __forceinline__ void confocal_tile(const ConfocalGatherParams& p, uin
                 for (int k = 0; k < KV; ++k) {
                     float* t = totals + ((size_t)blockIdx.x * KV + k) * (2 * NT) + tid;
                     float sum = chain ? t[0] : 0.f, comp = chain ? t[NT] : 0.f;
-                    kahan_add(s_kahan[(2 * k) * NT + tid], sum, comp);
-                    kahan_add(-s_kahan[(2 * k + 1) * NT + tid], sum, comp);
+                    kahan_fold(s_kahan[(2 * k) * NT + tid], s_kahan[(2 * k + 1) * NT + tid], sum, comp);
                     t[0] = sum;
                     t[NT] = comp;
                     s_kahan[(2 * k) * NT + tid] = s_kahan[(2 * k + 1) * NT + tid] = 0.f;

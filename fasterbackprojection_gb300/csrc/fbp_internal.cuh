@@ -208,6 +208,12 @@ __device__ __forceinline__ void kahan_add(float part, float& sum, float& comp) {
     comp = sub_rn(sub_rn(t, sum), y);
     sum = t;
 }
+// A part's compensated sum into another (an infinite one has no compensation:
+// its own is NaN).
+__device__ __forceinline__ void kahan_fold(float part, float part_comp, float& sum, float& comp) {
+    kahan_add(part, sum, comp);
+    if (isfinite(part)) kahan_add(-part_comp, sum, comp);
+}
 // a + p (round to nearest) where x < y, else a unchanged: one compare and a
 // predicated add.
 __device__ __forceinline__ float add_rn_if_lt(float a, float p, float x, float y) {
