@@ -41,17 +41,23 @@ struct FilterTaps {
 // are zero-padded to a multiple of 2Q (zero terms), and S is preceded by F
 // zero slots (3Q <= F < 4Q, making S-index + F of every window start a
 // multiple of Q) so the last, unused window loads stay in bounds.
-// Rows of S are 8 floats, 12 apart, so the 16-byte loads of 8 consecutive
-// threads (8 consecutive rows) fall in 8 different bank groups and every load
-// of a thread is an immediate offset from its first row (swapping the halves of
-// rows 8 floats apart cost 12 integer instructions per bin).
-constexpr int kFilterQ = 8, kFilterRow = 12;
+// Rows of S are 8 floats, ROW apart.  ROW = 12: the 16-byte loads of 8
+// consecutive threads (8 consecutive rows) fall in 8 different bank groups and
+// every load of a thread is an immediate offset from its first row.  ROW = 8, two
+// thirds of the shared memory, for long series: the halves of row k trade places
+// when bit 2 of k is set, which keeps the bank groups apart and costs 12
+// integer instructions per bin.
+constexpr int kFilterQ = 8, kRowPadded = 12, kRowDense = 8;
 
-__device__ __forceinline__ int srow_addr(int k, int half) { return k * kFilterRow + half * 4; }
+template <int ROW>
+__device__ __forceinline__ int srow_addr(int k, int half) {
+    return ROW == kRowDense ? (8 * k + (k & 4)) ^ (4 * half) : k * ROW + 4 * half;
+}
 
+template <int ROW>
 __device__ __forceinline__ void srow_load(const float* sh, int k, float (&v)[kFilterQ]) {
-    const float4 a = *reinterpret_cast<const float4*>(sh + srow_addr(k, 0));
-    const float4 b = *reinterpret_cast<const float4*>(sh + srow_addr(k, 1));
+    const float4 a = *reinterpret_cast<const float4*>(sh + srow_addr<ROW>(k, 0));
+    const float4 b = *reinterpret_cast<const float4*>(sh + srow_addr<ROW>(k, 1));
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
     v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
@@ -87,11 +93,14 @@ __device__ __forceinline__ void filter_block_shared(const float* s_taps, int J, 
 // series' samples before this one is filtered.
 // 65536 x 1024: 371 -> 298 us (FMA pipe 69 %, issue
 // 85 %).
-constexpr int kFilterThreads = 128, kPrefetch = 3;
+// Registers: 1024 threads to an SM, but NJ == 0 with 128 threads as many as it
+// likes (at 64 a thread, 4096 x 4096 with 30-bin waves takes 238 us for 228).
+constexpr int kPrefetch = 3;
+constexpr int filter_ctas(int nj, int nt) { return nj == 0 && nt == 128 ? 1 : 1024 / nt; }
 constexpr int filter_taps(int nj) { return nj > 0 ? 2 * kFilterQ * nj : kMaxTaps; }
 
-template <int NJ, int nt>
-__global__ void __launch_bounds__(nt, 1024 / nt) filter_h_kernel(float* __restrict__ data, uint64_t nseries, uint32_t T, int n,
+template <int NJ, int nt, int ROW>
+__global__ void __launch_bounds__(nt, filter_ctas(NJ, nt)) filter_h_kernel(float* __restrict__ data, uint64_t nseries, uint32_t T, int n,
                                                        int R, int pad, int edge, int F, int ntp, int rows,
                                                        const __grid_constant__ FilterTaps<filter_taps(NJ)> taps) {
     constexpr int Q = kFilterQ;
@@ -124,7 +133,7 @@ __global__ void __launch_bounds__(nt, 1024 / nt) filter_h_kernel(float* __restri
             kept |= (uint32_t)keep << (4 * u + b);
         }
     auto store_half = [&](int g, const float (&v)[4]) {
-        *reinterpret_cast<float4*>(sser + srow_addr(g >> 1, g & 1)) = make_float4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<float4*>(sser + srow_addr<ROW>(g >> 1, g & 1)) = make_float4(v[0], v[1], v[2], v[3]);
     };
     float pre[kPrefetch][4];
     auto prefetch = [&](const float* h) {
@@ -161,8 +170,8 @@ __global__ void __launch_bounds__(nt, 1024 / nt) filter_h_kernel(float* __restri
             // b = b0 + F (a multiple of Q), window of block J: slots b - J - Q .. b - J + Q.
             const int kb = (t0 + pad + 2 * R + F) >> 3;  // row of slot b
             float A[Q], B[Q], acc[Q];
-            srow_load(sser, kb - 1, A);
-            srow_load(sser, kb, B);
+            srow_load<ROW>(sser, kb - 1, A);
+            srow_load<ROW>(sser, kb, B);
 #pragma unroll
             for (int q = 0; q < Q; ++q) acc[q] = 0.f;
             if constexpr (NJ > 0) {
@@ -170,17 +179,17 @@ __global__ void __launch_bounds__(nt, 1024 / nt) filter_h_kernel(float* __restri
                 for (int jj = 0; jj < NJ; ++jj) {
                     const int k = kb - 2 * jj;  // kb - J / Q with J = 2Q jj
                     filter_block(taps.w + 2 * Q * jj, A, B, acc);
-                    srow_load(sser, k - 2, B);  // low window of block J + Q
+                    srow_load<ROW>(sser, k - 2, B);  // low window of block J + Q
                     filter_block(taps.w + 2 * Q * jj + Q, B, A, acc);
-                    srow_load(sser, k - 3, A);  // low window of block J + 2Q
+                    srow_load<ROW>(sser, k - 3, A);  // low window of block J + 2Q
                 }
             } else {
                 for (int J = 0; J < ntp; J += 2 * Q) {
                     const int k = kb - (J >> 3);
                     filter_block_shared(s_taps, J, A, B, acc);
-                    srow_load(sser, k - 2, B);  // low window of block J + Q
+                    srow_load<ROW>(sser, k - 2, B);  // low window of block J + Q
                     filter_block_shared(s_taps, J + Q, B, A, acc);
-                    srow_load(sser, k - 3, A);  // low window of block J + 2Q
+                    srow_load<ROW>(sser, k - 3, A);  // low window of block J + 2Q
                 }
             }
 #pragma unroll
@@ -250,30 +259,47 @@ fbp_status filter_h_device(fbp_context* ctx, float* data, uint64_t nseries, uint
     const int F = 3 * Q + (Q - (pad + 2 * R + 3 * Q) % Q) % Q;
     // Highest slot read: t0 + pad + 2R + F + Q - 1 with t0 <= T - 1 (< E + F + Q).
     const int rows = (n + 2 * R + F + Q) / Q + 1;
-    const size_t smem = ((size_t)ntp + (size_t)kFilterRow * rows) * sizeof(float);
-    if (smem > (size_t)ctx->smem_optin) return set_error(FBP_ERR_UNSUPPORTED, "filter_H: series too long for one CTA");
+    auto smem_of = [&](int row) { return ((size_t)ntp + (size_t)row * rows) * sizeof(float); };
+    if (smem_of(kRowDense) > (size_t)ctx->smem_optin)
+        return set_error(FBP_ERR_UNSUPPORTED, "filter_H: series too long for one CTA");
     taps.resize((size_t)ntp, 0.f);
-    auto launch = [&](auto nj, auto nt) -> fbp_status {
-        constexpr int NJ = decltype(nj)::value, threads = decltype(nt)::value;
-        auto kernel = filter_h_kernel<NJ, threads>;
+    auto fit = [&](int row) { return kSmSharedBytes / (smem_of(row) + kCtaReservedShared); };  // CTAs to an SM, by shared memory
+    auto launch = [&](auto nj, auto nt, auto row) -> fbp_status {
+        constexpr int NJ = decltype(nj)::value, threads = decltype(nt)::value, ROW = decltype(row)::value;
+        auto kernel = filter_h_kernel<NJ, threads, ROW>;
+        const size_t smem = smem_of(ROW);
         FilterTaps<filter_taps(NJ)> tp;
         std::copy(taps.begin(), taps.end(), tp.w);
         FBP_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         // One CTA per resident slot (64 registers a thread), or twice as many
-        // where that leaves each only a few series.
-        const size_t fit = std::min<size_t>(std::min<size_t>(32, 1024 / threads), kSmSharedBytes / (smem + kCtaReservedShared));
-        const uint64_t slots = (uint64_t)ctx->sm_count * std::max<size_t>(1, fit);
-        const unsigned blocks = (unsigned)std::min<uint64_t>(nseries, nseries < 8 * slots ? 2 * slots : slots);
-        kernel<<<blocks, threads, smem, stream>>>(data, nseries, T, n, R, pad, border == FBP_BORDER_EDGE, F, ntp, rows, tp);
+        // where that leaves each only a few series; long series, whose setup is
+        // nothing beside them, 16 to an SM.
+        const uint64_t slots = (uint64_t)ctx->sm_count * std::max<size_t>(1, std::min<size_t>(std::min<size_t>(32, 1024 / threads), fit(ROW)));
+        const uint64_t most = ROW == kRowDense ? (uint64_t)ctx->sm_count * 16 : nseries < 8 * slots ? 2 * slots : slots;
+        kernel<<<(unsigned)std::min<uint64_t>(nseries, most), threads, smem, stream>>>(
+            data, nseries, T, n, R, pad, border == FBP_BORDER_EDGE, F, ntp, rows, tp);
         FBP_CHECK_LAUNCH(ctx, "filter_h_kernel");
         return FBP_OK;
     };
     // Threads for one pass over a series (8 bins each): 65536 x 128 with 128
-    // threads 65.7 us, with 32 38.7 us.
+    // threads 65.7 us, with 32 38.7 us.  Padded rows while six series fit an SM
+    // (to some 6,000 bins); then dense ones (4096 x 10000, 4-bin waves: 243 us
+    // padded, 192 dense), from where four fit (some 11,000 bins) with 256 threads
+    // (4096 x 20000, 10-bin waves: 1045 us padded, 722 dense with 128 threads,
+    // 575 with 256).  Waves of more than 20 bins (NJ == 0) have borders and taps
+    // that outweigh the bins of a short series: never fewer than 128 threads
+    // (2000 x 128, 150-bin waves: 63 us with 32, 54 with 128).
     auto go = [&](auto nj) -> fbp_status {
-        if (T <= 32 * Q) return launch(nj, std::integral_constant<int, 32>{});
-        if (T <= 64 * Q) return launch(nj, std::integral_constant<int, 64>{});
-        return launch(nj, std::integral_constant<int, kFilterThreads>{});
+        constexpr int NJ = decltype(nj)::value;
+        constexpr std::integral_constant<int, kRowPadded> padded{};
+        constexpr std::integral_constant<int, kRowDense> dense{};
+        if (fit(kRowDense) <= 4) return launch(nj, std::integral_constant<int, 256>{}, dense);
+        if constexpr (NJ > 0) {
+            if (T <= 32 * Q) return launch(nj, std::integral_constant<int, 32>{}, padded);
+            if (T <= 64 * Q) return launch(nj, std::integral_constant<int, 64>{}, padded);
+            if (fit(kRowPadded) >= 6) return launch(nj, std::integral_constant<int, 128>{}, padded);
+        }
+        return launch(nj, std::integral_constant<int, 128>{}, dense);
     };
     // Unrolled forms for 2 .. 12 blocks of 16 taps (wavelengths of about 2
     // to 20 bins; 10 bins, the reference's default, gives 107 taps = 7 blocks).
