@@ -37,7 +37,7 @@ struct ExhaustiveGatherParams {
     // bounces), the SPAD's x differences to the tile's kv columns, the window's
     // source and length; two words per group.
     static constexpr int kGroup = 32;
-    static constexpr int kWindowBufs = 3;  // (two: 5 % slower)
+    static constexpr int kWindowBufs = 3;  // two (5 % slower) where a window leaves no room for three
     static constexpr int kPlanBufs = 8;
     __host__ __device__ static constexpr size_t meta_bytes(int kv) {
         return 128 +
@@ -71,13 +71,14 @@ enum { EX_T0ZERO = 0, EX_FAST = 1, EX_EXACT = 2 };
 // pair of triples takes (8^2 x 32^2 x 1024 -> 128^3: 43.4 ms).  Reciprocals of
 // their own for half or all of the weights (fewer products, more MUFU work)
 // take the same time; blocks of 1, 2 and 8 lasers 78, 58 and 46 ms.
-template <int KV, int WY, int WZ, int MODE, bool BOUNCE, bool CLAMP, int LB>
+template <int KV, int WY, int WZ, int MODE, bool BOUNCE, bool CLAMP, int LB, uint32_t NB = ExhaustiveGatherParams::kWindowBufs>
 __global__ void __launch_bounds__(32 * WY * WZ, 2)
 exhaustive_gather_kernel(ExhaustiveGatherParams p) {
     static_assert(KV % 8 == 0, "voxels per thread in packed pairs, four to a weight group");
     using P = ExhaustiveGatherParams;
     constexpr int NT = 32 * WY * WZ, NW = WY * WZ, ALIGN = 4;
-    constexpr uint32_t GRP = P::kGroup, NB = P::kWindowBufs, MB = P::kPlanBufs;
+    constexpr uint32_t GRP = P::kGroup, MB = P::kPlanBufs;
+    static_assert(NB <= P::kWindowBufs, "the barriers fit in front of the plans");
     constexpr int TY = 8 * WY, TZ = 4 * WZ;
     const uint32_t CH = p.ch;
 
@@ -400,9 +401,9 @@ namespace {
 constexpr int kKV = 8, kWY = 2, kWZ = 4;
 constexpr int kExhaustiveCtasPerSm = 2;  // 256 threads of up to 128 registers
 
-template <int MODE, bool BOUNCE, bool CLAMP, int LB>
+template <int MODE, bool BOUNCE, bool CLAMP, int LB, uint32_t NB = ExhaustiveGatherParams::kWindowBufs>
 fbp_status go_exhaustive(fbp_context* ctx, ExhaustiveGatherParams p, dim3 grid, size_t smem, cudaStream_t stream) {
-    auto kernel = exhaustive_gather_kernel<kKV, kWY, kWZ, MODE, BOUNCE, CLAMP, LB>;
+    auto kernel = exhaustive_gather_kernel<kKV, kWY, kWZ, MODE, BOUNCE, CLAMP, LB, NB>;
     FBP_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const uint64_t n = (uint64_t)p.Vx * p.Vy * p.Vz;
     grid.x *= p.chains;
@@ -430,6 +431,18 @@ fbp_status dispatch_exhaustive(fbp_context* ctx, const ExhaustiveGatherParams& p
     return go_exhaustive<EX_FAST, LB>(ctx, p, grid, smem, s, bounce, capped);
 }
 
+// Windows with room for two only (one pair to a stage).  EX_EXACT's results are
+// those of the other two where no path is negative.
+fbp_status dispatch_widest(fbp_context* ctx, const ExhaustiveGatherParams& p, dim3 grid, size_t smem, cudaStream_t s,
+                           bool bounce, bool capped) {
+    if (bounce) {
+        if (capped) return go_exhaustive<EX_EXACT, true, true, 1, 2>(ctx, p, grid, smem, s);
+        return go_exhaustive<EX_EXACT, true, false, 1, 2>(ctx, p, grid, smem, s);
+    }
+    if (capped) return go_exhaustive<EX_EXACT, false, true, 1, 2>(ctx, p, grid, smem, s);
+    return go_exhaustive<EX_EXACT, false, false, 1, 2>(ctx, p, grid, smem, s);
+}
+
 fbp_status launch_exhaustive(fbp_context* ctx, const fbp_recon_info& in, const void* cube, int dtype, const float* laser_xyz,
                              const float* sensor_xyz, float* volume, cudaStream_t stream) {
     const uint32_t L = in.num_laser_targets, Sn = in.num_sensor_targets, T = in.num_time_bins;
@@ -439,14 +452,22 @@ fbp_status launch_exhaustive(fbp_context* ctx, const fbp_recon_info& in, const v
     const double ey = (double)std::min<uint32_t>(4 * kWZ, Vz) * std::fabs(in.voxel_size[1]);
     const double ez = (double)std::min<uint32_t>(8 * kWY, Vy) * std::fabs(in.voxel_size[2]);
     WindowPlan wp;
-    FBP_TRY(plan_window(ctx, ex, ey, ez, in.time_step, T, ALIGN, sizeof(float), ExhaustiveGatherParams::meta_bytes(kKV),
-                        &wp, "fbp_backproject_exhaustive", 0.0, kExhaustiveCtasPerSm, ExhaustiveGatherParams::kWindowBufs));
+    auto plan = [&](int bufs) {
+        return plan_window(ctx, ex, ey, ez, in.time_step, T, ALIGN, sizeof(float), ExhaustiveGatherParams::meta_bytes(kKV),
+                           &wp, "fbp_backproject_exhaustive", 0.0, kExhaustiveCtasPerSm, bufs);
+    };
+    // Three windows to a CTA up to some 17,700 bins, two up to 26,600.
+    const bool widest = plan(ExhaustiveGatherParams::kWindowBufs) == FBP_ERR_UNSUPPORTED;
+    if (widest) {
+        clear_error();
+        FBP_TRY(plan(2));
+    }
     const uint32_t slot_w = wp.slot_w, pitch = wp.pitch;
     const uint64_t npairs = (uint64_t)L * Sn;
 
     // Laser blocks of 4 where padding the lasers to whole blocks costs no more
     // than a SPAD distance per pair would (about 8 of 21 issue cycles).
-    const bool blocks = wp.ch % 4 == 0 && (L + 3) / 4 * 4 * 3 <= L * 4;
+    const bool blocks = !widest && wp.ch % 4 == 0 && (L + 3) / 4 * 4 * 3 <= L * 4;
     const uint64_t groups = ((uint64_t)(blocks ? (L + 3) / 4 * 4 : L) * Sn + ExhaustiveGatherParams::kGroup - 1) /
                             ExhaustiveGatherParams::kGroup;
     ExhaustiveGatherParams p{};
@@ -477,6 +498,7 @@ fbp_status launch_exhaustive(fbp_context* ctx, const fbp_recon_info& in, const v
     p.exact_weights = ctx->weight_mode == FBP_WEIGHTS_REFERENCE;
     dim3 grid(cdiv(Vx, kKV), cdiv(Vy, 8 * kWY), cdiv(Vz, 4 * kWZ));
     const bool bounce = in.discard_first_last_bounces == 0;
+    if (widest) return dispatch_widest(ctx, p, grid, wp.smem, stream, bounce, wp.capped);
     if (blocks) return dispatch_exhaustive<4>(ctx, p, grid, wp.smem, stream, bounce, in.time_offset, wp.capped);
     return dispatch_exhaustive<1>(ctx, p, grid, wp.smem, stream, bounce, in.time_offset, wp.capped);
 }
