@@ -49,9 +49,8 @@ struct fbp_batch {
     int dtype = FBP_F32;
     int cfg = 0;
     // Device buffers owned by the batch.
-    void* rows = nullptr;
+    char* rows = nullptr;
     size_t rows_bytes = 0;
-    std::vector<size_t> rows_off;       // per capture, bytes
     float4* scan = nullptr;             // all scan tables back to back
     float* axes = nullptr;              // all axis tables back to back
     std::vector<size_t> scan_off, axes_off;
@@ -62,7 +61,8 @@ struct fbp_batch {
     float* d_totals = nullptr;
     size_t totals_cap = 0;  // floats
     std::vector<fbp::ConfocalGatherParams> params;
-    std::vector<fbp::BatchGroup> groups;
+    std::vector<fbp::BatchGroup> groups;  // empty: no plan (`planned` says why)
+    fbp_status planned = FBP_OK;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
     uint64_t graph_launches = 0;  // kernels one replay launches
@@ -106,17 +106,23 @@ fbp_status rows_any(fbp_context* ctx, int dtype, const fbp_capture_desc& c, uint
                           PrepTables{}, s);
 }
 
-// (Re)plan windows, parameters and work items for tile configuration `cfg`.
-fbp_status plan_config(fbp_batch* b, int cfg, cudaStream_t s) {
+// Windows, parameters and work items of a tile configuration.
+struct BatchPlan {
+    std::vector<ConfocalGatherParams> params;  // (without their rows)
+    std::vector<BatchGroup> groups;            // (without their buffers)
+    std::vector<size_t> rows_off;              // per capture, bytes
+    size_t rows_bytes = 0, total_items = 0;
+    std::vector<std::vector<BatchItem>> items;  // per group
+};
+
+// Works the plan out; the batch stays as it is.
+fbp_status make_plan(const fbp_batch* b, int cfg, BatchPlan* plan) {
     const TileCfg tc = kTileCfgs[cfg];
     const int align = (int)(16 / kRowBytes);
     const size_t meta = ConfocalGatherParams::meta_bytes(tc.kv) + kahan_smem_bytes(tc.kv, 32 * tc.wy * tc.wz) + 16;
     const uint32_t n = (uint32_t)b->caps.size();
-    b->params.assign(n, ConfocalGatherParams{});
-    b->groups.clear();
-    std::vector<uint32_t> pitches(n);
-    size_t rows_total = 0;
-    std::vector<size_t> rows_off(n);
+    plan->params.assign(n, ConfocalGatherParams{});
+    plan->rows_off.resize(n);
     for (uint32_t i = 0; i < n; ++i) {
         const fbp_recon_info& in = b->caps[i].info;
         const double ex = (double)std::min<uint32_t>(tc.kv, in.voxel_res[0]) * std::fabs(in.voxel_size[0]);
@@ -131,10 +137,9 @@ fbp_status plan_config(fbp_batch* b, int cfg, cudaStream_t s) {
         if (wp.smem + kBatchStaticSmem > (size_t)b->ctx->smem_optin)
             FBP_TRY(plan_window(b->ctx, ex, ey, ez, in.time_step, in.num_time_bins, align, kRowBytes,
                                 meta + kBatchStaticSmem, &wp, "fbp_batch", 0.0, kGatherCtasPerSm, ConfocalGatherParams::kWindowBufs));
-        pitches[i] = wp.pitch;
-        rows_off[i] = rows_total;
-        rows_total += ((size_t)in.num_laser_targets * wp.pitch * kRowBytes + 255) & ~size_t(255);
-        ConfocalGatherParams& p = b->params[i];
+        plan->rows_off[i] = plan->rows_bytes;
+        plan->rows_bytes += ((size_t)in.num_laser_targets * wp.pitch * kRowBytes + 255) & ~size_t(255);
+        ConfocalGatherParams& p = plan->params[i];
         p.scan = b->scan + b->scan_off[i];
         p.xs = b->axes + b->axes_off[i];
         p.ys = p.xs + in.voxel_res[0];
@@ -169,11 +174,11 @@ fbp_status plan_config(fbp_batch* b, int cfg, cudaStream_t s) {
         FBP_TRY(prepare_any(probe, &occ));
         if (occ < 1) return set_error(FBP_ERR_UNSUPPORTED, "fbp_batch: a capture's tile does not fit on an SM");
         BatchGroup* g = nullptr;
-        for (auto& gg : b->groups)
+        for (auto& gg : plan->groups)
             if (gg.path == path && gg.bounce == bounce && gg.clamp == clamp && gg.occ == occ) g = &gg;
         if (!g) {
-            b->groups.push_back(BatchGroup{});
-            g = &b->groups.back();
+            plan->groups.push_back(BatchGroup{});
+            g = &plan->groups.back();
             g->path = path;
             g->bounce = bounce;
             g->clamp = clamp;
@@ -183,25 +188,16 @@ fbp_status plan_config(fbp_batch* b, int cfg, cudaStream_t s) {
         g->work += (double)in.num_laser_targets * in.voxel_res[0] * in.voxel_res[1] * in.voxel_res[2];
         g->smem = std::max(g->smem, wp.smem);
     }
-    if (b->groups.size() > (size_t)kMaxGroups)
+    if (plan->groups.size() > (size_t)kMaxGroups)
         return set_error(FBP_ERR_UNSUPPORTED, "fbp_batch: too many (variant, occupancy) groups");
     // Largest group first: it starts on every SM, the others backfill.
-    std::stable_sort(b->groups.begin(), b->groups.end(),
+    std::stable_sort(plan->groups.begin(), plan->groups.end(),
                      [](const BatchGroup& x, const BatchGroup& y) { return x.work > y.work; });
-    // Rows buffer (grow only).
-    if (rows_total > b->rows_bytes) {
-        if (b->rows) FBP_TRY_CUDA(cudaFree(b->rows));
-        b->rows = nullptr;
-        FBP_TRY_CUDA(cudaMalloc(&b->rows, rows_total));
-        b->rows_bytes = rows_total;
-    }
-    b->rows_off = rows_off;
-    for (uint32_t i = 0; i < n; ++i) b->params[i].rows = static_cast<char*>(b->rows) + rows_off[i];
     // Work items, largest captures first within each group.
-    size_t total_items = 0;
-    std::vector<std::vector<BatchItem>> per_group(b->groups.size());
-    for (size_t gi = 0; gi < b->groups.size(); ++gi) {
-        auto& g = b->groups[gi];
+    plan->items.resize(plan->groups.size());
+    for (size_t gi = 0; gi < plan->groups.size(); ++gi) {
+        auto& g = plan->groups[gi];
+        auto& items = plan->items[gi];
         std::vector<uint32_t> order = g.captures;
         std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) {
             return b->caps[x].info.num_laser_targets > b->caps[y].info.num_laser_targets;
@@ -212,65 +208,88 @@ fbp_status plan_config(fbp_batch* b, int cfg, cudaStream_t s) {
                            gz = cdiv(in.voxel_res[2], 4 * tc.wz);
             for (uint32_t z = 0; z < gz; ++z)
                 for (uint32_t y = 0; y < gy; ++y)
-                    for (uint32_t x = 0; x < gx; ++x) per_group[gi].push_back(BatchItem{c, x, y, z});
+                    for (uint32_t x = 0; x < gx; ++x) items.push_back(BatchItem{c, x, y, z});
         }
-        total_items += per_group[gi].size();
-    }
-    if (total_items > b->items_cap) {
-        if (b->d_items) FBP_TRY_CUDA(cudaFree(b->d_items));
-        b->d_items = nullptr;
-        FBP_TRY_CUDA(cudaMalloc(&b->d_items, total_items * sizeof(BatchItem)));
-        b->items_cap = total_items;
-    }
-    size_t off = 0;
-    for (size_t gi = 0; gi < b->groups.size(); ++gi) {
-        auto& g = b->groups[gi];
-        g.d_items = b->d_items + off;
-        g.nitems = (uint32_t)per_group[gi].size();
-        FBP_TRY_CUDA(cudaMemcpyAsync(g.d_items, per_group[gi].data(), g.nitems * sizeof(BatchItem),
-                                     cudaMemcpyHostToDevice, s));
-        off += g.nitems;
-    }
-    FBP_TRY_CUDA(cudaMemcpyAsync(b->d_params, b->params.data(), n * sizeof(ConfocalGatherParams),
-                                 cudaMemcpyHostToDevice, s));
-    // Resident CTAs of each group (outside any capture), capped by its items.
-    for (auto& g : b->groups) {
-        BatchLaunch l{b->d_params, g.d_items, g.nitems, nullptr, nullptr, g.smem, g.path, g.bounce, g.clamp, cfg,
+        g.nitems = (uint32_t)items.size();
+        plan->total_items += items.size();
+        // Resident CTAs of the group (outside any capture), capped by its items.
+        BatchLaunch l{b->d_params, nullptr, g.nitems, nullptr, nullptr, g.smem, g.path, g.bounce, g.clamp, cfg,
                       (size_t)b->ctx->smem_optin};
         int occ = 0;
         FBP_TRY(prepare_any(l, &occ));
         g.ctas = (int)std::min<uint64_t>((uint64_t)std::max(1, occ) * b->ctx->sm_count, g.nitems);
     }
+    return FBP_OK;
+}
+
+// Room for `want` elements in a buffer of the batch that only grows.
+template <typename T>
+fbp_status grow(T** buf, size_t* have, size_t want) {
+    if (want <= *have) return FBP_OK;
+    if (*buf) FBP_TRY_CUDA(cudaFree(*buf));
+    *buf = nullptr;
+    *have = 0;
+    void* p = nullptr;
+    FBP_TRY_CUDA(cudaMalloc(&p, want * sizeof(T)));
+    *buf = static_cast<T*>(p);
+    *have = want;
+    return FBP_OK;
+}
+
+// The plan's buffers and tables; the groups are the plan's from here on.
+fbp_status install_plan(fbp_batch* b, int cfg, BatchPlan& plan, cudaStream_t s) {
+    const TileCfg tc = kTileCfgs[cfg];
+    FBP_TRY(grow(&b->rows, &b->rows_bytes, plan.rows_bytes));
+    FBP_TRY(grow(&b->d_items, &b->items_cap, plan.total_items));
     // The chains' totals (cfg 0 only): a slice per resident CTA of every group.
     const size_t slice = cfg == 0 ? (size_t)2 * tc.kv * 32 * tc.wy * tc.wz : 0;
     size_t totals = 0;
-    for (const auto& g : b->groups) totals += slice * g.ctas;
-    if (totals > b->totals_cap) {
-        if (b->d_totals) FBP_TRY_CUDA(cudaFree(b->d_totals));
-        b->d_totals = nullptr;
-        b->totals_cap = 0;
-        FBP_TRY_CUDA(cudaMalloc(&b->d_totals, totals * sizeof(float)));
-        b->totals_cap = totals;
-    }
+    for (const auto& g : plan.groups) totals += slice * g.ctas;
+    FBP_TRY(grow(&b->d_totals, &b->totals_cap, totals));
+    for (size_t i = 0; i < plan.params.size(); ++i) plan.params[i].rows = b->rows + plan.rows_off[i];
+    size_t off = 0;
     totals = 0;
-    for (auto& g : b->groups) {
+    for (size_t gi = 0; gi < plan.groups.size(); ++gi) {
+        auto& g = plan.groups[gi];
+        g.d_items = b->d_items + off;
         g.d_totals = b->d_totals + totals;
+        FBP_TRY_CUDA(cudaMemcpyAsync(g.d_items, plan.items[gi].data(), g.nitems * sizeof(BatchItem),
+                                     cudaMemcpyHostToDevice, s));
+        off += g.nitems;
         totals += slice * g.ctas;
     }
+    FBP_TRY_CUDA(cudaMemcpyAsync(b->d_params, plan.params.data(), plan.params.size() * sizeof(ConfocalGatherParams),
+                                 cudaMemcpyHostToDevice, s));
     // Side streams and events for the groups after the first.
     if (!b->fork) FBP_TRY_CUDA(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
-    while (b->side.size() + 1 < b->groups.size()) {
-        cudaStream_t st = nullptr;
+    while (b->join.size() + 1 < plan.groups.size()) {
+        if (b->side.size() == b->join.size()) {
+            cudaStream_t st = nullptr;
+            FBP_TRY_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+            b->side.push_back(st);
+        }
         cudaEvent_t ev = nullptr;
-        FBP_TRY_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-        b->side.push_back(st);
         FBP_TRY_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
         b->join.push_back(ev);
     }
-    FBP_TRY_CUDA(cudaStreamSynchronize(s));  // host-side vectors above are temporaries
+    FBP_TRY_CUDA(cudaStreamSynchronize(s));  // the plan's host vectors are temporaries
+    b->params = std::move(plan.params);
+    b->groups = std::move(plan.groups);
     b->cfg = cfg;
-    drop_graph(b);
     return FBP_OK;
+}
+
+// (Re)plan for tile configuration `cfg`.  A configuration that cannot be planned
+// leaves the batch as it was.  One whose buffers cannot be had leaves it without a
+// plan (and without the graph, whose kernels use the old buffers), so that a run is
+// refused until another configuration is set.
+fbp_status plan_config(fbp_batch* b, int cfg, cudaStream_t s) {
+    BatchPlan plan;
+    FBP_TRY(make_plan(b, cfg, &plan));
+    drop_graph(b);
+    b->groups.clear();
+    b->planned = FBP_ERR_INTERNAL;  // (what an exception leaves)
+    return b->planned = install_plan(b, cfg, plan, s);
 }
 
 // The captured sequence: rows of every capture, counters, then one
@@ -395,6 +414,8 @@ extern "C" fbp_status fbp_batch_run(fbp_batch* b, int use_graph, void* stream) {
         if (!b) return set_error(FBP_ERR_INVALID_ARG, "fbp_batch_run: null batch");
         FBP_TRY(check_ctx(b->ctx));
         cudaStream_t s = (cudaStream_t)stream;
+        if (b->groups.empty())
+            return set_error(b->planned, "fbp_batch_run: the last tile configuration could not be set up; set one again");
         if (!use_graph) return enqueue_run(b, s);
         if (s == nullptr)
             return set_error(FBP_ERR_INVALID_ARG, "fbp_batch_run: graph replay needs a non-default stream");

@@ -368,7 +368,9 @@ fbp_status fbp_batch_run(fbp_batch* batch, int use_graph, void* stream);
 fbp_status fbp_batch_autotune(fbp_batch* batch, void* stream, int* chosen);
 /* Selects tile shape `config` (0..3) explicitly: 16 x 16 x 16, 8 x 16 x 16,
  * 8 x 32 x 16 or 4 x 32 x 16 voxels (x, y, depth); 0 is the single-capture
- * gather's tile. */
+ * gather's tile.  A shape that does not fit (FBP_ERR_UNSUPPORTED) leaves the
+ * batch as it was; one whose buffers cannot be had leaves it without a plan, and
+ * runs return that status until a shape is set. */
 fbp_status fbp_batch_set_config(fbp_batch* batch, int config, void* stream);
 fbp_status fbp_batch_destroy(fbp_batch* batch);
 
