@@ -93,14 +93,13 @@ __device__ __forceinline__ void filter_block_shared(const float* s_taps, int J, 
 // series' samples before this one is filtered.
 // 65536 x 1024: 371 -> 298 us (FMA pipe 69 %, issue
 // 85 %).
-// Registers: 1024 threads to an SM, but NJ == 0 with 128 threads as many as it
-// likes (at 64 a thread, 4096 x 4096 with 30-bin waves takes 238 us for 228).
-constexpr int kPrefetch = 3;
-constexpr int filter_ctas(int nj, int nt) { return nj == 0 && nt == 128 ? 1 : 1024 / nt; }
+// (With many taps, NJ == 0, the fill is a small part: nothing is kept or loaded
+// ahead.)
+constexpr int prefetch_rows(int nj) { return nj > 0 ? 3 : 0; }
 constexpr int filter_taps(int nj) { return nj > 0 ? 2 * kFilterQ * nj : kMaxTaps; }
 
 template <int NJ, int nt, int ROW>
-__global__ void __launch_bounds__(nt, filter_ctas(NJ, nt)) filter_h_kernel(float* __restrict__ data, uint64_t nseries, uint32_t T, int n,
+__global__ void __launch_bounds__(nt, 1024 / nt) filter_h_kernel(float* __restrict__ data, uint64_t nseries, uint32_t T, int n,
                                                        int R, int pad, int edge, int F, int ntp, int rows,
                                                        const __grid_constant__ FilterTaps<filter_taps(NJ)> taps) {
     constexpr int Q = kFilterQ;
@@ -123,7 +122,8 @@ __global__ void __launch_bounds__(nt, filter_ctas(NJ, nt)) filter_h_kernel(float
     };
     // The slots of this thread's first kPrefetch half rows (the same for every
     // series): half row g holds slots 4 g - F and on.
-    uint32_t from[kPrefetch][4], kept = 0;
+    constexpr int kPrefetch = prefetch_rows(NJ);
+    uint32_t from[kPrefetch + 1][4], kept = 0;
 #pragma unroll
     for (int u = 0; u < kPrefetch; ++u)
 #pragma unroll
@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(nt, filter_ctas(NJ, nt)) filter_h_kernel(float
     auto store_half = [&](int g, const float (&v)[4]) {
         *reinterpret_cast<float4*>(sser + srow_addr<ROW>(g >> 1, g & 1)) = make_float4(v[0], v[1], v[2], v[3]);
     };
-    float pre[kPrefetch][4];
+    float pre[kPrefetch + 1][4];
     auto prefetch = [&](const float* h) {
 #pragma unroll
         for (int u = 0; u < kPrefetch; ++u)
@@ -283,21 +283,26 @@ fbp_status filter_h_device(fbp_context* ctx, float* data, uint64_t nseries, uint
     };
     // Threads for one pass over a series (8 bins each): 65536 x 128 with 128
     // threads 65.7 us, with 32 38.7 us.  Padded rows while six series fit an SM
-    // (to some 6,000 bins); then dense ones (4096 x 10000, 4-bin waves: 243 us
-    // padded, 192 dense), from where four fit (some 11,000 bins) with 256 threads
-    // (4096 x 20000, 10-bin waves: 1045 us padded, 722 dense with 128 threads,
-    // 575 with 256).  Waves of more than 20 bins (NJ == 0) have borders and taps
-    // that outweigh the bins of a short series: never fewer than 128 threads
-    // (2000 x 128, 150-bin waves: 63 us with 32, 54 with 128).
+    // (some 6,000 bins), or four (9,000) with taps enough to pay for it; then dense
+    // ones (1000 x 8192: 4-bin waves 40 us padded and 37 dense, 10-bin waves 50 and
+    // 55; 4096 x 10000, 4-bin waves 243 and 193), from where four of them fit (some
+    // 11,000 bins) with 256 threads (4096 x 20000, 10-bin waves: 1043 us padded,
+    // 583 so).  Waves of more than 20 bins (NJ == 0) have borders and taps that
+    // outweigh the bins of a short series: never fewer than 128 threads (2000 x
+    // 128, 150-bin waves: 63 us with 32, 53 with 128).
     auto go = [&](auto nj) -> fbp_status {
         constexpr int NJ = decltype(nj)::value;
         constexpr std::integral_constant<int, kRowPadded> padded{};
         constexpr std::integral_constant<int, kRowDense> dense{};
-        if (fit(kRowDense) <= 4) return launch(nj, std::integral_constant<int, 256>{}, dense);
+        if (fit(kRowDense) <= (NJ > 0 ? 4 : 2)) return launch(nj, std::integral_constant<int, 256>{}, dense);
         if constexpr (NJ > 0) {
-            if (T <= 32 * Q) return launch(nj, std::integral_constant<int, 32>{}, padded);
-            if (T <= 64 * Q) return launch(nj, std::integral_constant<int, 64>{}, padded);
-            if (fit(kRowPadded) >= 6) return launch(nj, std::integral_constant<int, 128>{}, padded);
+            // (few series: threads enough to load each in one go, too)
+            auto enough = [&](uint32_t nt) {
+                return T <= nt * Q && (nseries > 2ull * ctx->sm_count || 2 * (uint32_t)rows <= prefetch_rows(NJ) * nt);
+            };
+            if (enough(32)) return launch(nj, std::integral_constant<int, 32>{}, padded);
+            if (enough(64)) return launch(nj, std::integral_constant<int, 64>{}, padded);
+            if (fit(kRowPadded) >= (NJ >= 5 ? 4 : 6)) return launch(nj, std::integral_constant<int, 128>{}, padded);
         }
         return launch(nj, std::integral_constant<int, 128>{}, dense);
     };
