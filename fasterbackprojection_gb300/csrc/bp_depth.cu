@@ -529,13 +529,39 @@ __global__ void depth_rows_kernel(S* __restrict__ rows, const S* __restrict__ cu
     }
 }
 
+// Whether the tiles beat the row kernel for D planes.  Tiles always work on 16
+// planes and on whole 16 x 16 (or 256) scan points, so few planes of many scan
+// points are cheaper by rows, one thread per test point, which take about as
+// long for any number of points that fit the GPU at once.  Both in nanoseconds
+// per scan point walked, from measurements on 144^2 .. 240^2 points: rows 140
+// while they stay in the L2 and up to 215 from memory, for each 1536 points on
+// every SM; tiles 1.1 each with windows (1.5 for a tilted normal), 1.35, 1.65 or
+// 2.45 where whole rows leave room for 4, 2 or 1 scan points to a stage, as a few
+// planes far apart need.  Tiles against rows: 176^2 points, 512 bins, 2 planes 3.8
+// and 5.5 ms; 240^2, 512 bins, 2 planes 13.1 and 11.8 ms; 240^2, 2048 bins, 4
+// planes 30.3 and 14.0 ms.
+bool tiles_pay(const fbp_context* ctx, const fbp_recon_info& in, uint32_t D, size_t elem_bytes) {
+    using P = DepthTileParams;
+    const uint32_t L = in.num_laser_targets, T = in.num_time_bins;
+    const uint32_t side = (uint32_t)std::lround(std::sqrt((double)L));
+    const double tiles = (uint64_t)side * side == L ? (double)cdiv(side, 16) * cdiv(side, 16) : (double)cdiv(L, P::kThreads);
+    const bool yonly = in.wall_normal[0] == 0.f && in.wall_normal[2] == 0.f;
+    const bool plain = in.discard_first_last_bounces != 0 && in.time_offset == 0.f;
+    const uint32_t staged = P::kWindowFloats / 2 / (T + 8);  // whole rows to a stage
+    double tile = yonly ? (plain ? 1.1 : 1.2) : (plain ? 1.5 : 1.65);
+    if (D > 1 && T > 600) tile = (staged >= 4 ? 1.35 : staged >= 2 ? 1.65 : 2.45) * (yonly ? 1.0 : 1.3);
+    const double waves = std::ceil((double)L * D / (1536.0 * ctx->sm_count));
+    const double row = std::min(140.0 + 0.55e-6 * L * T * elem_bytes, 215.0) * (waves > 1.0 ? 1.2 * waves : 1.0);
+    return tiles * cdiv(D, P::kDepths) * tile * 152.0 / ctx->sm_count <= row;
+}
+
 template <typename S>
 fbp_status launch_depths(fbp_context* ctx, const fbp_recon_info& in, const void* cube, int layout,
                          const float* laser_xyz, const float* sensor_xyz, const double* depths, uint32_t D,
                          float* act, cudaStream_t stream) {
     const bool exhaustive = in.capture_system == FBP_EXHAUSTIVE;
     if (!exhaustive && in.num_time_bins <= DepthTileParams::kMaxBins && cdiv(D, DepthTileParams::kDepths) <= 65535 &&
-        workspace_ready(ctx, WS_CUBE_ROWS, DepthTileParams::row_bytes(in), stream)) {
+        tiles_pay(ctx, in, D, sizeof(S)) && workspace_ready(ctx, WS_CUBE_ROWS, DepthTileParams::row_bytes(in), stream)) {
         const fbp_status st = launch_depth_tiles(ctx, in, cube, dtype_of<S>(), layout, laser_xyz, depths, D, act, stream);
         if (st != FBP_ERR_OOM) return st;
         cudaGetLastError();  // no memory for FP32 rows: the kernel below needs the capture's own bytes

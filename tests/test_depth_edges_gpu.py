@@ -27,3 +27,31 @@ def test_a_non_finite_depth_stays_in_its_plane(ctx, cuda, side, flat, D, at, val
     assert want.any()
     for d in range(D):
         assert rel_l2(got[:, d], want[:, d]) < 1e-6, d
+
+
+@pytest.mark.parametrize("normal", [(0, -1, 0), (0.36, -0.8, 0.48)])
+def test_few_planes_of_many_points_go_by_rows(ctx, cuda, normal):
+    """Tiles work on 16 planes whatever their number: two planes of 240^2 scan points take the row
+    kernel, the bits of a capture with too many (zero) bins for tiles, sixteen the tiles."""
+    import torch
+
+    from fasterbackprojection_gb300 import make_info
+
+    side, T, most = 240, 64, 3700
+    L = side * side
+    gx, gz = np.meshgrid(np.linspace(-1, 1, side), np.linspace(-1, 1, side))
+    xyz = torch.from_numpy(np.stack([gx.ravel(), np.zeros(L), gz.ravel()], axis=1).astype(np.float32)).to(cuda)
+    cube = torch.zeros((L, most), device=cuda)
+    cube[:, :T] = torch.rand((L, T), generator=torch.Generator(device=cuda).manual_seed(1), device=cuda)
+    depths = torch.linspace(0.3, 1.2, 16, dtype=torch.float64, device=cuda)
+
+    def planes(bins, n):
+        info = make_info(num_laser_targets=L, num_time_bins=bins, time_step=4.0 / T, voxel_res=(1, 1, 1),
+                         hidden_min=(0, 0, 0), voxel_size=(1, 1, 1), wall_normal=normal)
+        return ctx.backproject_depths(info, cube[:, :bins].contiguous(), xyz, depths[:n].contiguous())
+
+    assert torch.equal(planes(T, 2), planes(most, 2))
+    got, want = planes(T, 16), planes(most, 16)
+    ctx.check_device_status()
+    assert bool(want.any()) and not torch.equal(got, want)
+    assert rel_l2(got.cpu().numpy(), want.cpu().numpy()) < 1e-6
