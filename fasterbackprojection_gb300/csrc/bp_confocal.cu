@@ -223,9 +223,10 @@ fbp_status gather_scratch(fbp_context* ctx, size_t row_bytes, uint32_t* chains, 
     if (have < bytes) {
         // A smaller volume may want more of this than a larger one, so a graph
         // captured before must not lose its buffer to a later call: an outgrown
-        // one lives as long as the context, and each at least doubles the last
-        // (up to kChainSumBytes, which bounds them all together at twice that).
-        const size_t grown = std::max(bytes, std::min(2 * have, kChainSumBytes));
+        // one lives as long as the context.  Each at least doubles the last, and one
+        // of more than half of kChainSumBytes is that large at once and the last of
+        // all: together they stay below twice kChainSumBytes.
+        const size_t grown = bytes > kChainSumBytes / 2 ? kChainSumBytes : std::max(bytes, 2 * have);
         void* p = nullptr;
         if (!workspace_ready(ctx, WS_CHAIN_SUMS, bytes, stream)) {
             *chains = 1;
