@@ -115,28 +115,79 @@ struct BatchPlan {
     std::vector<std::vector<BatchItem>> items;  // per group
 };
 
+// Bin windows of a capture's tiles, with stages of a size that keeps `ctas` CTAs
+// on an SM.
+fbp_status batch_window(const fbp_batch* b, const fbp_recon_info& in, const TileCfg& tc, int ctas, WindowPlan* wp) {
+    const size_t meta = ConfocalGatherParams::meta_bytes(tc.kv) + kahan_smem_bytes(tc.kv, 32 * tc.wy * tc.wz) + 16;
+    const double ex = (double)std::min<uint32_t>(tc.kv, in.voxel_res[0]) * std::fabs(in.voxel_size[0]);
+    const double ey = (double)std::min<uint32_t>(4 * tc.wz, in.voxel_res[2]) * std::fabs(in.voxel_size[1]);
+    const double ez = (double)std::min<uint32_t>(8 * tc.wy, in.voxel_res[1]) * std::fabs(in.voxel_size[2]);
+    auto plan = [&](size_t meta_bytes) {
+        return plan_window(b->ctx, ex, ey, ez, in.time_step, in.num_time_bins, (int)(16 / kRowBytes), kRowBytes, meta_bytes,
+                           wp, "fbp_batch", 0.0, ctas, ConfocalGatherParams::kWindowBufs);
+    };
+    FBP_TRY(plan(meta));
+    // Leave room for the persistent kernel's own static shared memory
+    // (replanning only the windows that fill the SM, so the others keep
+    // the single-capture gather's plan).
+    if (wp->smem + kBatchStaticSmem > (size_t)b->ctx->smem_optin) FBP_TRY(plan(meta + kBatchStaticSmem));
+    return FBP_OK;
+}
+
+// CTAs to an SM that the windows' stages are cut for.  More of them fill the SM
+// better; fewer leave room for stages of more scan points, which matter where a
+// CTA has the SM nearly for itself (a stage of 8 instead of 32 points costs an
+// eighth).  Modelled as rounds of that many CTAs per SM, each round in units of
+// a full SM's work (rates as for the chains of a single gather), the last one
+// with what is left: few items run with large stages, many with three CTAs.  64
+// captures of 24^3 voxels (512 items): three CTAs 921 us, two 880; 8 of 64^3 (512,
+// longer stages) 3496 and 3696.  Items of uneven length that are all resident at
+// once end with the longest ones, so those get two at most: 16 captures of
+// 24^2..48^2 scan points, 24..39 x 40 x 32..64 voxels (366 items) 1661 and 1169 us.
+fbp_status batch_ctas(const fbp_batch* b, const TileCfg& tc, int* ctas) {
+    const int most = gather_ctas(32 * tc.wy * tc.wz);
+    constexpr double kRate[kGatherCtasPerSm] = {0.68, 0.88, 1.0};
+    const uint64_t sms = (uint64_t)b->ctx->sm_count;
+    double best = 0.0;
+    *ctas = most;
+    for (int r = 1; r <= most; ++r) {
+        uint64_t items = 0;
+        double work = 0.0, small = 0.0;  // small: the captures' share of time lost to short stages, alone on an SM
+        uint32_t longest = 0;
+        for (const auto& c : b->caps) {
+            WindowPlan wp;
+            FBP_TRY(batch_window(b, c.info, tc, r, &wp));
+            const double n = (double)cdiv(c.info.voxel_res[0], tc.kv) * cdiv(c.info.voxel_res[1], 8 * tc.wy) *
+                             cdiv(c.info.voxel_res[2], 4 * tc.wz);
+            items += (uint64_t)n;
+            work += n * c.info.num_laser_targets;
+            longest = std::max(longest, c.info.num_laser_targets);
+            small += n * c.info.num_laser_targets * 0.042 * (32.0 / wp.ch - 1.0);
+        }
+        if (r == 3 && items <= sms * r && longest * (double)items > 1.25 * work) break;
+        const uint64_t rounds = items / (sms * r), left = cdiv(items - rounds * sms * r, sms);
+        const double alone = left == 1 ? small / work : left == 2 ? 0.5 * small / work : 0.0;
+        const double t = rounds * (r / kRate[r - 1]) + (left ? left / kRate[left - 1] * (1.0 + alone) : 0.0);
+        if (r == 1 || t < best) {
+            best = t;
+            *ctas = r;
+        }
+    }
+    return FBP_OK;
+}
+
 // Works the plan out; the batch stays as it is.
 fbp_status make_plan(const fbp_batch* b, int cfg, BatchPlan* plan) {
     const TileCfg tc = kTileCfgs[cfg];
-    const int align = (int)(16 / kRowBytes);
-    const size_t meta = ConfocalGatherParams::meta_bytes(tc.kv) + kahan_smem_bytes(tc.kv, 32 * tc.wy * tc.wz) + 16;
     const uint32_t n = (uint32_t)b->caps.size();
+    int ctas = 1;
+    FBP_TRY(batch_ctas(b, tc, &ctas));
     plan->params.assign(n, ConfocalGatherParams{});
     plan->rows_off.resize(n);
     for (uint32_t i = 0; i < n; ++i) {
         const fbp_recon_info& in = b->caps[i].info;
-        const double ex = (double)std::min<uint32_t>(tc.kv, in.voxel_res[0]) * std::fabs(in.voxel_size[0]);
-        const double ey = (double)std::min<uint32_t>(4 * tc.wz, in.voxel_res[2]) * std::fabs(in.voxel_size[1]);
-        const double ez = (double)std::min<uint32_t>(8 * tc.wy, in.voxel_res[1]) * std::fabs(in.voxel_size[2]);
-        WindowPlan wp;
-        FBP_TRY(plan_window(b->ctx, ex, ey, ez, in.time_step, in.num_time_bins, align, kRowBytes, meta, &wp,
-                            "fbp_batch", 0.0, kGatherCtasPerSm, ConfocalGatherParams::kWindowBufs));
-        // Leave room for the persistent kernel's own static shared memory
-        // (replanning only the windows that fill the SM, so the others keep
-        // the single-capture gather's plan).
-        if (wp.smem + kBatchStaticSmem > (size_t)b->ctx->smem_optin)
-            FBP_TRY(plan_window(b->ctx, ex, ey, ez, in.time_step, in.num_time_bins, align, kRowBytes,
-                                meta + kBatchStaticSmem, &wp, "fbp_batch", 0.0, kGatherCtasPerSm, ConfocalGatherParams::kWindowBufs));
+        WindowPlan wp, single;
+        FBP_TRY(batch_window(b, in, tc, ctas, &wp));
         plan->rows_off[i] = plan->rows_bytes;
         plan->rows_bytes += ((size_t)in.num_laser_targets * wp.pitch * kRowBytes + 255) & ~size_t(255);
         ConfocalGatherParams& p = plan->params[i];
@@ -157,7 +208,11 @@ fbp_status make_plan(const fbp_batch* b, int cfg, BatchPlan* plan) {
         p.slot_w = wp.slot_w;
         p.ch = wp.ch;
         // The single call's chains where the tile is the single call's.
-        p.chains = cfg == 0 ? gather_chains(b->ctx, in, wp.smem) : 1;
+        p.chains = 1;
+        if (cfg == 0) {
+            FBP_TRY(batch_window(b, in, tc, kGatherCtasPerSm, &single));
+            p.chains = gather_chains(b->ctx, in, single.smem);
+        }
         p.exact_weights = b->ctx->weight_mode == FBP_WEIGHTS_REFERENCE;
         // Group by arithmetic variant and occupancy.
         const int path = path_of(in);
