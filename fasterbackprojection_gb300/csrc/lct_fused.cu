@@ -62,9 +62,15 @@ struct LctFusedParams {
 // (Half the lines for the two longest, 35 KB, halves the width of the strided
 // accesses: 64^2 x 2048 in 450 against 347 us.)
 constexpr int z_lines(int log2z) { return log2z <= 11 ? 8 : 4; }
-constexpr int z_threads(int log2z) {
-    return (z_lines(log2z) / 2 << log2z) / 16 < 64 ? 64 : (z_lines(log2z) / 2 << log2z) / 16;
+// Where the lines are short and the CTAs all resident at once, up to 256 threads
+// instead: each has fewer loads, rows and stores in its chain (8^2 x 128 12.1 ->
+// 9.9 us, 64^2 x 128 21.8 -> 19.7; but 128^2 x 64, more CTAs than the GPU holds,
+// 46.5 -> 50.0).
+constexpr int z_threads(int log2z, bool wide) {
+    const int points = z_lines(log2z) / 2 << log2z;
+    return wide ? (points < 256 ? points : 256) : points / 16 < 64 ? 64 : points / 16;
 }
+constexpr int kWideLog2Z = 8;
 constexpr int z_ctas(int log2z) { return log2z <= 10 ? 4 : 2; }
 
 // The lines' stride and the two raw lines' within one: the 32 (line, bin) pairs of
@@ -89,10 +95,10 @@ constexpr int plane_threads() { return LOG2X >= 7 ? 512 : 256; }
 // shared-memory pipe they take (now 46 %).  64^2 x 512: 31.6 us with 512 threads
 // on as many lines, every element walking its own row of mtx; 20.7 with these
 // lines, threads and shared rows; 17.4 with the skews and the stage tables by r.
-template <int LOG2Z>
-__global__ void __launch_bounds__(z_threads(LOG2Z), z_ctas(LOG2Z)) lct_zfwd_kernel(LctFusedParams p) {
+template <int LOG2Z, bool WIDE>
+__global__ void __launch_bounds__(z_threads(LOG2Z, WIDE), z_ctas(LOG2Z)) lct_zfwd_kernel(LctFusedParams p) {
     constexpr int Z = 1 << LOG2Z, M = Z / 2, C = z_lines(LOG2Z), H = C / 2, LS = z_stride(LOG2Z),
-                  TWN = stage_table_size(LOG2Z), NT = z_threads(LOG2Z);
+                  TWN = stage_table_size(LOG2Z), NT = z_threads(LOG2Z, WIDE);
     extern __shared__ __align__(16) float2 sm[];
     float2* lines = sm;  // [H] complex lines: real line 2j in the real part, 2j + 1 in the imaginary part
     float2* tw = lines + H * LS;
@@ -341,10 +347,10 @@ __global__ void __launch_bounds__(kP128Threads, 2) lct_plane128_kernel(LctFusedP
 }
 
 // Bound like the forward pass; 27.9, 18.1 and 16.6 us by the same steps.
-template <int LOG2Z>
-__global__ void __launch_bounds__(z_threads(LOG2Z), z_ctas(LOG2Z)) lct_zinv_kernel(LctFusedParams p) {
+template <int LOG2Z, bool WIDE>
+__global__ void __launch_bounds__(z_threads(LOG2Z, WIDE), z_ctas(LOG2Z)) lct_zinv_kernel(LctFusedParams p) {
     constexpr int Z = 1 << LOG2Z, M = Z / 2, C = z_lines(LOG2Z), H = C / 2, LS = z_stride(LOG2Z),
-                  TWN = stage_table_size(LOG2Z), NT = z_threads(LOG2Z);
+                  TWN = stage_table_size(LOG2Z), NT = z_threads(LOG2Z, WIDE);
     extern __shared__ __align__(16) float2 sm[];
     float2* lines = sm;
     float2* tw = lines + H * LS;
@@ -544,14 +550,17 @@ fbp_status launch_rows_cols(fbp_context* ctx, const LctFusedParams& p, unsigned 
     return FBP_OK;
 }
 
-template <int LOG2Z>
+template <int LOG2Z, bool WIDE = false>
 fbp_status launch_z(fbp_context* ctx, const LctFusedParams& p, bool forward, cudaStream_t s) {
     const dim3 grid(p.N / z_lines(LOG2Z), p.N);  // N is a power of two of at least 8
+    if constexpr (LOG2Z <= kWideLog2Z && !WIDE) {
+        if (grid.x * grid.y <= (unsigned)(z_ctas(LOG2Z) * ctx->sm_count)) return launch_z<LOG2Z, true>(ctx, p, forward, s);
+    }
     constexpr size_t smem = z_smem<LOG2Z>();
     static_assert(smem * z_ctas(LOG2Z) <= 220 * 1024, "z tiles too large");
-    auto k = forward ? lct_zfwd_kernel<LOG2Z> : lct_zinv_kernel<LOG2Z>;
+    auto k = forward ? lct_zfwd_kernel<LOG2Z, WIDE> : lct_zinv_kernel<LOG2Z, WIDE>;
     FBP_TRY_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k<<<grid, z_threads(LOG2Z), smem, s>>>(p);
+    k<<<grid, z_threads(LOG2Z, WIDE), smem, s>>>(p);
     FBP_CHECK_LAUNCH(ctx, forward ? "lct_zfwd_kernel" : "lct_zinv_kernel");
     return FBP_OK;
 }
