@@ -137,10 +137,11 @@ struct ConfocalGatherParams {
 };
 
 // Shared memory holding the compensated (Kahan) sums of a CTA's voxels when a
-// thread owns 16 of them (sum and compensation per voxel, [2 KV][threads]):
-// kept there instead of in 64 registers, so three CTAs fit per SM.
-__host__ __device__ constexpr size_t kahan_smem_bytes(int kv, int threads) {
-    return kv >= 16 ? (size_t)2 * kv * threads * sizeof(float) : 0;
+// thread owns 16 of them, or walks 8 of the voxel-scattering variant (sum and
+// compensation per voxel, [2 KV][threads]): kept there instead of in 64 (or 16)
+// registers, so three (or four) CTAs fit per SM.
+__host__ __device__ constexpr size_t kahan_smem_bytes(int kv, int threads, bool scatter = false) {
+    return kv >= 16 || scatter ? (size_t)2 * kv * threads * sizeof(float) : 0;
 }
 
 // Window geometry shared by the gathers: the widest bin span a tile of the
@@ -160,6 +161,8 @@ fbp_status plan_window(const fbp_context* ctx, double ex, double ey, double ez, 
 // volume, whatever part of it a launch computes, so that slabs and batches sum
 // like the single call).
 uint32_t gather_chains(const fbp_context* ctx, const fbp_recon_info& in, size_t smem);
+// The same for the voxel-scattering variant, whose walks take `steps` steps.
+uint32_t scatter_chains(const fbp_context* ctx, const fbp_recon_info& in, size_t smem, double steps);
 // Chains for a launch of `tiles` tiles (whose warps are `busy` to that part)
 // that each walk `groups` groups of `group_us` microseconds (at an SM's full
 // rate) into n outputs, occ CTAs to an SM.
@@ -168,6 +171,7 @@ uint32_t split_chains(const fbp_context* ctx, uint64_t tiles, double busy, uint6
 // Part of the warps of 16 x 16 (rows, slices) tiles that own voxels of a volume.
 double busy_warps(const uint32_t res[3]);
 constexpr double kGatherGroupUs = 6.3;  // 32 scan points x 4096 voxels
+constexpr double kScatterStepUs = 2.5;  // 32 scan points x 2048 voxels, per step of the walk
 // out[i] = the chains' sums [chains][sum, compensation][n], folded in order.
 // Scratch of a gather: its rows and, for n outputs in several chains, their sums
 // ([chains][2][n]; *chains becomes 1 where there is no room for them: no memory,
@@ -180,7 +184,8 @@ inline int resident_ctas(size_t smem, int most) {
     const size_t n = kSmSharedBytes / (smem + kCtaReservedShared);
     return n < 1 ? 1 : (n < (size_t)most ? (int)n : most);
 }
-constexpr int kGatherCtasPerSm = 3;  // 256 threads of 80 registers
+constexpr int kGatherCtasPerSm = 3;   // 256 threads of 80 registers
+constexpr int kScatterCtasPerSm = 4;  // ... of 64: the voxel-scattering walk of 8 voxels
 
 // The confocal gather over all scan points (smp == nullptr) or over K sampled
 // scan points per tile (the unbiased MIS estimator).

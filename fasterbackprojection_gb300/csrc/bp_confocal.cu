@@ -72,13 +72,6 @@ fbp_status launch_confocal(fbp_context* ctx, const fbp_recon_info& in, const voi
     if (z_begin >= z_end) return FBP_OK;
     constexpr int ALIGN = 4;  // FP32 rows
 
-    // World extents of the largest tile (clamped to the volume).
-    const uint32_t kv = smp ? kKV : kKVFull;
-    const double ex = (double)std::min<uint32_t>(kv, Vx) * std::fabs(in.voxel_size[0]);
-    const double ey = (double)std::min<uint32_t>(4 * kWZ, Vz) * std::fabs(in.voxel_size[1]);
-    const double ez = (double)std::min<uint32_t>(8 * kWY, Vy) * std::fabs(in.voxel_size[2]);
-    WindowPlan wp;
-    // The sampled kernel also holds its cluster list in static shared memory.
     // The voxel-scattering variant reads every bin of dist -/+ half the voxel
     // diagonal, one step past the end (up to max(step, diagonal) from 0 where
     // a walk is clipped at 0).
@@ -86,16 +79,45 @@ fbp_status launch_confocal(fbp_context* ctx, const fbp_recon_info& in, const voi
                                    (double)in.voxel_size[1] * in.voxel_size[1] +
                                    (double)in.voxel_size[2] * in.voxel_size[2]);
     const double extra = scatter ? 1.52 * vdiag + 2.0 * std::fabs((double)in.time_step) : 0.0;
-    FBP_TRY(plan_window(ctx, ex, ey, ez, in.time_step, T, ALIGN, sizeof(float),
-                        ConfocalGatherParams::meta_bytes((int)kv) + (smp ? kSampledStaticSmem : 0) +
-                            kahan_smem_bytes((int)kv, 32 * kWY * kWZ) + 16,
-                        &wp, "fbp_backproject_confocal", extra,
-                        gather_ctas(32 * kWY * kWZ),
-                        ConfocalGatherParams::kWindowBufs));
-    if (smp) wp.smem -= kSampledStaticSmem;
+    // Steps per (voxel, scan point): at most ceil(diagonal / (dt + EPS)),
+    // one more where rounding lands on the end; the kernel unrolls 2..4
+    // of them and loops over the rest.  Where even the shortest walk
+    // takes all the unrolled steps (a 1e-4 m margin over the rounding of
+    // the path arithmetic below 64 m) they need no end test, and the
+    // unclamped window index of the other paths applies.
+    const double step = (double)in.time_step + (double)FBP_EPS;
+    const int sp = (int)std::min(std::max(std::ceil(vdiag / step), 2.0), (double)kScatterMaxPrefix);
+    const bool free_walk = scatter && (sp - 1) * step + 1e-4 < vdiag;
+    // ... and where none takes more (sp steps already pass the far end).
+    const bool exact_walk = free_walk && sp * step > vdiag + 1e-4;
 
+    // Windows of the largest tile (clamped to the volume) of kv voxels along x.
+    // The sampled kernel also holds its cluster list in static shared memory.
+    WindowPlan wp, wide;
+    auto plan = [&](uint32_t kv, bool narrow, WindowPlan* out) -> fbp_status {
+        const double ex = (double)std::min<uint32_t>(kv, Vx) * std::fabs(in.voxel_size[0]);
+        const double ey = (double)std::min<uint32_t>(4 * kWZ, Vz) * std::fabs(in.voxel_size[1]);
+        const double ez = (double)std::min<uint32_t>(8 * kWY, Vy) * std::fabs(in.voxel_size[2]);
+        return plan_window(ctx, ex, ey, ez, in.time_step, T, ALIGN, sizeof(float),
+                           ConfocalGatherParams::meta_bytes((int)kv) + (smp ? kSampledStaticSmem : 0) +
+                               kahan_smem_bytes((int)kv, 32 * kWY * kWZ, scatter) + 16,
+                           out, "fbp_backproject_confocal", extra, gather_ctas(32 * kWY * kWZ, narrow),
+                           ConfocalGatherParams::kWindowBufs);
+    };
     ConfocalGatherParams p{};
-    p.chains = smp ? 1 : gather_chains(ctx, in, wp.smem);
+    uint32_t kv = smp || scatter ? kKV : kKVFull;
+    FBP_TRY(plan(kv, scatter, &wp));
+    if (smp) wp.smem -= kSampledStaticSmem;
+    p.chains = smp ? 1 : scatter ? scatter_chains(ctx, in, wp.smem, vdiag / step) : gather_chains(ctx, in, wp.smem);
+    if (exact_walk) {
+        if (plan(kKVFull, false, &wide) != FBP_OK) {
+            clear_error();
+        } else if (gather_chains(ctx, in, wide.smem) == 1) {
+            kv = kKVFull;
+            wp = wide;
+            p.chains = 1;
+        }
+    }
     float* rows = nullptr;
     FBP_TRY(gather_scratch(ctx, (size_t)L * wp.pitch * sizeof(float), &p.chains, (uint64_t)Vx * Vy * (z_end - z_begin), stream,
                            &rows, &p.chain_sums));
@@ -123,18 +145,8 @@ fbp_status launch_confocal(fbp_context* ctx, const fbp_recon_info& in, const voi
     dim3 grid(cdiv(Vx, kv), cdiv(Vy, 8 * kWY), cdiv(z_end - z_begin, 4 * kWZ));
     const bool bounce = in.discard_first_last_bounces == 0;
     if (scatter) {
-        // Steps per (voxel, scan point): at most ceil(diagonal / (dt + EPS)),
-        // one more where rounding lands on the end; the kernel unrolls 2..4
-        // of them and loops over the rest.  Where even the shortest walk
-        // takes all the unrolled steps (a 1e-4 m margin over the rounding of
-        // the path arithmetic below 64 m) they need no end test, and the
-        // unclamped window index of the other paths applies.
-        const double step = (double)in.time_step + (double)FBP_EPS;
-        const double steps = std::ceil(vdiag / step);
-        const int sp = (int)std::min(std::max(steps, 2.0), (double)kScatterMaxPrefix);
-        const bool free_walk = (sp - 1) * step + 1e-4 < vdiag;
-        // ... and where none takes more (sp steps already pass the far end).
-        p.scat_exact = free_walk && sp * step > vdiag + 1e-4;
+        p.scat_exact = exact_walk;
+        if (kv == kKVFull) return gather_scatter_wide(ctx, p, grid, wp.smem, stream, sp, bounce, wp.capped);
         if (p.chains > 1) return gather_scatter_split(ctx, p, grid, wp.smem, stream, sp, free_walk, bounce, wp.capped);
         return gather_scatter(ctx, p, grid, wp.smem, stream, sp, free_walk, bounce, wp.capped);
     }
@@ -153,9 +165,9 @@ constexpr size_t kChainSumBytes = (size_t)128 << 20;
 // busy, else as many as a model of the launch asks for.  The model, in units of
 // one group at an SM's full rate: the busiest SM's CTAs, each with its share of
 // the groups and half a group of set-up, at the rate of the CTAs resident
-// together (one or two reach 0.68 and 0.88 of three), the uneven end (a whole
-// CTA where tiles differ in their idle warps), and the sums' way through memory
-// and the fold's launch.  One CTA per tile against this rule (both with the
+// together (one or two reach 0.68 and 0.88 of three; 0.55, 0.8 and 0.93 of four),
+// the uneven end (a whole CTA where tiles differ in their idle warps), and the
+// sums' way through memory and the fold's launch.  One CTA per tile against this rule (both with the
 // tables' launches of their own, which one launch for rows and tables has since
 // taken 8-28 us off): 32^2 x 256 -> 32^3 328 -> 45 us (16 chains), 64^2 x 512 ->
 // 64^3 1264 -> 432 us (7), 90^2 x 700 -> 75 x 101 x 83 4028 -> 2189 us (16),
@@ -165,7 +177,8 @@ constexpr size_t kChainSumBytes = (size_t)128 << 20;
 // part of a GPC's slots empty): 48, 483, 2596 us, 11.9 ms, 728 us.
 uint32_t split_chains(const fbp_context* ctx, uint64_t tiles, double busy, uint64_t groups, int occ, double group_us,
                       uint64_t n) {
-    constexpr double kRate[kGatherCtasPerSm] = {0.68, 0.88, 1.0};
+    constexpr double kRates[2][kScatterCtasPerSm] = {{0.68, 0.88, 1.0}, {0.55, 0.8, 0.93, 1.0}};
+    const double* const kRate = kRates[occ > kGatherCtasPerSm];
     constexpr uint32_t kMaxChains = 32;
     uint32_t best = 1;
     double best_t = 0.0;
@@ -195,6 +208,14 @@ uint32_t gather_chains(const fbp_context* ctx, const fbp_recon_info& in, size_t 
     return split_chains(ctx, tiles, busy_warps(in.voxel_res),
                         cdiv(in.num_laser_targets, ConfocalGatherParams::kGroup), resident_ctas(smem, kGatherCtasPerSm),
                         kGatherGroupUs, (uint64_t)in.voxel_res[0] * in.voxel_res[1] * in.voxel_res[2]);
+}
+
+uint32_t scatter_chains(const fbp_context* ctx, const fbp_recon_info& in, size_t smem, double steps) {
+    const uint64_t tiles = (uint64_t)cdiv(in.voxel_res[0], kKV) * cdiv(in.voxel_res[1], 8 * kWY) *
+                           cdiv(in.voxel_res[2], 4 * kWZ);
+    return split_chains(ctx, tiles, busy_warps(in.voxel_res),
+                        cdiv(in.num_laser_targets, ConfocalGatherParams::kGroup), resident_ctas(smem, kScatterCtasPerSm),
+                        kScatterStepUs * std::max(steps, 2.0), (uint64_t)in.voxel_res[0] * in.voxel_res[1] * in.voxel_res[2]);
 }
 
 fbp_status gather_scratch(fbp_context* ctx, size_t row_bytes, uint32_t* chains, uint64_t n, cudaStream_t stream,

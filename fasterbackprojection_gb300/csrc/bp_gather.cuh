@@ -37,6 +37,11 @@ constexpr int kScatterForms = kScatterMaxPrefix - 1;  // prefixes 2, 3, 4
 __host__ __device__ constexpr bool is_scatter(int path) { return path >= PATH_SCATTER; }
 __host__ __device__ constexpr int scatter_prefix(int path) { return (path - PATH_SCATTER) % kScatterForms + 2; }
 __host__ __device__ constexpr bool scatter_free(int path) { return path - PATH_SCATTER >= kScatterForms; }
+// The scattering walk of 8 voxels per thread.  It is bound by the latency of its
+// dependent steps, so four CTAs of 64 registers count for more than what 16
+// voxels share (their plan reads and stages); it keeps its voxels' x instead
+// of reading planned differences, the shared-memory pipe being half full.
+__host__ __device__ constexpr bool scatter_narrow(int kv, int path) { return is_scatter(path) && kv == 8; }
 
 // What the pair loop reads of a planned scan point (broadcast shared loads).
 // dx: the x differences to the tile's KV voxel columns, as packed pairs: the
@@ -55,7 +60,7 @@ template <int KV, int PATH, bool BOUNCE, bool CLAMP, bool SAFE, bool WEIGHTED>
 __device__ __forceinline__ void confocal_stage(const ScanPlan pl, int nl, float py,
                                                float pz, float neg_t0, float rcp_dt, uint32_t slot_w,
                                                float (&acc)[KV], float ext = 0.f, float step = 0.f,
-                                               bool tail = true) {
+                                               bool tail = true, const f32x2_t* px = nullptr) {
     const float rcp2 = 2.f * rcp_dt;  // exact
     if constexpr (is_scatter(PATH)) {
         constexpr int SP = scatter_prefix(PATH);
@@ -75,11 +80,17 @@ __device__ __forceinline__ void confocal_stage(const ScanPlan pl, int nl, float 
             const float dy = sub_rn(py, g.y), dz = sub_rn(pz, g.z);
             const float dy2 = mul_rn(dy, dy);
             f32x2_t dxp[KV / 2];
+            if constexpr (scatter_narrow(KV, PATH)) {
+                const f32x2_t gxp = pack2(g.x, g.x);
 #pragma unroll
-            for (int j = 0; j < KV / 4; ++j) {
-                const ulonglong2 v = pl.dx[(size_t)i * (KV / 4) + j];
-                dxp[2 * j] = v.x;
-                dxp[2 * j + 1] = v.y;
+                for (int j = 0; j < KV / 2; ++j) dxp[j] = sub_rn2(px[j], gxp);
+            } else {
+#pragma unroll
+                for (int j = 0; j < KV / 4; ++j) {
+                    const ulonglong2 v = pl.dx[(size_t)i * (KV / 4) + j];
+                    dxp[2 * j] = v.x;
+                    dxp[2 * j + 1] = v.y;
+                }
             }
             auto bin_at = [&](float dd) -> float {
                 const float x = ref_bin_ratio(dd, rcp_dt);
@@ -349,6 +360,12 @@ __device__ __forceinline__ void confocal_tile(const ConfocalGatherParams& p, uin
     const float py = p.ys[min(vz, p.Vz - 1)];
     const float pz = p.zs[min(vy, p.Vy - 1)];
 
+    constexpr bool PX = scatter_narrow(KV, PATH);
+    f32x2_t px[PX ? KV / 2 : 1];
+#pragma unroll
+    for (int j = 0; j < (PX ? KV / 2 : 0); ++j)
+        px[j] = pack2(p.xs[min(tx0 + 2 * j, p.Vx - 1)], p.xs[min(tx0 + 2 * j + 1, p.Vx - 1)]);
+
     const float rcp_dt = rcp_approx(p.dt);
     const float neg_t0 = -p.t0;
     // PATH_SCATTER: length(voxelSize) / 2 and the step timeStep + EPS, in the
@@ -539,7 +556,7 @@ __device__ __forceinline__ void confocal_tile(const ConfocalGatherParams& p, uin
                 s_meta[gb + pos] = make_int4(bias, bias, (int)slot, 0);
                 float* dx = reinterpret_cast<float*>(s_dx + (gb + pos) * (KV / 4));
 #pragma unroll
-                for (int k = 0; k < KV; ++k) dx[k] = sub_rn(p.xs[min(tx0 + k, p.Vx - 1)], g.x);
+                for (int k = 0; k < (PX ? 0 : KV); ++k) dx[k] = sub_rn(p.xs[min(tx0 + k, p.Vx - 1)], g.x);
                 s_cnt[gb + pos] = cnt;
                 s_src[gb + pos] = static_cast<const float*>(p.rows) + (size_t)l * p.row_pitch + a;
                 s_w[gb + pos] = wgt;
@@ -576,10 +593,10 @@ __device__ __forceinline__ void confocal_tile(const ConfocalGatherParams& p, uin
                       bytes, bar_full + 8 * buf);
     };
 
-    // Compensated sums: in registers, or (16 voxels per thread) in shared
-    // memory behind the windows, [2 KV][NT] so a warp's accesses are
-    // consecutive words.
-    constexpr bool KSMEM = kahan_smem_bytes(KV, NT) > 0;
+    // Compensated sums: in registers, or (16 voxels per thread, the scattering
+    // walk) in shared memory behind the windows, [2 KV][NT] so a warp's accesses
+    // are consecutive words.
+    constexpr bool KSMEM = kahan_smem_bytes(KV, NT, is_scatter(PATH)) > 0;
     static_assert(!SPLIT || KSMEM, "a split tile keeps its compensated sums in shared memory");
     float* s_kahan = reinterpret_cast<float*>(
         smem_raw + ((slots_off + (size_t)NB * CH * slot_stride * sizeof(float) + 15) & ~size_t(15)));
@@ -615,11 +632,11 @@ __device__ __forceinline__ void confocal_tile(const ConfocalGatherParams& p, uin
                 const ScanPlan plan{s_geo + o, s_meta + o, s_dx + o * (KV / 4), s_w + o};
                 if (!grp.y) {
                     confocal_stage<KV, PATH, BOUNCE, CLAMP, false, SAMPLED>(plan, nl, py, pz, neg_t0, rcp_dt, p.slot_w,
-                                                                            acc, scat_ext, scat_step, !p.scat_exact);
+                                                                            acc, scat_ext, scat_step, !p.scat_exact, px);
                     if (PATH == PATH_2D) scale = 0.25f;  // w was rcp(d^2) = 4 rcp(dist^2)
                 } else {
                     confocal_stage<KV, PATH, BOUNCE, CLAMP, true, SAMPLED>(plan, nl, py, pz, neg_t0, rcp_dt, p.slot_w,
-                                                                           acc, scat_ext, scat_step);
+                                                                           acc, scat_ext, scat_step, true, px);
                 }
             }
             __syncwarp();
@@ -678,11 +695,13 @@ __device__ __forceinline__ void confocal_tile(const ConfocalGatherParams& p, uin
     }
 }
 
-// Registers for three CTAs of 256 threads (80 each).
-constexpr int gather_ctas(int threads) { return threads > 256 ? 1 : kGatherCtasPerSm; }
+// Registers for three CTAs of 256 threads (80 each), or four (64).
+constexpr int gather_ctas(int threads, bool narrow = false) {
+    return threads > 256 ? 1 : narrow ? kScatterCtasPerSm : kGatherCtasPerSm;
+}
 
 template <int KV, int WY, int WZ, int PATH, bool BOUNCE, bool SAMPLED, bool CLAMP, bool SPLIT = false>
-__global__ void __launch_bounds__(32 * WY * WZ, gather_ctas(32 * WY * WZ))
+__global__ void __launch_bounds__(32 * WY * WZ, gather_ctas(32 * WY * WZ, scatter_narrow(KV, PATH)))
 confocal_gather_kernel(ConfocalGatherParams p) {
     const uint32_t cs = SPLIT ? p.chains : 1, bx = blockIdx.x / cs;
     const unsigned long long tile_id = ((unsigned long long)blockIdx.z * gridDim.y + blockIdx.y) * (gridDim.x / cs) + bx;

@@ -8,9 +8,11 @@ namespace fbp {
 
 // Voxels per thread along x: 16 (the scan point's geometry and the stage's
 // bookkeeping amortised over more pairs: 2.67e12 -> 2.74e12 pairs/s at 256^3
-// with the gather as it then was; the voxel-scattering walk 52.2 -> 48.8 ms
-// for 64^2 x 1024 -> 256^3), 8 for the sampled gather (its tiles are the MIS
-// sampling tiles).
+// with the gather as it then was), 8 for the sampled gather (its tiles are the MIS
+// sampling tiles) and for the voxel-scattering walk, which takes 16 only where
+// every walk is as long as its unrolled steps and the volume needs no chains:
+// 64^2 x 1024 -> 256^3 50.8 against 53.5 ms, but with longer walks (64^2 x 2048)
+// 118.0 against 116.2, and 40^2 x 1024 -> 160^3 10.26 against 9.76.
 constexpr int kKV = 8, kKVFull = 16, kWY = 2, kWZ = 4;
 
 fbp_status gather_full(fbp_context* ctx, const ConfocalGatherParams& p, dim3 grid, size_t smem, cudaStream_t stream,
@@ -21,6 +23,9 @@ fbp_status gather_sampled(fbp_context* ctx, const ConfocalGatherParams& p, dim3 
 // them all.
 fbp_status gather_scatter(fbp_context* ctx, const ConfocalGatherParams& p, dim3 grid, size_t smem, cudaStream_t stream,
                           int sp, bool free_walk, bool bounce, bool capped);
+// 16 voxels per thread: free walks.
+fbp_status gather_scatter_wide(fbp_context* ctx, const ConfocalGatherParams& p, dim3 grid, size_t smem,
+                               cudaStream_t stream, int sp, bool bounce, bool capped);
 // The same with p.chains CTAs per tile.
 fbp_status gather_full_split(fbp_context* ctx, const ConfocalGatherParams& p, dim3 grid, size_t smem,
                              cudaStream_t stream, bool bounce, float t0, bool capped);
@@ -28,9 +33,8 @@ fbp_status gather_scatter_split(fbp_context* ctx, const ConfocalGatherParams& p,
                                 cudaStream_t stream, int sp, bool free_walk, bool bounce, bool capped);
 
 // One launch of the gather; SPLIT: p.chains CTAs per tile, then the fold.
-template <int PATH, bool BOUNCE, bool SAMPLED, bool CLAMP, bool SPLIT>
+template <int PATH, bool BOUNCE, bool SAMPLED, bool CLAMP, bool SPLIT, int KV = SAMPLED ? kKV : kKVFull>
 fbp_status go_confocal(fbp_context* ctx, ConfocalGatherParams p, dim3 grid, size_t smem, cudaStream_t stream) {
-    constexpr int KV = SAMPLED ? kKV : kKVFull;
     auto kernel = confocal_gather_kernel<KV, kWY, kWZ, PATH, BOUNCE, SAMPLED, CLAMP, SPLIT>;
     FBP_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const uint64_t n = (uint64_t)p.Vx * p.Vy * p.Vz;
@@ -61,30 +65,32 @@ fbp_status dispatch_confocal(fbp_context* ctx, const ConfocalGatherParams& p, di
 
 // The voxel-scattering walks of prefix SP: predicated steps (clamped window
 // index), or unconditional ones, clamped only where the window is the row.
-template <int SP, bool SPLIT>
+template <int SP, bool SPLIT, int KV>
 fbp_status dispatch_scatter(fbp_context* ctx, const ConfocalGatherParams& p, dim3 grid, size_t smem,
                             cudaStream_t stream, bool free_walk, bool bounce, bool capped) {
     constexpr int W = PATH_SCATTER + SP - 2, F = W + kScatterForms;
-    if (!free_walk) {
-        if (bounce) return go_confocal<W, true, false, true, SPLIT>(ctx, p, grid, smem, stream);
-        return go_confocal<W, false, false, true, SPLIT>(ctx, p, grid, smem, stream);
+    if constexpr (KV == kKV) {
+        if (!free_walk) {
+            if (bounce) return go_confocal<W, true, false, true, SPLIT, KV>(ctx, p, grid, smem, stream);
+            return go_confocal<W, false, false, true, SPLIT, KV>(ctx, p, grid, smem, stream);
+        }
     }
     if (bounce) {
-        if (capped) return go_confocal<F, true, false, true, SPLIT>(ctx, p, grid, smem, stream);
-        return go_confocal<F, true, false, false, SPLIT>(ctx, p, grid, smem, stream);
+        if (capped) return go_confocal<F, true, false, true, SPLIT, KV>(ctx, p, grid, smem, stream);
+        return go_confocal<F, true, false, false, SPLIT, KV>(ctx, p, grid, smem, stream);
     }
-    if (capped) return go_confocal<F, false, false, true, SPLIT>(ctx, p, grid, smem, stream);
-    return go_confocal<F, false, false, false, SPLIT>(ctx, p, grid, smem, stream);
+    if (capped) return go_confocal<F, false, false, true, SPLIT, KV>(ctx, p, grid, smem, stream);
+    return go_confocal<F, false, false, false, SPLIT, KV>(ctx, p, grid, smem, stream);
 }
 
-template <bool SPLIT>
+template <bool SPLIT, int KV = kKV>
 fbp_status dispatch_scatter(fbp_context* ctx, const ConfocalGatherParams& p, dim3 grid, size_t smem,
                             cudaStream_t stream, int sp, bool free_walk, bool bounce, bool capped) {
     static_assert(kScatterMaxPrefix == 4, "one case per prefix");
     switch (sp) {
-        case 2: return dispatch_scatter<2, SPLIT>(ctx, p, grid, smem, stream, free_walk, bounce, capped);
-        case 3: return dispatch_scatter<3, SPLIT>(ctx, p, grid, smem, stream, free_walk, bounce, capped);
-        case 4: return dispatch_scatter<4, SPLIT>(ctx, p, grid, smem, stream, free_walk, bounce, capped);
+        case 2: return dispatch_scatter<2, SPLIT, KV>(ctx, p, grid, smem, stream, free_walk, bounce, capped);
+        case 3: return dispatch_scatter<3, SPLIT, KV>(ctx, p, grid, smem, stream, free_walk, bounce, capped);
+        case 4: return dispatch_scatter<4, SPLIT, KV>(ctx, p, grid, smem, stream, free_walk, bounce, capped);
         default: return set_error(FBP_ERR_INTERNAL, "voxel scattering: no kernel for this step prefix");
     }
 }
