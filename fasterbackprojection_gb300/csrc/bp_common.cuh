@@ -172,12 +172,12 @@ uint32_t split_chains(const fbp_context* ctx, uint64_t tiles, double busy, uint6
 double busy_warps(const uint32_t res[3]);
 constexpr double kGatherGroupUs = 6.3;  // 32 scan points x 4096 voxels
 constexpr double kScatterStepUs = 2.5;  // 32 scan points x 2048 voxels, per step of the walk
-// out[i] = the chains' sums [chains][sum, compensation][n], folded in order.
 // Scratch of a gather: its rows and, for n outputs in several chains, their sums
 // ([chains][2][n]; *chains becomes 1 where there is no room for them: no memory,
 // or a stream under capture and too small a buffer).
 fbp_status gather_scratch(fbp_context* ctx, size_t row_bytes, uint32_t* chains, uint64_t n, cudaStream_t stream,
                           float** rows, float** sums);
+// out[i] = the chains' sums [chains][sum, compensation][n], folded in order.
 fbp_status fold_chains(fbp_context* ctx, const float* sums, uint32_t chains, uint64_t n, float* out, cudaStream_t stream);
 // CTAs of `smem` bytes of dynamic shared memory an SM holds, at most `most`.
 inline int resident_ctas(size_t smem, int most) {

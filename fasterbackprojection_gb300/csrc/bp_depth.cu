@@ -4,10 +4,15 @@
 // (Laser.cu:379-480) and backprojectConfocal / backprojectExhaustive
 // (transient_reconstruction.cuh:41-91).  Test points are
 //   laser_xyz[c] + wall_normal * float(depths[d])
-// and contributions are unweighted.  One thread owns one test point and sums
-// over every scan point (or laser/SPAD pair) from the padded rows in a fixed
-// order (FP32 per block of 64, Kahan across blocks), instead of one atomic per
-// pair.  Time bins follow the reference's FP32 expression exactly.
+// and contributions are unweighted, summed in a fixed order instead of by one
+// atomic per pair.  Time bins follow the reference's FP32 expression exactly.
+//   Confocal: depth_tile_kernel, a thread for 16 test points of a tile, windows
+//   of the rows in shared memory, FP32 sums of 32 scan points folded with
+//   compensation.
+//   Few planes of many scan points (tiles_pay), rows too long for the tiles'
+//   windows, no memory for FP32 rows, and every exhaustive capture: a thread per
+//   test point that reads the rows from global memory (FP32 sums of 64, Kahan
+//   across them).
 #include "fbp_internal.cuh"
 #include "bp_common.cuh"
 

@@ -27,7 +27,7 @@ struct ExhaustiveGatherParams {
     uint32_t Vx, Vy, Vz, L, S, T;
     float t0, dt;
     uint32_t row_pitch, slot_w;
-    int ch;             // pairs per window stage (a power of two, 4..32)
+    int ch;             // pairs per window stage (a power of two up to 32; at least 4 in blocks of 4 lasers)
     uint32_t chains;    // contiguous ranges of pair groups with compensated sums of their own, one CTA each
     float* chain_sums;  // chains > 1: [chains][sum, compensation][volume]
     int exact_weights;  // 1: every weight by its own rcp.approx (FBP_WEIGHTS_REFERENCE)
@@ -166,8 +166,8 @@ exhaustive_gather_kernel(ExhaustiveGatherParams p) {
             const int bhi = (int)fmaxf(fminf(floorf(pmax * rcp_dt), 1.0e9f), -1.0e9f) + 2;
             // Paths this short make dist^2 <= EPS possible, paths this long
             // (or NaN) could take the shared reciprocal's product out of the
-            // FP32 range, bins this high are no subnormal's bits: those groups
-            // weigh each triple on its own and clamp each bin.
+            // FP32 range, bins this high lie past any row: those groups weigh
+            // each triple on its own and clamp each bin.
             near = pmin < 0.0035f || !(pmax < 1.0e4f) || bhi >= (1 << 22);
             a = max(blo, 0) & ~(ALIGN - 1);
             read = bhi >= 0 && blo < (int)p.T && lp < p.L;

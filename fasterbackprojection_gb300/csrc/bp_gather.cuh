@@ -183,8 +183,9 @@ __device__ __forceinline__ void confocal_stage(const ScanPlan pl, int nl, float 
         // Voxel pairs (k, k + 1) in packed FP32 pairs: the bins are the scalar
         // loop's operations, bit for bit, in half the instructions.  A packed
         // instruction holds the issue port for two cycles, and the port is what
-        // bounds this loop (issue 66 % + second cycles 34 % of all cycles,
-        // MUFU pipe 76 %, before the differences left it: 362 -> 347 ms).
+        // bounds this loop: issue 66 % and second cycles 34 % of all cycles, MUFU
+        // pipe 76 % (362 ms with the x differences worked out here, 347 with the
+        // planner's).
         //
         // Weights by simultaneous inversion (P. L. Montgomery, "Speeding the
         // Pollard and elliptic curve methods of factorization", Math. Comp. 48
@@ -568,7 +569,7 @@ __device__ __forceinline__ void confocal_tile(const ConfocalGatherParams& p, uin
     };
 
     // A wait that ran out of polls (status FBP_ERR_TIMEOUT): the warp keeps
-    // walking the barriers of the cluster but touches nothing else.
+    // arriving at the CTA's barriers but touches nothing else.
     bool dead = false;
     auto wait = [&](uint32_t bar, uint32_t parity) {
         if (!dead && !mbar_wait_parity(bar, parity)) {
