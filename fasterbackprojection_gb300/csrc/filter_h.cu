@@ -93,9 +93,9 @@ __device__ __forceinline__ void filter_block_shared(const float* s_taps, int J, 
 // series' samples before this one is filtered.
 // 65536 x 1024: 371 -> 298 us (FMA pipe 69 %, issue
 // 85 %).
-// (With many taps, NJ == 0, the fill is a small part: nothing is kept or loaded
-// ahead.)
-constexpr int prefetch_rows(int nj) { return nj > 0 ? 3 : 0; }
+// (With many taps, NJ == 0, and 128 threads or more the fill is a small part:
+// nothing is kept or loaded ahead.)
+constexpr int prefetch_rows(int nj, int nt) { return nj > 0 || nt <= 64 ? 3 : 0; }
 constexpr int filter_taps(int nj) { return nj > 0 ? 2 * kFilterQ * nj : kMaxTaps; }
 
 template <int NJ, int nt, int ROW>
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(nt, 1024 / nt) filter_h_kernel(float* __restri
     };
     // The slots of this thread's first kPrefetch half rows (the same for every
     // series): half row g holds slots 4 g - F and on.
-    constexpr int kPrefetch = prefetch_rows(NJ);
+    constexpr int kPrefetch = prefetch_rows(NJ, nt);
     uint32_t from[kPrefetch + 1][4], kept = 0;
 #pragma unroll
     for (int u = 0; u < kPrefetch; ++u)
@@ -288,8 +288,9 @@ fbp_status filter_h_device(fbp_context* ctx, float* data, uint64_t nseries, uint
     // 55; 4096 x 10000, 4-bin waves 243 and 193), from where four of them fit (some
     // 11,000 bins) with 256 threads (4096 x 20000, 10-bin waves: 1043 us padded,
     // 583 so).  Waves of more than 20 bins (NJ == 0) have borders and taps that
-    // outweigh the bins of a short series: never fewer than 128 threads (2000 x
-    // 128, 150-bin waves: 63 us with 32, 53 with 128).
+    // outweigh the bins of a short series: 32 or 64 threads only where there are
+    // series enough to fill the GPU with them (150-bin waves: 2000 x 128 63 us with
+    // 32 threads, 53 with 128; 60-bin waves: 20000 x 128 152 and 185).
     auto go = [&](auto nj) -> fbp_status {
         constexpr int NJ = decltype(nj)::value;
         constexpr std::integral_constant<int, kRowPadded> padded{};
@@ -298,11 +299,14 @@ fbp_status filter_h_device(fbp_context* ctx, float* data, uint64_t nseries, uint
         if constexpr (NJ > 0) {
             // (few series: threads enough to load each in one go, too)
             auto enough = [&](uint32_t nt) {
-                return T <= nt * Q && (nseries > 2ull * ctx->sm_count || 2 * (uint32_t)rows <= prefetch_rows(NJ) * nt);
+                return T <= nt * Q && (nseries > 2ull * ctx->sm_count || 2 * (uint32_t)rows <= prefetch_rows(NJ, 32) * nt);
             };
             if (enough(32)) return launch(nj, std::integral_constant<int, 32>{}, padded);
             if (enough(64)) return launch(nj, std::integral_constant<int, 64>{}, padded);
             if (fit(kRowPadded) >= (NJ >= 5 ? 4 : 6)) return launch(nj, std::integral_constant<int, 128>{}, padded);
+        } else if (T <= 64 * Q && fit(kRowPadded) >= 6) {
+            if (T <= 32 * Q && nseries > 50ull * ctx->sm_count) return launch(nj, std::integral_constant<int, 32>{}, padded);
+            if (T > 32 * Q && nseries > 4ull * ctx->sm_count) return launch(nj, std::integral_constant<int, 64>{}, padded);
         }
         return launch(nj, std::integral_constant<int, 128>{}, dense);
     };
