@@ -274,7 +274,8 @@ fbp_status filter_h_device(fbp_context* ctx, float* data, uint64_t nseries, uint
         // One CTA per resident slot (64 registers a thread), or twice as many
         // where that leaves each only a few series; long series, whose setup is
         // nothing beside them, 16 to an SM.
-        const uint64_t slots = (uint64_t)ctx->sm_count * std::max<size_t>(1, std::min<size_t>(std::min<size_t>(32, 1024 / threads), fit(ROW)));
+        const size_t resident = std::max<size_t>(1, std::min<size_t>(std::min<size_t>(32, 1024 / threads), fit(ROW)));
+        const uint64_t slots = (uint64_t)ctx->sm_count * resident;
         const uint64_t most = ROW == kRowDense ? (uint64_t)ctx->sm_count * 16 : nseries < 8 * slots ? 2 * slots : slots;
         kernel<<<(unsigned)std::min<uint64_t>(nseries, most), threads, smem, stream>>>(
             data, nseries, T, n, R, pad, border == FBP_BORDER_EDGE, F, ntp, rows, tp);
